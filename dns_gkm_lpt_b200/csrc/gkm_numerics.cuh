@@ -11,14 +11,17 @@
 //
 // Two forms of the flux.  gks_flux_mcal keeps the reference's moment algebra
 // (one MCal per table, weight and slope vector) and is what the operation
-// counter measures.  gks_flux_tau, the one the kernels run, takes the same
-// moments of the same slope vectors as contractions of the normal tables with
-// tangential functionals of each slope polynomial, and forms each reciprocal
-// once (grouped divisions, one reciprocal square root per state).  The two
-// forms and the reference differ only by rounding.
+// counter measures.  gks_flux_peculiar, the one the kernels run, takes the same
+// moments of the same slope vectors in the velocity frame of each state, where
+// most of them are closed forms, and forms each reciprocal once (grouped
+// divisions, one reciprocal square root per state).  The two forms and the
+// reference differ only by rounding.
 #pragma once
 
 #include <math.h>
+
+#include <type_traits>
+#include <utility>
 
 #ifdef __CUDACC__
 #include <cuda_runtime.h>
@@ -34,7 +37,7 @@
 // GKM_REFERENCE_FORM 1 keeps the reference's arithmetic in the shared helpers
 // (two divisions per WENO scalar, the divisions of temperature and face energy)
 // and its MCal moment algebra; the operation counter compiles that form.  The
-// kernels (0) form each reciprocal once and fold the moments.
+// kernels (0) form each reciprocal once and take the moments in the peculiar frames.
 #ifndef GKM_REFERENCE_FORM
 #define GKM_REFERENCE_FORM 0
 #endif
@@ -69,6 +72,10 @@ struct Phys {
     T gm1;        // gam - 1
     T Rg;         // gas constant in the working units
     int K;        // internal degrees of freedom (int((5-3g)/(g-1)))
+    T iK3 = T(1) / T(K + 3);
+    // what the energy of a Maxwellian with K internal degrees of freedom exceeds p / (gam - 1) by, over p:
+    // zero but for rounding where (5-3g)/(g-1) is whole
+    T dK = T(0.5 * (K + 3)) - T(1) / gm1;
 };
 
 // ---------------------------------------------------------------- WENO ----
@@ -224,27 +231,12 @@ GKM_HD T face_energy_ir(T r, T ir, T m1, T m2, T m3, T Tf, const Phys<T>& ph)
 // Maxwellian moments of one state: x half-space table H (and H2 for the
 // equilibrium state's other half), full tables X (x), Y (y), Z (z).
 // src/GKMflux.cpp:45-68 (l, r) and :85-103 (e).
-// The tangential tables enter the moments only as products Y[b] Z[c] with
-// b + c <= 5, so they are kept as that 21-entry product table: every triple
-// product of MCal then costs one multiplication instead of two.
-// (GKM_SHARED_YZ 0 keeps the separate tables and forms every triple product
-// with two multiplications as the reference's MCal does; the operation counter
-// uses that to count the reference formulation.)
-#ifndef GKM_SHARED_YZ
-#define GKM_SHARED_YZ (!GKM_REFERENCE_FORM)
-#endif
-constexpr int kYZ = 21;
-GKM_HD constexpr int yz(int b, int c) { return 6 * c - c * (c - 1) / 2 + b; }
 
 template <class T>
 struct Moments {
     T H[7];
     T X[7];
-#if GKM_SHARED_YZ
-    T YZ[kYZ];
-#else
     T Y[6], Z[6];
-#endif
     T Ie2, Ie4;
 };
 
@@ -323,29 +315,13 @@ GKM_HD void build_moments(Moments<T>& M, const T U[3], T lam, int K, int half)
     M.Ie4 = T(3 * K + K * (K - 1)) * inv2lam * inv2lam;
     half_table<T>(M.H, U[0], lam, inv2lam, half);
     full_table<T, 7>(M.X, U[0], inv2lam);
-#if GKM_SHARED_YZ
-    T Y[6], Z[6];
-    full_table<T, 6>(Y, U[1], inv2lam);
-    full_table<T, 6>(Z, U[2], inv2lam);
-#pragma unroll
-    for (int c = 0; c < 6; c++)
-#pragma unroll
-        for (int b = 0; b + c < 6; b++) M.YZ[yz(b, c)] = Y[b] * Z[c];
-#else
     full_table<T, 6>(M.Y, U[1], inv2lam);
     full_table<T, 6>(M.Z, U[2], inv2lam);
-#endif
 }
 
-#if GKM_SHARED_YZ
-#define GKM_TABLES(S) S.YZ
-#define TM(A, B, C) (I[k + (A)] * YZ[yz(l + (B), m + (C))])
-#define GKM_YZ_PARAM const T* YZ
-#else
 #define GKM_TABLES(S) S.Y, S.Z
 #define TM(A, B, C) (I[k + (A)] * Y[l + (B)] * Z[m + (C)])
 #define GKM_YZ_PARAM const T* Y, const T* Z
-#endif
 
 // ----------------------------------------------------------- MCal -----
 // <psi (u^k v^l w^m) (a0 + a1 u + a2 v + a3 w + a4 psi4)> with psi = (1,u,v,w,psi4),
@@ -504,7 +480,7 @@ struct FaceInput {
 
 // The flux with the reference's moment algebra: one MCal (25 triple products
 // and their sums) per table, weight and slope vector.  The operation counter
-// instantiates this form; the kernels run gks_flux_tau below.
+// instantiates this form; the kernels run gks_flux_peculiar below.
 template <class T, class Prov>
 GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, T F[5])
 {
@@ -654,110 +630,33 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
     for (int q = 0; q < 5; q++) F[q] = Facc[q];
 }
 
-#if GKM_SHARED_YZ
-// ------------------------------------------------ moment functionals ----
-// Every moment the flux takes is <u^k psi_i P>_N for a table N (full or half
-// space) and a polynomial P built from slope vectors: P = psi.a, or
-// G = u (psi.a_n) + v (psi.a_y) + w (psi.a_z).  Writing P = sum_p u^p Q_p(v, w, xi^2),
-//   <u^k psi_i P>_N = sum_p N[p + k] tau_i(Q_p)          (i = 0, 2, 3)
-//   <u^k psi_1 P>_N = sum_p N[p + k + 1] tau_0(Q_p)
-//   <u^k psi_4 P>_N = sum_p (N[p + k + 2] tau_0(Q_p) / 2 + N[p + k] tau_4(Q_p))
-// with the tangential functionals tau_0 = <Q>, tau_2 = <v Q>, tau_3 = <w Q>,
-// tau_4 = <(v^2 + w^2 + xi^2) Q> / 2.  They involve the tangential tables only,
-// so one set serves the full and the half-space table and the weights u^0 and
-// u^1: a contraction costs 24 multiply-adds where MCal forms 25 triple
-// products and their sums again.  Same moments, summed in another order.
-template <class T>
-struct Tau {
-    T c0[4], cv[4], cw[4], c4[4];   // tau_0, tau_2, tau_3, tau_4 of Q_0 .. Q_3
-};
+// ---------------------------------------------- the peculiar-frame flux ----
+// The moments of a Maxwellian are Gaussian in the peculiar velocity
+// (c, v', w') = (u, v, w) - U: over the full space the odd ones vanish and the even ones are
+// products of s = 1/(2 lam); over a half space only the normal direction keeps a table,
+// J_k = <c^k>_{u>0}.  Written in psi'' = (1, c, v', w', (c^2 + v'^2 + w'^2 + xi^2)/2),
+//   * the slope solve is diagonal (SlopeP, solve_lab / solve_pec);
+//   * the full-space moments of G = u (psi.a_n) + v (psi.a_y) + w (psi.a_z) are closed forms
+//     of a few products (full_G): with A = U a_n + V a_y + W a_z and D = c P_n + v' P_y + w' P_z,
+//     G = psi''.A + D;
+//   * the half-space moments of G and of psi.a are sums of four or three J_k per component,
+//     because the tangential average of zeta = v'^2 + w'^2 + xi^2 against a polynomial differs
+//     from <zeta> times its average by one product with s (half_G, half_P).
+// Every moment, slope and time coefficient is the reference's (src/GKMflux.cpp:11-229); the
+// frames, and so the order of the sums, are not.  Each side's moments go from its own frame to
+// the equilibrium state's by psi_e = T(U - U_e) psi'' (to_frame), where the equilibrium's slopes
+// are solved, and the summed flux to the laboratory frame at the end.  The reference's
+// gamma_1 (moments of the equilibrium) + gamma_3 (its conserved state), gamma_3 = -gamma_1, has
+// an energy component only, gamma_1 p dK (Phys).  About 900 operations per face beside the divisions and
+// the special functions, where the moments in the laboratory frame took about 2,000; the sweeps
+// are bound by the FP64 (mixed: FP32) arithmetic.  Measured at 256^3 with the default shapes: a step
+// 18.00 -> 13.97 ms in FP64, 10.62 -> 8.26 ms in the mixed form; errors against extended precision
+// equal (mass, tangential momentum) or smaller (normal momentum, energy).
 
-template <bool ADD, class T, class V>
-GKM_HD void put(T& x, const V& v)
-{
-    if constexpr (ADD) x += v;
-    else x = v;
-}
-
-// mu(q, r, s) = <v^q w^r xi^(2s)>
-template <int Q, int R, int S, class T>
-GKM_HD T mu(const Moments<T>& M)
-{
-    static_assert(Q + R <= 5 && S <= 2, "tangential moment beyond the tables");
-    if constexpr (S == 0) return M.YZ[yz(Q, R)];
-    else if constexpr (S == 1) return M.YZ[yz(Q, R)] * M.Ie2;
-    else return M.YZ[yz(Q, R)] * M.Ie4;
-}
-
-// <v^q w^r xi^(2s) R(a)>, R(a) = a0 + a2 v + a3 w + (a4/2)(v^2 + w^2 + xi^2) the u-free part of psi.a
-template <int Q, int R, int S, class T>
-GKM_HD T rho_moment(const T a[5], T h4, const Moments<T>& M)
-{
-    return a[0] * mu<Q, R, S>(M) + a[2] * mu<Q + 1, R, S>(M) + a[3] * mu<Q, R + 1, S>(M) +
-           h4 * (mu<Q + 2, R, S>(M) + mu<Q, R + 2, S>(M) + mu<Q, R, S + 1>(M));
-}
-
-// functionals of Q = v^q w^r R(a) into entry p
-template <bool ADD, int Q, int R, int P, class T>
-GKM_HD void tau_R(Tau<T>& t, const T a[5], T h4, const Moments<T>& M)
-{
-    put<ADD>(t.c0[P], rho_moment<Q, R, 0>(a, h4, M));
-    put<ADD>(t.cv[P], rho_moment<Q + 1, R, 0>(a, h4, M));
-    put<ADD>(t.cw[P], rho_moment<Q, R + 1, 0>(a, h4, M));
-    put<ADD>(t.c4[P], T(0.5) * (rho_moment<Q + 2, R, 0>(a, h4, M) + rho_moment<Q, R + 2, 0>(a, h4, M) +
-                                rho_moment<Q, R, 1>(a, h4, M)));
-}
-
-// functionals of Q = c v^q w^r into entry p
-template <bool ADD, int Q, int R, int P, class T>
-GKM_HD void tau_mono(Tau<T>& t, T c, const Moments<T>& M)
-{
-    put<ADD>(t.c0[P], c * mu<Q, R, 0>(M));
-    put<ADD>(t.cv[P], c * mu<Q + 1, R, 0>(M));
-    put<ADD>(t.cw[P], c * mu<Q, R + 1, 0>(M));
-    put<ADD>(t.c4[P], (T(0.5) * c) * (mu<Q + 2, R, 0>(M) + mu<Q, R + 2, 0>(M) + mu<Q, R, 1>(M)));
-}
-
-// functionals of psi.a: Q_0 = R(a), Q_1 = a1, Q_2 = a4/2
-template <class T>
-GKM_HD void tau_psi(Tau<T>& t, const T a[5], const Moments<T>& M)
-{
-    const T h4 = T(0.5) * a[4];
-    tau_R<false, 0, 0, 0>(t, a, h4, M);
-    tau_mono<false, 0, 0, 1>(t, a[1], M);
-    tau_mono<false, 0, 0, 2>(t, h4, M);
-}
-
-// out_i = <u^k psi_i P>_N, P = sum_{p = P0..P1} u^p Q_p
-template <int K, int P0, int P1, class T>
-GKM_HD void contract(T out[5], const T* N, const Tau<T>& t)
-{
-    static_assert(P1 + K + 2 <= 6, "normal moment beyond the table");
-    T o0 = N[P0 + K] * t.c0[P0];
-    T o1 = N[P0 + K + 1] * t.c0[P0];
-    T o2 = N[P0 + K] * t.cv[P0];
-    T o3 = N[P0 + K] * t.cw[P0];
-    T o4 = N[P0 + K] * t.c4[P0] + T(0.5) * N[P0 + K + 2] * t.c0[P0];
-#pragma unroll
-    for (int p = P0 + 1; p <= P1; p++) {
-        o0 += N[p + K] * t.c0[p];
-        o1 += N[p + K + 1] * t.c0[p];
-        o2 += N[p + K] * t.cv[p];
-        o3 += N[p + K] * t.cw[p];
-        o4 += N[p + K] * t.c4[p] + T(0.5) * N[p + K + 2] * t.c0[p];
-    }
-    out[0] = o0;
-    out[1] = o1;
-    out[2] = o2;
-    out[3] = o3;
-    out[4] = o4;
-}
-
-// Primitive values of a state with the reciprocals the flux reuses: 1/rho,
-// lam = rho / (2 p) and 1 / (2 lam) = p / rho.
+// Primitive values of a state: 1/rho, p, s = 1 / (2 lam) = p / rho and 1 / s.
 template <class T>
 struct Prim {
-    T den, ir, U[3], P, lam, inv2lam;
+    T den, ir, U[3], P, s, is;
 };
 
 // both face states together, with pd = p rho = (gamma - 1)(E rho - |m|^2 / 2) known before any
@@ -781,16 +680,16 @@ GKM_HD void prim_pair(const T wl[5], const T wr[5], T gm1, Prim<T>& l, Prim<T>& 
     inv_psum = dd * (dd * pp * inv);
     Prim<T>* st[2] = {&l, &r};
     const T* w[2] = {wl, wr};
-    const T pd[2] = {pdl, pdr}, iP[2] = {iPl, iPr};
+    const T iP[2] = {iPl, iPr};
 #pragma unroll
     for (int k = 0; k < 2; k++) {
-        Prim<T>& s = *st[k];
-        s.U[0] = w[k][1] * s.ir;
-        s.U[1] = w[k][2] * s.ir;
-        s.U[2] = w[k][3] * s.ir;
-        s.P = pd[k] * s.ir;
-        s.lam = T(0.5) * s.den * iP[k];
-        s.inv2lam = s.P * s.ir;
+        Prim<T>& p = *st[k];
+        p.U[0] = w[k][1] * p.ir;
+        p.U[1] = w[k][2] * p.ir;
+        p.U[2] = w[k][3] * p.ir;
+        p.P = gm1 * (w[k][4] - T(0.5) * (w[k][1] * p.U[0] + w[k][2] * p.U[1] + w[k][3] * p.U[2]));
+        p.s = p.P * p.ir;
+        p.is = p.den * iP[k];
     }
 }
 
@@ -798,147 +697,214 @@ GKM_HD void prim_pair(const T wl[5], const T wr[5], T gm1, Prim<T>& l, Prim<T>& 
 template <class T>
 GKM_HD Prim<T> prim(const T W[5], T gm1)
 {
-    Prim<T> s;
-    s.den = W[0];
-    const T pd = gm1 * (W[4] * s.den - T(0.5) * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]));
-    const T inv = T(1) / (s.den * pd);
-    s.ir = pd * inv;
-    s.U[0] = W[1] * s.ir;
-    s.U[1] = W[2] * s.ir;
-    s.U[2] = W[3] * s.ir;
-    s.P = pd * s.ir;
-    s.lam = T(0.5) * s.den * (s.den * s.den * inv);
-    s.inv2lam = s.P * s.ir;
-    return s;
+    Prim<T> p;
+    p.den = W[0];
+    const T pd = gm1 * (W[4] * p.den - T(0.5) * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]));
+    const T inv = T(1) / (p.den * pd);
+    p.ir = pd * inv;
+    p.U[0] = W[1] * p.ir;
+    p.U[1] = W[2] * p.ir;
+    p.U[2] = W[3] * p.ir;
+    p.P = gm1 * (W[4] - T(0.5) * (W[1] * p.U[0] + W[2] * p.U[1] + W[3] * p.U[2]));
+    p.s = p.P * p.ir;
+    p.is = p.den * (p.den * p.den * inv);
+    return p;
 }
 
-// moment tables of a state (build_moments) with sqrt(lam) and 1/sqrt(lam pi) from one
-// reciprocal square root
+// <1> and <c> over the half space u > 0 (half > 0) or u < 0: J_0 = erfc(-+ sqrt(lam) U)/2 and
+// J_1 = +- exp(-lam U^2) / (2 sqrt(pi lam)), with sqrt(s) from one reciprocal square root
 template <class T>
-GKM_HD void build_moments_prim(Moments<T>& M, const Prim<T>& st, int K, int half)
+GKM_HD void half_space(const Prim<T>& p, int half, T& J0, T& g)
 {
-    const T inv2lam = st.inv2lam, U0 = st.U[0];
-    M.Ie2 = T(K) * inv2lam;
-    M.Ie4 = T(3 * K + K * (K - 1)) * inv2lam * inv2lam;
-    const T isl = rsqrt_t<T>(st.lam);
-    const T sl = st.lam * isl;
-    const T g = T(0.28209479177387814347) * exp_t<T>(-st.lam * U0 * U0) * isl;   // 1 / (2 sqrt(pi))
-    if (half > 0) {
-        M.H[0] = T(0.5) * erfc_t<T>(-sl * U0);
-        M.H[1] = U0 * M.H[0] + g;
-    } else {
-        M.H[0] = T(0.5) * erfc_t<T>(sl * U0);
-        M.H[1] = U0 * M.H[0] - g;
+    const T rs = rsqrt_t<T>(p.is);                                    // sqrt(s)
+    const T x = p.U[0] * (p.is * rs) * T(0.70710678118654752440);     // sqrt(lam) U
+    const T e = T(0.39894228040143267794) * exp_t<T>(-x * x) * rs;    // sqrt(s / (2 pi)) exp(-lam U^2)
+    J0 = T(0.5) * erfc_t<T>(half > 0 ? -x : x);
+    g = half > 0 ? e : -e;
+}
+
+// J_k = <c^k> over that half space: J_k = (k - 1) s J_{k-2} + (-U)^{k-1} g
+template <class T, int N>
+GKM_HD void half_moments(T* J, T J0, T g, T U, T s)
+{
+    J[0] = J0;
+    J[1] = g;
+    T q = g;
+#pragma unroll
+    for (int k = 2; k < N; k++) {
+        q = -U * q;
+        J[k] = (T(k - 1) * s) * J[k - 2] + q;
     }
-#pragma unroll
-    for (int i = 2; i < 7; i++) M.H[i] = U0 * M.H[i - 1] + M.H[i - 2] * (T(i - 1) * inv2lam);
-    full_table<T, 7>(M.X, U0, inv2lam);
-    T Y[6], Z[6];
-    full_table<T, 6>(Y, st.U[1], inv2lam);
-    full_table<T, 6>(Z, st.U[2], inv2lam);
-#pragma unroll
-    for (int c = 0; c < 6; c++)
-#pragma unroll
-        for (int b = 0; b + c < 6; b++) M.YZ[yz(b, c)] = Y[b] * Z[c];
 }
 
-// slope_state without divisions: (K+3)/(2 lam) = (K+3) inv2lam; iK3 = 1/(K+3)
+// one slope vector in the peculiar frame of its state: psi.a = a0 + a1 c + a2 v' + a3 w' + 2 h psi4''
 template <class T>
-GKM_HD SlopeState<T> slope_state_prim(const Prim<T>& st, T iK3, int K)
+struct SlopeP {
+    T a0, a1, a2, a3, h;
+};
+
+// what the solves of one state share: uq = (|U|^2 + (K+3) s)/2, z3 = (K+3) s, hf = 1/(Pr (K+3) s^2)
+template <class T>
+struct SolveP {
+    T uq, z3, hf;
+};
+template <class T>
+GKM_HD SolveP<T> solve_consts(const Prim<T>& p, T iK3, int K)
 {
-    SlopeState<T> s;
-    s.U[0] = st.U[0];
-    s.U[1] = st.U[1];
-    s.U[2] = st.U[2];
-    s.lam2 = T(2) * st.lam;
-    s.usqc = st.U[0] * st.U[0] + st.U[1] * st.U[1] + st.U[2] * st.U[2] + T(K + 3) * st.inv2lam;
-    s.a4fac = T(1.0 / kPrandtl) * (T(4) * st.lam * st.lam) * iK3;
-    return s;
+    SolveP<T> c;
+    c.z3 = T(K + 3) * p.s;
+    c.uq = T(0.5) * (p.U[0] * p.U[0] + p.U[1] * p.U[1] + p.U[2] * p.U[2] + c.z3);
+    c.hf = (T(1.0 / kPrandtl) * iK3) * (p.is * p.is);
+    return c;
 }
 
-// The equilibrium part of the flux (src/GKMflux.cpp:73-229 after the two half-Maxwellians):
-// the equilibrium state We at the face, its slopes from the cell averages and the tangential
-// slopes by_, bz_ the sides gathered, the time derivative from Bacc, and the flux moments added to
-// Facc.  gm1..p2 are the time coefficients of src/GKMflux.cpp:162-167,197-204.
+// the slope solver (src/GKMflux.cpp:283-297) of sc * b, b the moments in the laboratory frame
+template <class T>
+GKM_HD SlopeP<T> solve_lab(T b0, T b1, T b2, T b3, T b4, T sc, const Prim<T>& p, const SolveP<T>& c)
+{
+    const T r1 = b1 - p.U[0] * b0, r2 = b2 - p.U[1] * b0, r3 = b3 - p.U[2] * b0;
+    const T e = b4 - p.U[0] * r1 - p.U[1] * r2 - p.U[2] * r3 - c.uq * b0;
+    const T l = sc * p.is;
+    SlopeP<T> a;
+    a.h = (sc * c.hf) * e;
+    a.a1 = l * r1;
+    a.a2 = l * r2;
+    a.a3 = l * r3;
+    a.a0 = sc * b0 - a.h * c.z3;
+    return a;
+}
+// the same of moments already in the state's peculiar frame
+template <class T>
+GKM_HD SlopeP<T> solve_pec(const T b[5], const Prim<T>& p, const SolveP<T>& c)
+{
+    SlopeP<T> a;
+    a.h = c.hf * (b[4] - (T(0.5) * c.z3) * b[0]);
+    a.a1 = p.is * b[1];
+    a.a2 = p.is * b[2];
+    a.a3 = p.is * b[3];
+    a.a0 = b[0] - a.h * c.z3;
+    return a;
+}
+
+// moments in a frame moving with U -> the frame moving with U - d: psi -> T(d) psi, hd = |d|^2/2
+template <class T>
+GKM_HD void to_frame(T o[5], const T d[3], T hd)
+{
+    o[4] += d[0] * o[1] + d[1] * o[2] + d[2] * o[3] + hd * o[0];
+    o[1] += d[0] * o[0];
+    o[2] += d[1] * o[0];
+    o[3] += d[2] * o[0];
+}
+
+// <psi'' (psi.a)> with the normal weight N_k (N = J: weight 1; N = L: weight u)
+template <class T>
+GKM_HD void half_P(T o[5], const T* N, const SlopeP<T>& a, T s, T hz1)
+{
+    const T hz = a.h * (hz1 + hz1);            // h <zeta>
+    const T t = a.a0 + hz;
+    const T s0 = t * N[0] + a.a1 * N[1] + a.h * N[2];
+    const T s1 = t * N[1] + a.a1 * N[2] + a.h * N[3];
+    const T s2 = t * N[2] + a.a1 * N[3] + a.h * N[4];
+    const T sn = s * N[0];
+    o[0] = s0;
+    o[1] = s1;
+    o[2] = sn * a.a2;
+    o[3] = sn * a.a3;
+    o[4] = hz1 * s0 + T(0.5) * s2 + sn * hz;
+}
+
+// the same with weights 1 and u (o and p) over one table
+template <class T>
+GKM_HD void half_P2(T o[5], T p[5], const T* N, const SlopeP<T>& a, T s, T U, T hz1)
+{
+    const T hz = a.h * (hz1 + hz1);
+    const T t = a.a0 + hz;
+    const T s0 = t * N[0] + a.a1 * N[1] + a.h * N[2];
+    const T s1 = t * N[1] + a.a1 * N[2] + a.h * N[3];
+    const T s2 = t * N[2] + a.a1 * N[3] + a.h * N[4];
+    const T s3 = t * N[3] + a.a1 * N[4] + a.h * N[5];
+    const T sn = s * N[0], sm = s * (N[1] + U * N[0]);
+    o[0] = s0;
+    o[1] = s1;
+    o[2] = sn * a.a2;
+    o[3] = sn * a.a3;
+    o[4] = hz1 * s0 + T(0.5) * s2 + sn * hz;
+    p[0] = s1 + U * s0;
+    p[1] = s2 + U * s1;
+    p[2] = sm * a.a2;
+    p[3] = sm * a.a3;
+    p[4] = hz1 * p[0] + T(0.5) * (s3 + U * s2) + sm * hz;
+}
+
+// the convective part of G: A = U a_n + V a_y + W a_z
+template <class T>
+GKM_HD SlopeP<T> convect(const T U[3], const SlopeP<T>& n, const SlopeP<T>& y, const SlopeP<T>& z)
+{
+    SlopeP<T> A;
+    A.a0 = U[0] * n.a0 + U[1] * y.a0 + U[2] * z.a0;
+    A.a1 = U[0] * n.a1 + U[1] * y.a1 + U[2] * z.a1;
+    A.a2 = U[0] * n.a2 + U[1] * y.a2 + U[2] * z.a2;
+    A.a3 = U[0] * n.a3 + U[1] * y.a3 + U[2] * z.a3;
+    A.h = U[0] * n.h + U[1] * y.h + U[2] * z.h;
+    return A;
+}
+
+// <psi'' G> with weights 1 and u (o and p) over the half space of J
+template <class T>
+GKM_HD void half_G(T o[5], T p[5], const T* J, const SlopeP<T>& A, const SlopeP<T>& n, const SlopeP<T>& y,
+                   const SlopeP<T>& z, T s, T U, T hz1, T k4)
+{
+    // <G>_tan = c0 + c1 c + c2 c^2 + c3 c^3, <zeta G>_tan / 2 = hz1 <G>_tan + s (y0 + y1 c)
+    const T z1 = hz1 + hz1;
+    const T y0 = A.h * z1 + s * (y.a2 + z.a3), y1 = n.h * z1;
+    const T c0 = A.a0 + y0, c1 = A.a1 + n.a0 + y1, c2 = A.h + n.a1, c3 = n.h;
+    const T s0 = c0 * J[0] + c1 * J[1] + c2 * J[2] + c3 * J[3];
+    const T s1 = c0 * J[1] + c1 * J[2] + c2 * J[3] + c3 * J[4];
+    const T s2 = c0 * J[2] + c1 * J[3] + c2 * J[4] + c3 * J[5];
+    const T s3 = c0 * J[3] + c1 * J[4] + c2 * J[5] + c3 * J[6];
+    // <v' G>_tan = s (v0 + v1 c + h_y c^2), <w' G>_tan likewise
+    const T v0 = A.a2 + y.a0 + y.h * k4, v1 = n.a2 + y.a1;
+    const T w0 = A.a3 + z.a0 + z.h * k4, w1 = n.a3 + z.a1;
+    const T va = v0 * J[0] + v1 * J[1] + y.h * J[2], vb = v0 * J[1] + v1 * J[2] + y.h * J[3];
+    const T wa = w0 * J[0] + w1 * J[1] + z.h * J[2], wb = w0 * J[1] + w1 * J[2] + z.h * J[3];
+    const T ea = y0 * J[0] + y1 * J[1], eb = y0 * J[1] + y1 * J[2];
+    o[0] = s0;
+    o[1] = s1;
+    o[2] = s * va;
+    o[3] = s * wa;
+    o[4] = hz1 * s0 + T(0.5) * s2 + s * ea;
+    p[0] = s1 + U * s0;
+    p[1] = s2 + U * s1;
+    p[2] = s * (vb + U * va);
+    p[3] = s * (wb + U * wa);
+    p[4] = hz1 * p[0] + T(0.5) * (s3 + U * s2) + s * (eb + U * ea);
+}
+
+// a face provider may give raw differences and their common factors instead of slopes:
+//   T dW(int v, int q), the difference; T scale(int v), the factor (slope = scale * dW)
+template <class Prov, class = void>
+struct has_raw : std::false_type {};
+template <class Prov>
+struct has_raw<Prov, std::void_t<decltype(std::declval<const Prov&>().scale(0))>> : std::true_type {};
+
 template <class T, class Prov>
-GKM_HD void gks_equilibrium_part(const Prov& in, const T We[5], const T by_[5], const T bz_[5], T Bacc[5], T Facc[5],
-                                 T gm1, T gm2, T gm3, T p0, T p1, T p2, T iK3, T dx, const Phys<T>& ph, T F[5])
+GKM_HD SlopeP<T> face_slope(const Prov& in, int v, const Prim<T>& p, const SolveP<T>& c)
+{
+    if constexpr (has_raw<Prov>::value)
+        return solve_lab<T>(in.dW(v, 0), in.dW(v, 1), in.dW(v, 2), in.dW(v, 3), in.dW(v, 4), in.scale(v), p, c);
+    else
+        return solve_lab<T>(in.DW(v, 0), in.DW(v, 1), in.DW(v, 2), in.DW(v, 3), in.DW(v, 4), T(1), p, c);
+}
+
+// The flux of gks_flux_mcal with every moment taken in the peculiar frames.  The slopes of a side
+// are kept times its density (and the equilibrium's times its own), which is the factor their
+// moments enter the flux with.
+template <class T, class Prov>
+GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, T F[5])
 {
     const int K = ph.K;
-    T M[5];
-    const Prim<T> ste = prim<T>(We, ph.gm1);
-    const T dene = ste.den;
-    Moments<T> E;
-    build_moments_prim<T>(E, ste, K, +1);
-    // the negative half space of the equilibrium: full table minus the positive half
-    T H2[7];
-#pragma unroll
-    for (int i = 0; i < 7; i++) H2[i] = E.X[i] - E.H[i];
-    SlopeState<T> se = slope_state_prim<T>(ste, iK3, K);
-    Tau<T> tp;
-    T b[5], a[5];
-    const T idx2 = (T(2) / dx) * ste.ir;
-    // normal equilibrium slopes from the cell averages, src/GKMflux.cpp:115-116
-#pragma unroll
-    for (int q = 0; q < 5; q++) b[q] = (We[q] - in.WL(q)) * idx2;
-    slope_solve<T>(b, se, a);
-    tau_psi<T>(tp, a, E);
-    contract<1, 0, 2>(M, E.H, tp);
-    axpy5<T>(Bacc, gm2 * dene, M);
-    contract<2, 0, 2>(M, E.H, tp);
-    axpy5<T>(Facc, p2 * dene, M);
-#pragma unroll
-    for (int q = 0; q < 5; q++) b[q] = (in.WR(q) - We[q]) * idx2;
-    slope_solve<T>(b, se, a);
-    tau_psi<T>(tp, a, E);
-    contract<1, 0, 2>(M, H2, tp);
-    axpy5<T>(Bacc, gm2 * dene, M);
-    contract<2, 0, 2>(M, H2, tp);
-    axpy5<T>(Facc, p2 * dene, M);
-    // tangential equilibrium slopes: G_E = v (psi.a_y) + w (psi.a_z),
-    //   Q_0 = v R(a_y) + w R(a_z), Q_1 = a1y v + a1z w, Q_2 = (a4y/2) v + (a4z/2) w
-    slope_solve<T>(by_, se, a);
-    {
-        const T h4 = T(0.5) * a[4];
-        tau_R<false, 1, 0, 0>(tp, a, h4, E);
-        tau_mono<false, 1, 0, 1>(tp, a[1], E);
-        tau_mono<false, 1, 0, 2>(tp, h4, E);
-    }
-    slope_solve<T>(bz_, se, a);
-    {
-        const T h4 = T(0.5) * a[4];
-        tau_R<true, 0, 1, 0>(tp, a, h4, E);
-        tau_mono<true, 0, 1, 1>(tp, a[1], E);
-        tau_mono<true, 0, 1, 2>(tp, h4, E);
-    }
-    contract<0, 0, 2>(M, E.X, tp);
-    axpy5<T>(Bacc, gm2 * dene, M);
-    contract<1, 0, 2>(M, E.X, tp);
-    axpy5<T>(Facc, p2 * dene, M);
-    // time derivative of the equilibrium, src/GKMflux.cpp:183-191
-    mcal0<0, 0, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2);
-    const T idene = ste.ir;
-#pragma unroll
-    for (int q = 0; q < 5; q++) b[q] = (gm1 * dene * M[q] + Bacc[q] + gm3 * We[q]) * idene;
-    slope_solve<T>(b, se, a);
-    tau_psi<T>(tp, a, E);
-    contract<1, 0, 2>(M, E.X, tp);
-    axpy5<T>(Facc, p1 * dene, M);
-    mcal0<1, 0, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2);
-    axpy5<T>(Facc, p0 * dene, M);
-#pragma unroll
-    for (int q = 0; q < 5; q++) F[q] = Facc[q];
-}
-
-// The flux of gks_flux_mcal with the moment functionals above: the same
-// moments of the same slope vectors (src/GKMflux.cpp:11-229), grouped per
-// polynomial instead of per MCal call.
-template <class T, class Prov>
-GKM_HD void gks_flux_tau(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, T F[5])
-{
-    const int K = ph.K;
-    const T iK3 = T(1) / T(K + 3);
-    Prim<T> stl, str;
+    const T iK3 = ph.iK3;
+    Prim<T> st[2];
     T inv_psum;
     {
         T wl[5], wr[5];
@@ -947,23 +913,36 @@ GKM_HD void gks_flux_tau(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, 
             wl[q] = in.Wl(q);
             wr[q] = in.Wr(q);
         }
-        prim_pair<T>(wl, wr, ph.gm1, stl, str, inv_psum);
+        prim_pair<T>(wl, wr, ph.gm1, st[0], st[1], inv_psum);
     }
-
     // collision time with the pressure-jump correction, src/GKMflux.cpp:156-157:
     // |rho_l/lam_l - rho_r/lam_r| / |rho_l/lam_l + rho_r/lam_r| with rho/lam = 2 p (p > 0)
     const TimeCoefs<wide_t<T>> tc = time_coefs<wide_t<T>, (sizeof(T) < sizeof(wide_t<T>))>(
-        wide_t<T>(tau0) + wide_t<T>(dt) * wide_t<T>(fabs(stl.P - str.P) * inv_psum), wide_t<T>(dt));
-    const T gm1 = T(tc.gm1), gm2 = T(tc.gm2), gm3 = T(tc.gm3), gm4 = T(tc.gm4), gm5 = T(tc.gm5);
+        wide_t<T>(tau0) + wide_t<T>(dt) * wide_t<T>(fabs(st[0].P - st[1].P) * inv_psum), wide_t<T>(dt));
+    const T gm1 = T(tc.gm1), gm2 = T(tc.gm2), gm4 = T(tc.gm4), gm5 = T(tc.gm5);
     const T p0 = T(tc.p0), p1 = T(tc.p1), p2 = T(tc.p2), p3 = T(tc.p3), p4 = T(tc.p4), p5 = T(tc.p5);
-
-    T We[5] = {0, 0, 0, 0, 0};      // equilibrium state at the face, src/GKMflux.cpp:73-77
-    T by_[5] = {0, 0, 0, 0, 0}, bz_[5] = {0, 0, 0, 0, 0};
-    T Bacc[5] = {0, 0, 0, 0, 0};   // B_ * dene, without the gm1/gm3 terms
-    T Facc[5] = {0, 0, 0, 0, 0};
-    T M[5];
-
     const T cB = gm4 + gm5;
+
+    // the equilibrium state at the face (src/GKMflux.cpp:73-77), from both half-Maxwellians
+    T We[5], J0[2], g[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const Prim<T>& p = st[j];
+        half_space<T>(p, j == 0 ? +1 : -1, J0[j], g[j]);
+        const T m = p.den * J0[j], mu = p.den * (p.U[0] * J0[j] + g[j]);   // rho <1>, rho <u>
+        const T o2 = m * p.U[1], o3 = m * p.U[2];
+        const T o4 = T(0.5) * (mu * p.U[0] + o2 * p.U[1] + o3 * p.U[2] + T(K + 3) * (p.P * J0[j]));
+        if (j == 0) {
+            We[0] = m; We[1] = mu; We[2] = o2; We[3] = o3; We[4] = o4;
+        } else {
+            We[0] += m; We[1] += mu; We[2] += o2; We[3] += o3; We[4] += o4;
+        }
+    }
+    const Prim<T> e = prim<T>(We, ph.gm1);
+
+    // sums over the sides, in the equilibrium's frame: the tangential slopes of the equilibrium
+    // (times its density), rho_e B_ and the flux
+    T by[5] = {0, 0, 0, 0, 0}, bz[5] = {0, 0, 0, 0, 0}, B[5] = {0, 0, 0, 0, 0}, Fe[5] = {0, 0, 0, 0, 0};
     // ---------------- one side (l: positive half with left state, r: negative half with right state)
 #if GKM_UNROLL_SIDES
 #pragma unroll
@@ -971,88 +950,139 @@ GKM_HD void gks_flux_tau(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, 
 #pragma unroll 1
 #endif
     for (int side = 0; side < 2; side++) {
-        const Prim<T>& st = side == 0 ? stl : str;
-        const T den = st.den;
-        Moments<T> S;
-        build_moments_prim<T>(S, st, K, side == 0 ? +1 : -1);
-        SlopeState<T> ss = slope_state_prim<T>(st, iK3, K);
-        const T iden = st.ir;
-        mcal0<0, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2);
-        axpy5<T>(We, den, M);
-        // G = u (psi.a_n) + v (psi.a_y) + w (psi.a_z):
-        //   Q_0 = v R(a_y) + w R(a_z), Q_1 = R(a_n) + a1y v + a1z w,
-        //   Q_2 = a1n + (a4y/2) v + (a4z/2) w, Q_3 = a4n/2
-        Tau<T> tg, tp;
-        T b[5], a[5];
-        // normal slope
+        const Prim<T> p = side == 0 ? st[0] : st[1];
+        const T s = p.s, U = p.U[0];
+        const T hz1 = T(0.5 * (K + 2)) * s, k4 = T(K + 4) * s;
+        const SolveP<T> sv = solve_consts<T>(p, iK3, K);
+        const T d[3] = {U - e.U[0], p.U[1] - e.U[1], p.U[2] - e.U[2]};
+        const T hd = T(0.5) * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        T J[7];
+        half_moments<T, 7>(J, side == 0 ? J0[0] : J0[1], side == 0 ? g[0] : g[1], U, s);
+        const T wy = e.den * p.ir;
+        T o[5], q[5];
+        const SlopeP<T> ay = face_slope<T>(in, 2 + side, p, sv);
+        half_P<T>(o, J, ay, s, hz1);
+        to_frame<T>(o, d, hd);
+        axpy5<T>(by, wy, o);
+        const SlopeP<T> az = face_slope<T>(in, 4 + side, p, sv);
+        half_P<T>(o, J, az, s, hz1);
+        to_frame<T>(o, d, hd);
+        axpy5<T>(bz, wy, o);
+        const SlopeP<T> an = face_slope<T>(in, side, p, sv);
+        const SlopeP<T> A = convect<T>(p.U, an, ay, az);
+        half_G<T>(o, q, J, A, an, ay, az, s, U, hz1, k4);
+        // this side's time slope (src/GKMflux.cpp:145-151): the slopes of -<psi G> over the full space
+        const T S = an.a1 + ay.a2 + az.a3, k5 = T(K + 5) * s;
+        SlopeP<T> at;
+        at.h = T(-1.0 / kPrandtl) * (A.h + iK3 * S);
+        at.a1 = -(A.a1 + an.a0 + an.h * k5);
+        at.a2 = -(A.a2 + ay.a0 + ay.h * k5);
+        at.a3 = -(A.a3 + az.a0 + az.h * k5);
+        at.a0 = -(A.a0 + s * S + (A.h + at.h) * sv.z3);
 #pragma unroll
-        for (int q = 0; q < 5; q++) b[q] = in.DW(0 + side, q) * iden;
-        slope_solve<T>(b, ss, a);
-        {
-            const T h4 = T(0.5) * a[4];
-            tau_R<false, 0, 0, 1>(tg, a, h4, S);
-            tau_mono<false, 0, 0, 2>(tg, a[1], S);
-            tau_mono<false, 0, 0, 3>(tg, h4, S);
+        for (int i = 0; i < 5; i++) {
+            o[i] *= cB;
+            q[i] *= p4;
         }
-        // first tangential slope: <psi (psi.a_y)>_H feeds the equilibrium's y slope
-#pragma unroll
-        for (int q = 0; q < 5; q++) b[q] = in.DW(2 + side, q) * iden;
-        slope_solve<T>(b, ss, a);
+        T x[5], y[5];
+        half_P2<T>(x, y, J, at, s, U, hz1);
+        axpy5<T>(o, gm5, x);
+        axpy5<T>(q, p5, y);
+        // free transport of the initial half-Maxwellian: rho <u psi''>
         {
-            const T h4 = T(0.5) * a[4];
-            tau_psi<T>(tp, a, S);
-            contract<0, 0, 2>(M, S.H, tp);
-            axpy5<T>(by_, T(1), M);
-            tau_R<false, 1, 0, 0>(tg, a, h4, S);
-            tau_mono<true, 1, 0, 1>(tg, a[1], S);
-            tau_mono<true, 1, 0, 2>(tg, h4, S);
+            const T r = p3 * p.den;
+            const T m0 = r * (J[1] + U * J[0]), m1 = r * (J[2] + U * J[1]);
+            q[0] += m0;
+            q[1] += m1;
+            q[4] += hz1 * m0 + T(0.5) * (r * (J[3] + U * J[2]));
         }
-        // second tangential slope
+        to_frame<T>(o, d, hd);
+        to_frame<T>(q, d, hd);
 #pragma unroll
-        for (int q = 0; q < 5; q++) b[q] = in.DW(4 + side, q) * iden;
-        slope_solve<T>(b, ss, a);
-        {
-            const T h4 = T(0.5) * a[4];
-            tau_psi<T>(tp, a, S);
-            contract<0, 0, 2>(M, S.H, tp);
-            axpy5<T>(bz_, T(1), M);
-            tau_R<true, 0, 1, 0>(tg, a, h4, S);
-            tau_mono<true, 0, 1, 1>(tg, a[1], S);
-            tau_mono<true, 0, 1, 2>(tg, h4, S);
+        for (int i = 0; i < 5; i++) {
+            B[i] += o[i];
+            Fe[i] += q[i];
         }
-        // -<psi G>_X is the right-hand side of this side's time slope, src/GKMflux.cpp:145-151
-        contract<0, 0, 3>(M, S.X, tg);
-#pragma unroll
-        for (int q = 0; q < 5; q++) b[q] = -M[q];
-        contract<0, 0, 3>(M, S.H, tg);
-        axpy5<T>(Bacc, cB * den, M);
-        contract<1, 0, 3>(M, S.H, tg);
-        axpy5<T>(Facc, p4 * den, M);
-        // time slope of this side
-        slope_solve<T>(b, ss, a);
-        tau_psi<T>(tp, a, S);
-        contract<0, 0, 2>(M, S.H, tp);
-        axpy5<T>(Bacc, gm5 * den, M);
-        contract<1, 0, 2>(M, S.H, tp);
-        axpy5<T>(Facc, p5 * den, M);
-        // free transport of the initial half-Maxwellian
-        mcal0<1, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2);
-        axpy5<T>(Facc, p3 * den, M);
     }
-    gks_equilibrium_part<T>(in, We, by_, bz_, Bacc, Facc, gm1, gm2, gm3, p0, p1, p2, iK3, dx, ph, F);
+
+    // ---------------- equilibrium part, in its own frame
+    const T s = e.s, U = e.U[0];
+    const T hz1 = T(0.5 * (K + 2)) * s, k5 = T(K + 5) * s, k7 = T(K + 7) * s;
+    const SolveP<T> sv = solve_consts<T>(e, iK3, K);
+    // normal slopes from the cell averages (src/GKMflux.cpp:115-116), left minus right and right:
+    // <P_l>_{u>0} + <P_r>_{u<0} = <P_l - P_r>_{u>0} + <P_r>
+    const T idx2 = T(2) / dx;
+    T br[5], bd[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        const T WL = in.WL(i), WR = in.WR(i);
+        br[i] = WR - We[i];
+        bd[i] = (We[i] - WL) - br[i];
+    }
+    {
+        T J0e, ge, J[7], L[6], o[5], q[5];
+        half_space<T>(e, +1, J0e, ge);
+        half_moments<T, 7>(J, J0e, ge, U, s);
+#pragma unroll
+        for (int k = 0; k < 6; k++) L[k] = J[k + 1] + U * J[k];   // <u c^k>
+        const SlopeP<T> ad = solve_lab<T>(bd[0], bd[1], bd[2], bd[3], bd[4], idx2, e, sv);
+        half_P2<T>(o, q, L, ad, s, U, hz1);
+        axpy5<T>(B, gm2, o);
+        axpy5<T>(Fe, p2, q);
+    }
+    {
+        // G with the right normal slope and the tangential slopes, over the full space
+        const SlopeP<T> an = solve_lab<T>(br[0], br[1], br[2], br[3], br[4], idx2, e, sv);
+        const SlopeP<T> ay = solve_pec<T>(by, e, sv), az = solve_pec<T>(bz, e, sv);
+        const SlopeP<T> A = convect<T>(e.U, an, ay, az);
+        const T S = an.a1 + ay.a2 + az.a3, sS = s * S, w = A.a0 + A.h * k5;
+        const T x0 = A.a0 + A.h * sv.z3 + sS;
+        const T x1 = s * (A.a1 + an.a0 + an.h * k5);
+        const T x2 = s * (A.a2 + ay.a0 + ay.h * k5);
+        const T x3 = s * (A.a3 + az.a0 + az.h * k5);
+        const T x4 = T(0.5) * (sv.z3 * w + k5 * sS);
+        const T ss = s * s;
+        const T c1 = s * (w + sS + T(2) * s * an.a1);
+        const T c4 = T(0.5) * k5 * (s * (A.a1 + an.a0 + an.h * k7));
+        B[0] += gm2 * x0;
+        B[1] += gm2 * x1;
+        B[2] += gm2 * x2;
+        B[3] += gm2 * x3;
+        B[4] += gm2 * x4 + (gm1 * ph.dK) * e.P;
+        Fe[0] += p2 * (x1 + U * x0);
+        Fe[1] += p2 * (c1 + U * x1);
+        Fe[2] += p2 * (ss * (an.a2 + ay.a1) + U * x2);
+        Fe[3] += p2 * (ss * (an.a3 + az.a1) + U * x3);
+        Fe[4] += p2 * (c4 + U * x4);
+    }
+    {
+        // the equilibrium's time slope (src/GKMflux.cpp:183-191): <psi'' (psi.a)> of the slopes of B is B
+        // itself but for the Prandtl-corrected energy component
+        const SlopeP<T> a = solve_pec<T>(B, e, sv);
+        const T w = a.a0 + a.h * k5, y4 = T(0.5) * sv.z3 * w;
+        Fe[0] += p1 * (B[1] + U * B[0]);
+        Fe[1] += p1 * (s * w + U * B[1]);
+        Fe[2] += p1 * (U * B[2]);
+        Fe[3] += p1 * (U * B[3]);
+        Fe[4] += p1 * (T(0.5) * k5 * B[1] + U * y4);
+        const T r = p0 * e.P;
+        Fe[0] += p0 * We[1];
+        Fe[1] += r;
+        Fe[4] += (T(0.5 * (K + 3)) * U) * r;
+    }
+    to_frame<T>(Fe, e.U, T(0.5) * (e.U[0] * e.U[0] + e.U[1] * e.U[1] + e.U[2] * e.U[2]));
+#pragma unroll
+    for (int i = 0; i < 5; i++) F[i] = Fe[i];
 }
 
-#endif
-
-// The flux the kernels run: the functional form where the tangential product
-// table exists (GKM_SHARED_YZ), else the reference's MCal form.
+// The flux the kernels run; the operation counter takes the reference's MCal form.
 template <class T, class Prov>
 GKM_HD void gks_flux(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, T F[5])
 {
-#if GKM_SHARED_YZ
-    gks_flux_tau<T>(in, tau0, dt, dx, ph, F);
-#else
+#if GKM_REFERENCE_FORM
     gks_flux_mcal<T>(in, tau0, dt, dx, ph, F);
+#else
+    gks_flux_peculiar<T>(in, tau0, dt, dx, ph, F);
 #endif
 }
 

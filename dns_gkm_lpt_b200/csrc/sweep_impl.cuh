@@ -41,16 +41,15 @@ __device__ __forceinline__ Strides strides(int nt)
     return {1, nt2, nt};                 // normal k; window (j, i)
 }
 
-// Tangential neighbour faces in window coordinates (da, db) and the scale of
-// the first tangential slope.  "N/S" feed the y-slot slope and "F/B" the
-// z-slot slope, as the reference pairs them (src/update.cpp:231-257,303-329,412-438).
+// Tangential neighbour faces in window coordinates (da, db): "N/S" feed the y-slot slope and
+// "F/B" the z-slot slope, as the reference pairs them (src/update.cpp:231-257,303-329,412-438; in
+// its y sweep N is the lower neighbour and the slope's factor negative, the same value).
 template <int DIR>
 struct Neigh {
-    static constexpr int Na = DIR == 0 ? 1 : (DIR == 1 ? -1 : 0);
+    static constexpr int Na = DIR == 2 ? 0 : 1;
     static constexpr int Nb = DIR == 2 ? 1 : 0;
     static constexpr int Fa = DIR == 2 ? 1 : 0;
     static constexpr int Fb = DIR == 2 ? 0 : 1;
-    static constexpr double ys = DIR == 1 ? -0.5 : 0.5;
 };
 
 template <int DIR, class T, int kWC>
@@ -64,21 +63,23 @@ struct SmemFace {
     __device__ __forceinline__ T WR(int q) const { return wf1[perm<DIR>(q) * kWC + c]; }
     __device__ __forceinline__ T Wl(int q) const { return rec[perm<DIR>(q) * kWC + c]; }
     __device__ __forceinline__ T Wr(int q) const { return rec[(5 + perm<DIR>(q)) * kWC + c]; }
-    __device__ __forceinline__ T DW(int v, int q) const
+    // slope vectors v = 0..5 (normal, first and second tangential; left, right) as a difference and
+    // its factor: one-sided over half a cell, central over two
+    __device__ __forceinline__ T dW(int v, int q) const
     {
         const int p = perm<DIR>(q);
         const T* l = rec + p * kWC;
         const T* r = rec + (5 + p) * kWC;
-        const T ys = T(Neigh<DIR>::ys);
         switch (v) {
-            case 0: return T(2) * (l[c] - wf[p * kWC + c]) * inv_dx;
-            case 1: return T(2) * (wf1[p * kWC + c] - r[c]) * inv_dx;
-            case 2: return ys * (l[cN] - l[cS]) * inv_dx;
-            case 3: return ys * (r[cN] - r[cS]) * inv_dx;
-            case 4: return T(0.5) * (l[cF] - l[cB]) * inv_dx;
-            default: return T(0.5) * (r[cF] - r[cB]) * inv_dx;
+            case 0: return l[c] - wf[p * kWC + c];
+            case 1: return wf1[p * kWC + c] - r[c];
+            case 2: return l[cN] - l[cS];
+            case 3: return r[cN] - r[cS];
+            case 4: return l[cF] - l[cB];
+            default: return r[cF] - r[cB];
         }
     }
+    __device__ __forceinline__ T scale(int v) const { return (v < 2 ? T(2) : T(0.5)) * inv_dx; }
 };
 
 // tau0 = mu(T) / p of a cell (src/update.cpp:276-278) with one division: Sutherland
