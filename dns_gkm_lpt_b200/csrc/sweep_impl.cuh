@@ -707,20 +707,24 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                         T pq[4];
 #pragma unroll
                         for (int q = 0; q < 4; q++) pq[q] = D[q][0] * D[q][1];
-                        const T p01 = pq[0] * pq[1], p23 = pq[2] * pq[3];
-                        const T inv = T(1) / (p01 * p23);
-                        const T i01 = p23 * inv, i23 = p01 * inv;   // 1 / p01, 1 / p23
+                        // times 2^-24 each: the product of the eight, 4^24 (eps + IS)^24, back to its
+                        // indicators' own size before it can overflow
+                        constexpr T k24 = T(1.0 / 16777216.0);
+                        const T p01 = k24 * (pq[0] * pq[1]), p23 = k24 * (pq[2] * pq[3]);
+                        const T inv = T(1.0 / 6.0 / 16777216.0) / (p01 * p23);
+                        const T i01 = p23 * inv, i23 = p01 * inv;   // 1 / (6 p01), 1 / (6 p23)
                         const T iq[4] = {pq[1] * i01, pq[0] * i01, pq[3] * i23, pq[2] * i23};
 #pragma unroll
                         for (int q = 0; q < 4; q++) {
-                            l[q] = N[q][0] * (D[q][1] * iq[q]);
-                            r[q] = N[q][1] * (D[q][0] * iq[q]);
+                            l[q] = s2[q * kWC + c] + N[q][0] * (D[q][1] * iq[q]);
+                            r[q] = s2[q * kWC + c] + N[q][1] * (D[q][0] * iq[q]);
                         }
                     }
                     const T pT = D[4][0] * D[4][1], plr = l[0] * r[0];
                     const T inv2 = T(1) / (pT * plr);
-                    const T iT = plr * inv2, ilr = pT * inv2;   // 1 / pT, 1 / (rho_l rho_r)
-                    const T Tl = N[4][0] * (D[4][1] * iT), Tr = N[4][1] * (D[4][0] * iT);
+                    const T iT = T(1.0 / 6.0) * (plr * inv2), ilr = pT * inv2;   // 1 / (6 pT), 1 / (rho_l rho_r)
+                    const T Tc = s2[5 * kWC + c];
+                    const T Tl = Tc + N[4][0] * (D[4][1] * iT), Tr = Tc + N[4][1] * (D[4][0] * iT);
                     l[4] = face_energy_ir<T>(l[0], r[0] * ilr, l[1], l[2], l[3], Tl, ph);
                     r[4] = face_energy_ir<T>(r[0], l[0] * ilr, r[1], r[2], r[3], Tr, ph);
                 }
