@@ -755,15 +755,61 @@ GKM_HD Prim<T> prim(const T W[5], T gm1)
     return p;
 }
 
-// <1> and <c> over the half space u > 0 (half > 0) or u < 0: J_0 = erfc(-+ sqrt(lam) U)/2 and
-// J_1 = +- exp(-lam U^2) / (2 sqrt(pi lam)), with sqrt(s) from one reciprocal square root
+// Horner's rule, c[0] + c[1] t + ..
+template <class T, int N>
+GKM_HD T horner(const double (&c)[N], T t)
+{
+    T r = T(c[N - 1]);
+#pragma unroll
+    for (int k = N - 2; k >= 0; k--) r = r * t + T(c[k]);
+    return r;
+}
+
+// exp(-x^2/2) and erf(x/sqrt(2))/2 for x^2 <= 2 as polynomials in t = x^2: the interpolants of
+// exp(-t/2) and erf(sqrt(t/2)) / (2 sqrt(t)) at the Chebyshev points of [0, 2] (degrees 12 and 11:
+// within 8e-18 of the functions, relative; erf of degree 6 in single precision: 1.4e-9)
+template <class T>
+GKM_HD void gauss_small(T x, T t, T& ex, T& herf)
+{
+    if constexpr (single_t<T>::value) {
+        const double q[7] = {0.39894227996049447, -0.066490358435689789, 0.0099733829240630997, -0.001186799713508448,
+                            0.00011466371578999978, -8.8574673457925686e-06, 4.3508473942210419e-07};
+        ex = exp_t<T>(T(-0.5) * t);
+        herf = x * horner<T>(q, t);
+    } else {
+        const double p[13] = {1, -0.4999999999999995, 0.12499999999998568, -0.020833333333175521,
+                            0.0026041666657620841, -0.00026041666357754114, 2.1701382107946786e-05, -1.5500892124483604e-06,
+                            9.6871088514534077e-08, -5.3752300794789401e-09, 2.657581414044206e-10, -1.1184386854931272e-11,
+                            3.1052342897486384e-13};
+        const double q[12] = {0.3989422804014327, -0.066490380066905067, 0.0099735570100268726, -0.0011873282153967736,
+                            0.00011543468721120926, -9.444655101548686e-06, 6.659672481574838e-07, -4.1224151072896811e-08,
+                            2.271501082181806e-09, -1.1192508602593551e-10, 4.7370852926482607e-12, -1.3458332338909829e-13};
+        ex = horner<T>(p, t);
+        herf = x * horner<T>(q, t);
+    }
+}
+
+// <1> and <c> over the half space u > 0 (half > 0) or u < 0: J_0 = erfc(-+ x/sqrt(2))/2 and
+// J_1 = +- sqrt(s / (2 pi)) exp(-x^2/2), x = U / sqrt(s), with sqrt(s) from one reciprocal square
+// root.  Normal velocities up to sqrt(2 s) (Mach 1.2) take the polynomials: erfc and exp of the
+// library cost 105 and 28 FP64 issue slots each, the two polynomials 24 together (256^3 step,
+// default shapes: FP64 13.00 -> 12.06 ms, mixed 8.05 -> 7.91 ms).
 template <class T>
 GKM_HD void half_space(const Prim<T>& p, int half, T& J0, T& g)
 {
-    const T rs = rsqrt_t<T>(p.is);                                    // sqrt(s)
-    const T x = p.U[0] * (p.is * rs) * T(0.70710678118654752440);     // sqrt(lam) U
-    const T e = T(0.39894228040143267794) * exp_t<T>(-x * x) * rs;    // sqrt(s / (2 pi)) exp(-lam U^2)
-    J0 = T(0.5) * erfc_t<T>(half > 0 ? -x : x);
+    const T rs = rsqrt_t<T>(p.is);   // sqrt(s)
+    const T x = p.U[0] * (p.is * rs), t = x * x;
+    T ex;
+    if (t <= T(2)) {
+        T herf;
+        gauss_small<T>(x, t, ex, herf);
+        J0 = half > 0 ? T(0.5) + herf : T(0.5) - herf;
+    } else {
+        const T y = x * T(0.70710678118654752440);
+        ex = exp_t<T>(-y * y);
+        J0 = T(0.5) * erfc_t<T>(half > 0 ? -y : y);
+    }
+    const T e = (T(0.39894228040143267794) * rs) * ex;
     g = half > 0 ? e : -e;
 }
 
