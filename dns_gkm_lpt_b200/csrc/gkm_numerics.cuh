@@ -73,9 +73,9 @@ struct Phys {
     T Rg;         // gas constant in the working units
     int K;        // internal degrees of freedom (int((5-3g)/(g-1)))
     T iK3 = T(1) / T(K + 3);
-    // what the energy of a Maxwellian with K internal degrees of freedom exceeds p / (gam - 1) by, over p:
-    // zero but for rounding where (5-3g)/(g-1) is whole
-    T dK = T(0.5 * (K + 3)) - T(1) / gm1;
+    // twice what the energy of a Maxwellian with K internal degrees of freedom exceeds p / (gam - 1) by,
+    // over p: zero but for rounding where (5-3g)/(g-1) is whole
+    T dK2 = T(K + 3) - T(2) / gm1;
 };
 
 // ---------------------------------------------------------------- WENO ----
@@ -474,17 +474,12 @@ struct TimeCoefs {
 };
 
 // BGK time integrals over [0, dt] with e = exp(-dt/tau) (src/GKMflux.cpp:162-167,197-204).
-// EXPM1: 1 - e as -expm1(-dt/tau), exact where dt/tau is small (the mixed form,
-// whose flux runs in FP32 and gets these FP64 coefficients); otherwise the
-// reference's 1 - e.
-template <class D, bool EXPM1 = false>
+template <class D>
 GKM_HD TimeCoefs<D> time_coefs(D tau, D dt)
 {
     TimeCoefs<D> c;
     D ex = exp_t<D>(-dt / tau);
-    D omx;
-    if constexpr (EXPM1) omx = -expm1(-dt / tau);
-    else omx = D(1) - ex;
+    D omx = D(1) - ex;
     D gm0 = dt - tau * omx;
     D igm0 = D(1) / gm0;
     c.gm1 = -omx * igm0;
@@ -545,7 +540,7 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
 
     // collision time with the pressure-jump correction, src/GKMflux.cpp:156-157
     T ql = denl / laml, qr = denr / lamr;
-    const TimeCoefs<wide_t<T>> tc = time_coefs<wide_t<T>, (sizeof(T) < sizeof(wide_t<T>))>(
+    const TimeCoefs<wide_t<T>> tc = time_coefs<wide_t<T>>(
         wide_t<T>(tau0) + wide_t<T>(dt) * wide_t<T>(fabs(ql - qr) / fabs(ql + qr)), wide_t<T>(dt));
     const T gm1 = T(tc.gm1), gm2 = T(tc.gm2), gm3 = T(tc.gm3), gm4 = T(tc.gm4), gm5 = T(tc.gm5);
     const T p0 = T(tc.p0), p1 = T(tc.p1), p2 = T(tc.p2), p3 = T(tc.p3), p4 = T(tc.p4), p5 = T(tc.p5);
@@ -691,7 +686,7 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
 // the equilibrium state's by psi_e = T(U - U_e) psi'' (to_frame), where the equilibrium's slopes
 // are solved, and the summed flux to the laboratory frame at the end.  The reference's
 // gamma_1 (moments of the equilibrium) + gamma_3 (its conserved state), gamma_3 = -gamma_1, has
-// an energy component only, gamma_1 p dK (Phys).  About 900 operations per face beside the divisions and
+// an energy component only, gamma_1 p dK2 / 2 (Phys).  About 900 operations per face beside the divisions and
 // the special functions, where the moments in the laboratory frame took about 2,000; the sweeps
 // are bound by the FP64 (mixed: FP32) arithmetic.  Measured at 256^3 with the default shapes: a step
 // 18.00 -> 13.97 ms in FP64, 10.62 -> 8.26 ms in the mixed form; errors against extended precision
@@ -827,7 +822,11 @@ GKM_HD void half_moments(T* J, T J0, T g, T U, T s)
     }
 }
 
-// one slope vector in the peculiar frame of its state: psi.a = a0 + a1 c + a2 v' + a3 w' + 2 h psi4''
+// Below, psi'' is taken with its last component doubled, c^2 + v'^2 + w'^2 + xi^2, which spares the
+// halves; its moments are halved once, in the flux.
+
+// one slope vector in the peculiar frame of its state:
+// psi.a = a0 + a1 c + a2 v' + a3 w' + h (c^2 + v'^2 + w'^2 + xi^2)
 template <class T>
 struct SlopeP {
     T a0, a1, a2, a3, h;
@@ -868,7 +867,7 @@ template <class T>
 GKM_HD SlopeP<T> solve_pec(const T b[5], const Prim<T>& p, const SolveP<T>& c)
 {
     SlopeP<T> a;
-    a.h = c.hf * (b[4] - (T(0.5) * c.z3) * b[0]);
+    a.h = (T(0.5) * c.hf) * (b[4] - c.z3 * b[0]);
     a.a1 = p.is * b[1];
     a.a2 = p.is * b[2];
     a.a3 = p.is * b[3];
@@ -876,21 +875,32 @@ GKM_HD SlopeP<T> solve_pec(const T b[5], const Prim<T>& p, const SolveP<T>& c)
     return a;
 }
 
-// moments in a frame moving with U -> the frame moving with U - d: psi -> T(d) psi, hd = |d|^2/2
+// acc += w o with o taken from a frame moving with U to the frame moving with U - d:
+// psi -> T(d) psi, d2 = 2 d, dd = |d|^2
 template <class T>
-GKM_HD void to_frame(T o[5], const T d[3], T hd)
+GKM_HD void add_in_frame(T acc[5], T w, const T o[5], const T d[3], const T d2[3], T dd)
 {
-    o[4] += d[0] * o[1] + d[1] * o[2] + d[2] * o[3] + hd * o[0];
-    o[1] += d[0] * o[0];
-    o[2] += d[1] * o[0];
-    o[3] += d[2] * o[0];
+    acc[0] += w * o[0];
+    acc[1] += w * (o[1] + d[0] * o[0]);
+    acc[2] += w * (o[2] + d[1] * o[0]);
+    acc[3] += w * (o[3] + d[2] * o[0]);
+    acc[4] += w * (o[4] + d2[0] * o[1] + d2[1] * o[2] + d2[2] * o[3] + dd * o[0]);
+}
+template <class T>
+GKM_HD void add_in_frame(T acc[5], const T o[5], const T d[3], const T d2[3], T dd)
+{
+    acc[0] += o[0];
+    acc[1] = (acc[1] + o[1]) + d[0] * o[0];
+    acc[2] = (acc[2] + o[2]) + d[1] * o[0];
+    acc[3] = (acc[3] + o[3]) + d[2] * o[0];
+    acc[4] = (acc[4] + o[4]) + (d2[0] * o[1] + d2[1] * o[2] + d2[2] * o[3] + dd * o[0]);
 }
 
-// <psi'' (psi.a)> with the normal weight N_k (N = J: weight 1; N = L: weight u)
+// <psi'' (psi.a)> with the normal weight N_k (N = J: weight 1; N = L: weight u); z1 = (K+2) s = <zeta>
 template <class T>
-GKM_HD void half_P(T o[5], const T* N, const SlopeP<T>& a, T s, T hz1)
+GKM_HD void half_P(T o[5], const T* N, const SlopeP<T>& a, T s, T z1)
 {
-    const T hz = a.h * (hz1 + hz1);            // h <zeta>
+    const T hz = a.h * z1;
     const T t = a.a0 + hz;
     const T s0 = t * N[0] + a.a1 * N[1] + a.h * N[2];
     const T s1 = t * N[1] + a.a1 * N[2] + a.h * N[3];
@@ -900,30 +910,30 @@ GKM_HD void half_P(T o[5], const T* N, const SlopeP<T>& a, T s, T hz1)
     o[1] = s1;
     o[2] = sn * a.a2;
     o[3] = sn * a.a3;
-    o[4] = hz1 * s0 + T(0.5) * s2 + sn * hz;
+    o[4] = z1 * s0 + (s2 + (sn + sn) * hz);
 }
 
 // the same with weights 1 and u (o and p) over one table
 template <class T>
-GKM_HD void half_P2(T o[5], T p[5], const T* N, const SlopeP<T>& a, T s, T U, T hz1)
+GKM_HD void half_P2(T o[5], T p[5], const T* N, const SlopeP<T>& a, T s, T U, T z1)
 {
-    const T hz = a.h * (hz1 + hz1);
+    const T hz = a.h * z1;
     const T t = a.a0 + hz;
     const T s0 = t * N[0] + a.a1 * N[1] + a.h * N[2];
     const T s1 = t * N[1] + a.a1 * N[2] + a.h * N[3];
     const T s2 = t * N[2] + a.a1 * N[3] + a.h * N[4];
     const T s3 = t * N[3] + a.a1 * N[4] + a.h * N[5];
-    const T sn = s * N[0], sm = s * (N[1] + U * N[0]);
+    const T sn = s * N[0], sm = s * N[1] + U * sn;
     o[0] = s0;
     o[1] = s1;
     o[2] = sn * a.a2;
     o[3] = sn * a.a3;
-    o[4] = hz1 * s0 + T(0.5) * s2 + sn * hz;
+    o[4] = z1 * s0 + (s2 + (sn + sn) * hz);
     p[0] = s1 + U * s0;
     p[1] = s2 + U * s1;
     p[2] = sm * a.a2;
     p[3] = sm * a.a3;
-    p[4] = hz1 * p[0] + T(0.5) * (s3 + U * s2) + sm * hz;
+    p[4] = z1 * p[0] + ((s3 + U * s2) + (sm + sm) * hz);
 }
 
 // the convective part of G: A = U a_n + V a_y + W a_z
@@ -942,32 +952,32 @@ GKM_HD SlopeP<T> convect(const T U[3], const SlopeP<T>& n, const SlopeP<T>& y, c
 // <psi'' G> with weights 1 and u (o and p) over the half space of J
 template <class T>
 GKM_HD void half_G(T o[5], T p[5], const T* J, const SlopeP<T>& A, const SlopeP<T>& n, const SlopeP<T>& y,
-                   const SlopeP<T>& z, T s, T U, T hz1, T k4)
+                   const SlopeP<T>& z, T s, T U, T z1, T k4)
 {
-    // <G>_tan = c0 + c1 c + c2 c^2 + c3 c^3, <zeta G>_tan / 2 = hz1 <G>_tan + s (y0 + y1 c)
-    const T z1 = hz1 + hz1;
+    // <G>_tan = c0 + c1 c + c2 c^2 + c3 c^3, <zeta G>_tan = z1 <G>_tan + 2 s (y0 + y1 c)
     const T y0 = A.h * z1 + s * (y.a2 + z.a3), y1 = n.h * z1;
-    const T c0 = A.a0 + y0, c1 = A.a1 + n.a0 + y1, c2 = A.h + n.a1, c3 = n.h;
+    const T c0 = A.a0 + y0, c1 = (A.a1 + n.a0) + y1, c2 = A.h + n.a1, c3 = n.h;
     const T s0 = c0 * J[0] + c1 * J[1] + c2 * J[2] + c3 * J[3];
     const T s1 = c0 * J[1] + c1 * J[2] + c2 * J[3] + c3 * J[4];
     const T s2 = c0 * J[2] + c1 * J[3] + c2 * J[4] + c3 * J[5];
     const T s3 = c0 * J[3] + c1 * J[4] + c2 * J[5] + c3 * J[6];
     // <v' G>_tan = s (v0 + v1 c + h_y c^2), <w' G>_tan likewise
-    const T v0 = A.a2 + y.a0 + y.h * k4, v1 = n.a2 + y.a1;
-    const T w0 = A.a3 + z.a0 + z.h * k4, w1 = n.a3 + z.a1;
+    const T v0 = (A.a2 + y.a0) + y.h * k4, v1 = n.a2 + y.a1;
+    const T w0 = (A.a3 + z.a0) + z.h * k4, w1 = n.a3 + z.a1;
     const T va = v0 * J[0] + v1 * J[1] + y.h * J[2], vb = v0 * J[1] + v1 * J[2] + y.h * J[3];
     const T wa = w0 * J[0] + w1 * J[1] + z.h * J[2], wb = w0 * J[1] + w1 * J[2] + z.h * J[3];
     const T ea = y0 * J[0] + y1 * J[1], eb = y0 * J[1] + y1 * J[2];
+    const T ss = s + s;
     o[0] = s0;
     o[1] = s1;
     o[2] = s * va;
     o[3] = s * wa;
-    o[4] = hz1 * s0 + T(0.5) * s2 + s * ea;
+    o[4] = z1 * s0 + (s2 + ss * ea);
     p[0] = s1 + U * s0;
     p[1] = s2 + U * s1;
     p[2] = s * (vb + U * va);
     p[3] = s * (wb + U * wa);
-    p[4] = hz1 * p[0] + T(0.5) * (s3 + U * s2) + s * (eb + U * ea);
+    p[4] = z1 * p[0] + ((s3 + U * s2) + ss * (eb + U * ea));
 }
 
 // a face provider may give raw differences and their common factors instead of slopes:
@@ -984,6 +994,45 @@ GKM_HD SlopeP<T> face_slope(const Prov& in, int v, const Prim<T>& p, const Solve
         return solve_lab<T>(in.dW(v, 0), in.dW(v, 1), in.dW(v, 2), in.dW(v, 3), in.dW(v, 4), in.scale(v), p, c);
     else
         return solve_lab<T>(in.DW(v, 0), in.DW(v, 1), in.DW(v, 2), in.DW(v, 3), in.DW(v, 4), T(1), p, c);
+}
+
+// The time integrals the peculiar form needs, from src/GKMflux.cpp:162-167,197-204 with
+// gm0 = dt - tau (1 - e), e = exp(-dt/tau), multiplied out: the slope of the equilibrium is solved
+// from gm0 B_, so the coefficients are
+//   of the sides  gm0 (gm4 + gm5) = dt e, gm0 gm5 = P, p3 = P, p4 = tau (dt e - 2 P), p5 = -tau P,
+//   of the rest   gm0 gm1 = -(1 - e), gm0 gm2 = h = 2 P - dt - dt e, p2 = tau h, p0 = gm0,
+//                 p1 / gm0 = dt^2 / (2 gm0) - tau,
+// with P = tau (1 - e).  They are formed in double precision whatever the flux runs in, as
+// differences of nearly equal terms where dt / tau is small.  EXPM1: 1 - e as -expm1(-dt/tau),
+// exact there (the mixed form); otherwise the reference's 1 - e.  Fewer values stay live across the
+// moments than with the reference's eleven coefficients, and the mixed form needs no FP64 exp: 256^3
+// step FP64 12.06 -> 11.99 ms, mixed 7.91 -> 7.78 ms.
+template <class T>
+struct RelaxCoefs {
+    T tau, omx, P, dte, h, p0, p1g;
+};
+template <class T, bool EXPM1>
+GKM_HD RelaxCoefs<T> relax_coefs(wide_t<T> tau, wide_t<T> dt)
+{
+    using D = wide_t<T>;
+    D e, omx;
+    if constexpr (EXPM1) {
+        omx = -expm1(-dt / tau);
+        e = D(1) - omx;
+    } else {
+        e = exp_t<D>(-dt / tau);
+        omx = D(1) - e;
+    }
+    const D P = tau * omx, dte = dt * e, gm0 = dt - P;
+    RelaxCoefs<T> c;
+    c.tau = T(tau);
+    c.omx = T(omx);
+    c.P = T(P);
+    c.dte = T(dte);
+    c.h = T((P - dt) + (P - dte));
+    c.p0 = T(gm0);
+    c.p1g = T(D(0.5) * dt * dt / gm0 - tau);
+    return c;
 }
 
 // The flux of gks_flux_mcal with every moment taken in the peculiar frames.  The slopes of a side
@@ -1007,11 +1056,8 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
     }
     // collision time with the pressure-jump correction, src/GKMflux.cpp:156-157:
     // |rho_l/lam_l - rho_r/lam_r| / |rho_l/lam_l + rho_r/lam_r| with rho/lam = 2 p (p > 0)
-    const TimeCoefs<wide_t<T>> tc = time_coefs<wide_t<T>, (sizeof(T) < sizeof(wide_t<T>))>(
+    const RelaxCoefs<T> rc = relax_coefs<T, (sizeof(T) < sizeof(wide_t<T>))>(
         wide_t<T>(tau0) + wide_t<T>(dt) * wide_t<T>(fabs(st[0].P - st[1].P) * inv_psum), wide_t<T>(dt));
-    const T gm1 = T(tc.gm1), gm2 = T(tc.gm2), gm4 = T(tc.gm4), gm5 = T(tc.gm5);
-    const T p0 = T(tc.p0), p1 = T(tc.p1), p2 = T(tc.p2), p3 = T(tc.p3), p4 = T(tc.p4), p5 = T(tc.p5);
-    const T cB = gm4 + gm5;
 
     // the equilibrium state at the face (src/GKMflux.cpp:73-77), from both half-Maxwellians
     T We[5], J0[2], g[2];
@@ -1031,7 +1077,7 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
     const Prim<T> e = prim<T>(We, ph.gm1);
 
     // sums over the sides, in the equilibrium's frame: the tangential slopes of the equilibrium
-    // (times its density), rho_e B_ and the flux
+    // (times its density), gm0 rho_e B_ and the flux
     T by[5] = {0, 0, 0, 0, 0}, bz[5] = {0, 0, 0, 0, 0}, B[5] = {0, 0, 0, 0, 0}, Fe[5] = {0, 0, 0, 0, 0};
     // ---------------- one side (l: positive half with left state, r: negative half with right state)
 #if GKM_UNROLL_SIDES
@@ -1042,63 +1088,58 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
     for (int side = 0; side < 2; side++) {
         const Prim<T> p = side == 0 ? st[0] : st[1];
         const T s = p.s, U = p.U[0];
-        const T hz1 = T(0.5 * (K + 2)) * s, k4 = T(K + 4) * s;
+        const T z1 = T(K + 2) * s, k4 = T(K + 4) * s;
         const SolveP<T> sv = solve_consts<T>(p, iK3, K);
         const T d[3] = {U - e.U[0], p.U[1] - e.U[1], p.U[2] - e.U[2]};
-        const T hd = T(0.5) * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+        const T d2[3] = {d[0] + d[0], d[1] + d[1], d[2] + d[2]};
+        const T dd = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
         T J[7];
         half_moments<T, 7>(J, side == 0 ? J0[0] : J0[1], side == 0 ? g[0] : g[1], U, s);
         const T wy = e.den * p.ir;
         T o[5], q[5];
         const SlopeP<T> ay = face_slope<T>(in, 2 + side, p, sv);
-        half_P<T>(o, J, ay, s, hz1);
-        to_frame<T>(o, d, hd);
-        axpy5<T>(by, wy, o);
+        half_P<T>(o, J, ay, s, z1);
+        add_in_frame<T>(by, wy, o, d, d2, dd);
         const SlopeP<T> az = face_slope<T>(in, 4 + side, p, sv);
-        half_P<T>(o, J, az, s, hz1);
-        to_frame<T>(o, d, hd);
-        axpy5<T>(bz, wy, o);
+        half_P<T>(o, J, az, s, z1);
+        add_in_frame<T>(bz, wy, o, d, d2, dd);
         const SlopeP<T> an = face_slope<T>(in, side, p, sv);
         const SlopeP<T> A = convect<T>(p.U, an, ay, az);
-        half_G<T>(o, q, J, A, an, ay, az, s, U, hz1, k4);
-        // this side's time slope (src/GKMflux.cpp:145-151): the slopes of -<psi G> over the full space
+        half_G<T>(o, q, J, A, an, ay, az, s, U, z1, k4);
+        // this side's time slope (src/GKMflux.cpp:145-151) with its sign changed: the slopes of
+        // <psi G> over the full space
         const T S = an.a1 + ay.a2 + az.a3, k5 = T(K + 5) * s;
         SlopeP<T> at;
-        at.h = T(-1.0 / kPrandtl) * (A.h + iK3 * S);
-        at.a1 = -(A.a1 + an.a0 + an.h * k5);
-        at.a2 = -(A.a2 + ay.a0 + ay.h * k5);
-        at.a3 = -(A.a3 + az.a0 + az.h * k5);
-        at.a0 = -(A.a0 + s * S + (A.h + at.h) * sv.z3);
+        at.h = T(1.0 / kPrandtl) * (A.h + iK3 * S);
+        at.a1 = (A.a1 + an.a0) + an.h * k5;
+        at.a2 = (A.a2 + ay.a0) + ay.h * k5;
+        at.a3 = (A.a3 + az.a0) + az.h * k5;
+        at.a0 = (A.a0 + s * S) + (A.h - at.h) * sv.z3;
+        T x[5], y[5];
+        half_P2<T>(x, y, J, at, s, U, z1);
+        const T dte = rc.dte, P = rc.P, p5 = rc.tau * P, p4 = rc.tau * dte - (p5 + p5);
 #pragma unroll
         for (int i = 0; i < 5; i++) {
-            o[i] *= cB;
-            q[i] *= p4;
+            o[i] = dte * o[i] - P * x[i];
+            q[i] = p4 * q[i] + p5 * y[i];
         }
-        T x[5], y[5];
-        half_P2<T>(x, y, J, at, s, U, hz1);
-        axpy5<T>(o, gm5, x);
-        axpy5<T>(q, p5, y);
         // free transport of the initial half-Maxwellian: rho <u psi''>
         {
-            const T r = p3 * p.den;
+            const T r = P * p.den;
             const T m0 = r * (J[1] + U * J[0]), m1 = r * (J[2] + U * J[1]);
             q[0] += m0;
             q[1] += m1;
-            q[4] += hz1 * m0 + T(0.5) * (r * (J[3] + U * J[2]));
+            q[4] += z1 * m0 + r * (J[3] + U * J[2]);
         }
-        to_frame<T>(o, d, hd);
-        to_frame<T>(q, d, hd);
-#pragma unroll
-        for (int i = 0; i < 5; i++) {
-            B[i] += o[i];
-            Fe[i] += q[i];
-        }
+        add_in_frame<T>(B, o, d, d2, dd);
+        add_in_frame<T>(Fe, q, d, d2, dd);
     }
 
     // ---------------- equilibrium part, in its own frame
     const T s = e.s, U = e.U[0];
-    const T hz1 = T(0.5 * (K + 2)) * s, k5 = T(K + 5) * s, k7 = T(K + 7) * s;
+    const T z1 = T(K + 2) * s, k5 = T(K + 5) * s, k7 = T(K + 7) * s;
     const SolveP<T> sv = solve_consts<T>(e, iK3, K);
+    const T h = rc.h, p2 = rc.tau * h;
     // normal slopes from the cell averages (src/GKMflux.cpp:115-116), left minus right and right:
     // <P_l>_{u>0} + <P_r>_{u<0} = <P_l - P_r>_{u>0} + <P_r>
     const T idx2 = T(2) / dx;
@@ -1116,8 +1157,8 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
 #pragma unroll
         for (int k = 0; k < 6; k++) L[k] = J[k + 1] + U * J[k];   // <u c^k>
         const SlopeP<T> ad = solve_lab<T>(bd[0], bd[1], bd[2], bd[3], bd[4], idx2, e, sv);
-        half_P2<T>(o, q, L, ad, s, U, hz1);
-        axpy5<T>(B, gm2, o);
+        half_P2<T>(o, q, L, ad, s, U, z1);
+        axpy5<T>(B, h, o);
         axpy5<T>(Fe, p2, q);
     }
     {
@@ -1126,19 +1167,19 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
         const SlopeP<T> ay = solve_pec<T>(by, e, sv), az = solve_pec<T>(bz, e, sv);
         const SlopeP<T> A = convect<T>(e.U, an, ay, az);
         const T S = an.a1 + ay.a2 + az.a3, sS = s * S, w = A.a0 + A.h * k5;
-        const T x0 = A.a0 + A.h * sv.z3 + sS;
-        const T x1 = s * (A.a1 + an.a0 + an.h * k5);
-        const T x2 = s * (A.a2 + ay.a0 + ay.h * k5);
-        const T x3 = s * (A.a3 + az.a0 + az.h * k5);
-        const T x4 = T(0.5) * (sv.z3 * w + k5 * sS);
+        const T x0 = (A.a0 + sS) + A.h * sv.z3;
+        const T x1 = s * ((A.a1 + an.a0) + an.h * k5);
+        const T x2 = s * ((A.a2 + ay.a0) + ay.h * k5);
+        const T x3 = s * ((A.a3 + az.a0) + az.h * k5);
+        const T x4 = sv.z3 * w + k5 * sS;
         const T ss = s * s;
-        const T c1 = s * (w + sS + T(2) * s * an.a1);
-        const T c4 = T(0.5) * k5 * (s * (A.a1 + an.a0 + an.h * k7));
-        B[0] += gm2 * x0;
-        B[1] += gm2 * x1;
-        B[2] += gm2 * x2;
-        B[3] += gm2 * x3;
-        B[4] += gm2 * x4 + (gm1 * ph.dK) * e.P;
+        const T c1 = s * ((w + sS) + (s + s) * an.a1);
+        const T c4 = k5 * (s * ((A.a1 + an.a0) + an.h * k7));
+        B[0] += h * x0;
+        B[1] += h * x1;
+        B[2] += h * x2;
+        B[3] += h * x3;
+        B[4] += h * x4 - (rc.omx * ph.dK2) * e.P;
         Fe[0] += p2 * (x1 + U * x0);
         Fe[1] += p2 * (c1 + U * x1);
         Fe[2] += p2 * (ss * (an.a2 + ay.a1) + U * x2);
@@ -1149,20 +1190,24 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
         // the equilibrium's time slope (src/GKMflux.cpp:183-191): <psi'' (psi.a)> of the slopes of B is B
         // itself but for the Prandtl-corrected energy component
         const SlopeP<T> a = solve_pec<T>(B, e, sv);
-        const T w = a.a0 + a.h * k5, y4 = T(0.5) * sv.z3 * w;
+        const T w = a.a0 + a.h * k5, p1 = rc.p1g;
         Fe[0] += p1 * (B[1] + U * B[0]);
         Fe[1] += p1 * (s * w + U * B[1]);
         Fe[2] += p1 * (U * B[2]);
         Fe[3] += p1 * (U * B[3]);
-        Fe[4] += p1 * (T(0.5) * k5 * B[1] + U * y4);
-        const T r = p0 * e.P;
-        Fe[0] += p0 * We[1];
+        Fe[4] += p1 * (k5 * B[1] + U * (sv.z3 * w));
+        const T r = rc.p0 * e.P;
+        Fe[0] += rc.p0 * We[1];
         Fe[1] += r;
-        Fe[4] += (T(0.5 * (K + 3)) * U) * r;
+        Fe[4] += (T(K + 3) * U) * r;
     }
-    to_frame<T>(Fe, e.U, T(0.5) * (e.U[0] * e.U[0] + e.U[1] * e.U[1] + e.U[2] * e.U[2]));
-#pragma unroll
-    for (int i = 0; i < 5; i++) F[i] = Fe[i];
+    // to the laboratory frame
+    F[0] = Fe[0];
+    F[1] = Fe[1] + U * Fe[0];
+    F[2] = Fe[2] + e.U[1] * Fe[0];
+    F[3] = Fe[3] + e.U[2] * Fe[0];
+    F[4] = T(0.5) * Fe[4] + U * Fe[1] + e.U[1] * Fe[2] + e.U[2] * Fe[3] +
+           (T(0.5) * (U * U + e.U[1] * e.U[1] + e.U[2] * e.U[2])) * Fe[0];
 }
 
 // The flux the kernels run; the operation counter takes the reference's MCal form.
