@@ -55,8 +55,16 @@ struct SweepTile {
 // FP64: 16 x 8 (255 registers, two 128-thread CTAs per SM) and 16 x 16 (one 256-thread CTA)
 using SweepTile64a = SweepTile<16, 8, 2>;
 using SweepTile64b = SweepTile<16, 16, 1>;
-// FP32: 16 x 8 (168 registers, three CTAs per SM)
-using SweepTile32a = SweepTile<16, 8, 3>;
+// FP32: 16 x 8; CTAs per SM: four in the x and y sweeps (128 registers), three in the z sweep, whose
+// landing area and bricks take 68 KB of shared memory (168 registers).  256^3 / 512^3, ms, three CTAs
+// against four: x 1.536 / 11.86 -> 1.522 / 11.30, y 1.688 / 13.14 -> 1.651 / 12.36, z 1.969 / 14.77 -> 2.117 /
+// 15.45 (128 registers without the fourth CTA)
+using SweepTile32a = SweepTile<16, 8, 4>;
+template <int DIR, class T, class Tile>
+constexpr int sweep_ctas()
+{
+    return sizeof(T) == 4 && DIR == 2 ? 3 : Tile::ctas;
+}
 // variant 2: 16 x 16 windows, warp-specialized (a producer warpgroup reconstructs face f+1 while
 // two consumer warpgroups compute the fluxes of face f; sweep_ws.cuh); ensembles: its persistent
 // form for x and y

@@ -42,12 +42,6 @@
 #define GKM_REFERENCE_FORM 0
 #endif
 
-// Code shape of the flux: both half-Maxwellian sides unrolled (one copy of the
-// side code per side) or one loop body.
-#ifndef GKM_UNROLL_SIDES
-#define GKM_UNROLL_SIDES 1
-#endif
-
 namespace gkm {
 
 // single-precision arithmetic: float, and the packed pair F2 (f32x2.cuh)
@@ -553,11 +547,7 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
 
     const T cB = gm4 + gm5;
     // ---------------- one side (l: positive half with left state, r: negative half with right state)
-#if GKM_UNROLL_SIDES
 #pragma unroll
-#else
-#pragma unroll 1
-#endif
     for (int side = 0; side < 2; side++) {
         const T den = side == 0 ? denl : denr;
         const T* Us = side == 0 ? Ul : Ur;
@@ -1080,11 +1070,7 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
     // (times its density), gm0 rho_e B_ and the flux
     T by[5] = {0, 0, 0, 0, 0}, bz[5] = {0, 0, 0, 0, 0}, B[5] = {0, 0, 0, 0, 0}, Fe[5] = {0, 0, 0, 0, 0};
     // ---------------- one side (l: positive half with left state, r: negative half with right state)
-#if GKM_UNROLL_SIDES
 #pragma unroll
-#else
-#pragma unroll 1
-#endif
     for (int side = 0; side < 2; side++) {
         const Prim<T> p = side == 0 ? st[0] : st[1];
         const T s = p.s, U = p.U[0];

@@ -902,7 +902,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
 }
 
 template <int DIR, class T, class Tile, int MM = kMapsRuntime>
-__global__ void __launch_bounds__(Tile::threads, Tile::ctas) sweep_kernel(SweepArgs a)
+__global__ void __launch_bounds__(Tile::threads, (sweep_ctas<DIR, T, Tile>())) sweep_kernel(SweepArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     sweep_block<DIR, T, Tile, MM>(a, blockIdx.x, blockIdx.y + a.tile_a0, blockIdx.z, smem_raw);
@@ -978,7 +978,7 @@ __device__ __forceinline__ void ensemble_item(const MemberDev* __restrict__ mem,
 // m uses segments of md.seg_len[DIR] faces; the list holds the members in the
 // order order[] (longest items first), off[] their work-item offsets.
 template <int DIR, class T, class Tile>
-__global__ void __launch_bounds__(Tile::threads, Tile::ctas)
+__global__ void __launch_bounds__(Tile::threads, (sweep_ctas<DIR, T, Tile>()))
     ensemble_sweep_kernel(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
                           const long long* __restrict__ order, int nm, int parity, unsigned long long* next)
 {
@@ -1028,7 +1028,7 @@ cudaError_t launch_ensemble_sweep_t(int dir, const MemberDev* mem, const long lo
                                     int parity, unsigned long long* next, cudaStream_t s)
 {
     const dim3 block(Tile::TB, Tile::TA);
-    const int grid = 148 * Tile::ctas;
+    const int grid = 148 * (dir == 2 ? sweep_ctas<2, T, Tile>() : Tile::ctas);
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
     if (dir == 0)

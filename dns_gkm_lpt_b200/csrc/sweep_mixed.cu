@@ -6,9 +6,7 @@
 //
 // Compiled with fast single-precision math (-use_fast_math: approximate
 // division, square root and exp, denormals flushed; the FP64 arithmetic of
-// this file is unaffected by that flag) and with the flux's two half-Maxwellian
-// sides as one loop body (-DGKM_UNROLL_SIDES=0), the faster code shape for
-// the single-precision flux.
+// this file is unaffected by that flag).
 #include "sweep_impl.cuh"
 
 namespace gkm {
