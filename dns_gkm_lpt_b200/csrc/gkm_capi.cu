@@ -8,6 +8,7 @@
 // buffer parity.
 #include "gkm.h"
 #include "gkm_handle.h"
+#include "gkm_numerics.cuh"
 
 #include <cuda.h>   // CUtensorMap and its enums (the encoder comes from the driver at run time)
 
@@ -520,6 +521,15 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     fc.fscale[0] = P.den0 * fc.dx;
     fc.fscale[1] = fc.fscale[2] = fc.fscale[3] = P.den0 * fc.u_s * fc.dx;
     fc.fscale[4] = P.p0 * fc.dx;
+    fc.k2 = K + 2;
+    fc.k3 = K + 3;
+    fc.k4 = K + 4;
+    fc.k5 = K + 5;
+    fc.k7 = K + 7;
+    fc.iK3 = 1.0 / (K + 3);
+    fc.iPrK3 = (1.0 / gkm::kPrandtl) * fc.iK3;
+    fc.dK2 = (K + 3) - 2.0 / fc.gm1;
+    fc.suth_c = fc.mu0 * (fc.T0 + 110.4) * gkm::kR / ((gkm::kR * fc.T0) * std::sqrt(gkm::kR * fc.T0));
 
     for (int d = 0; d < 3; d++) h->sweep[d] = default_choice(fc, cfg->precision == GKM_PREC_MIXED, 0);
 

@@ -60,13 +60,42 @@ constexpr double kR = 287.0;        // gas constant, src/param.h:21
 constexpr double kPrandtl = 0.70;   // src/param.h:19
 constexpr double kWenoEps = 1e-10;  // pow(10,-10), src/param.h:18
 
+// 1/x.  In double precision on the device the hardware's approximate reciprocal (20 bits) with one
+// third-order step in fused multiply-adds, r + r (e + e^2), e = 1 - x r (Newton's iteration carried one
+// term further): within an ulp for normal x and 1/x, four dependent instructions and no branch, where
+// a division takes about ten and a branch.  Zero and infinite x give NaN.  The sweeps wait on these
+// chains (256^3 FP64 step 11.99 -> 11.08 ms, with the reciprocal square roots and the constants of K
+// taken from the launch).
+template <class T>
+GKM_HD T recip(T x)
+{
+    return T(1) / x;
+}
+#ifdef __CUDACC__
+template <>
+GKM_HD double recip<double>(double x)
+{
+#ifdef __CUDA_ARCH__
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+#else
+    return 1.0 / x;
+#endif
+}
+#endif
+
 template <class T>
 struct Phys {
     T gam;        // ratio of specific heats
     T gm1;        // gam - 1
     T Rg;         // gas constant in the working units
     int K;        // internal degrees of freedom (int((5-3g)/(g-1)))
-    T iK3 = T(1) / T(K + 3);
+    // K + 2 .. K + 7 and 1 / (Pr (K + 3)) as the flux uses them (the sweeps take them from the launch's
+    // constants, so they occupy no registers)
+    T k2 = T(K + 2), k3 = T(K + 3), k4 = T(K + 4), k5 = T(K + 5), k7 = T(K + 7);
+    T iK3 = T(1) / T(K + 3), iPrK3 = T(1.0 / kPrandtl) * (T(1) / T(K + 3));
     // twice what the energy of a Maxwellian with K internal degrees of freedom exceeds p / (gam - 1) by,
     // over p: zero but for rounding where (5-3g)/(g-1) is whole
     T dK2 = T(K + 3) - T(2) / gm1;
@@ -228,7 +257,7 @@ GKM_HD void weno_scalar(T a3, T a2, T a1, T b1, T b2, T b3, T eps, T& fl, T& fr)
         weno_nd<T>(a3, a2, a1, b1, b2, b3, eps, Nl, Dl, Nr, Dr);
         // both sides with one division: D ranges from about 80 (4 eps)^3 (flat stencil) to about
         // 64 IS_max^3, so Dl Dr stays far inside the double range for any physical state
-        const T inv = T(1.0 / 6.0) / (Dl * Dr);
+        const T inv = T(1.0 / 6.0) * recip<T>(Dl * Dr);
         fl = a1 + Nl * (Dr * inv);
         fr = a1 + Nr * (Dl * inv);
     }
@@ -239,10 +268,11 @@ GKM_HD void weno_scalar(T a3, T a2, T a1, T b1, T b2, T b3, T eps, T& fl, T& fr)
 template <class T>
 GKM_HD T temperature(T r, T m1, T m2, T m3, T E, const Phys<T>& ph)
 {
-    T ir = T(1) / r;
 #if GKM_REFERENCE_FORM
+    T ir = T(1) / r;
     return ph.gm1 * (E * ir - T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) * ir * ir) / ph.Rg;
 #else
+    const T ir = recip<T>(r);
     return (E * ir - T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) * ir * ir) * (ph.gm1 / ph.Rg);
 #endif
 }
@@ -254,7 +284,7 @@ GKM_HD T face_energy(T r, T m1, T m2, T m3, T Tf, const Phys<T>& ph)
 #if GKM_REFERENCE_FORM
     return r * ph.Rg * Tf / ph.gm1 + T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) / r;
 #else
-    return r * Tf * (ph.Rg / ph.gm1) + T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) / r;
+    return r * Tf * (ph.Rg / ph.gm1) + T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) * recip<T>(r);
 #endif
 }
 
@@ -296,14 +326,18 @@ template <>
 GKM_HD double sqrt_t<double>(double x) { return sqrt(x); }
 template <>
 GKM_HD float sqrt_t<float>(float x) { return sqrtf(x); }
-// 1 / sqrt(x): the device's reciprocal square root (within 1 ulp), on the host 1 / sqrt
+// 1 / sqrt(x) for normal x > 0, within 2 ulp; on the host 1 / sqrt
 template <class T>
 GKM_HD T rsqrt_t(T x);
 template <>
 GKM_HD double rsqrt_t<double>(double x)
 {
 #ifdef __CUDA_ARCH__
-    return rsqrt(x);
+    // as recip: r + r (e/2 + 3 e^2/8), e = 1 - x r^2
+    double r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x * r, r, 1.0);
+    return fma(r * e, fma(0.375, e, 0.5), r);
 #else
     return 1.0 / sqrt(x);
 #endif
@@ -700,7 +734,7 @@ GKM_HD void prim_pair(const T wl[5], const T wr[5], T gm1, Prim<T>& l, Prim<T>& 
     const T pdr = gm1 * (wr[4] * r.den - T(0.5) * (wr[1] * wr[1] + wr[2] * wr[2] + wr[3] * wr[3]));
     const T dd = l.den * r.den, pp = pdl * pdr;
     const T S = pdl * r.den + pdr * l.den;
-    const T inv = T(1) / ((dd * pp) * S);
+    const T inv = recip<T>((dd * pp) * S);
     const T ppS = pp * S * inv;   // 1 / dd
     l.ir = r.den * ppS;
     r.ir = l.den * ppS;
@@ -729,7 +763,7 @@ GKM_HD Prim<T> prim(const T W[5], T gm1)
     Prim<T> p;
     p.den = W[0];
     const T pd = gm1 * (W[4] * p.den - T(0.5) * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]));
-    const T inv = T(1) / (p.den * pd);
+    const T inv = recip<T>(p.den * pd);
     p.ir = pd * inv;
     p.U[0] = W[1] * p.ir;
     p.U[1] = W[2] * p.ir;
@@ -828,12 +862,12 @@ struct SolveP {
     T uq, z3, hf;
 };
 template <class T>
-GKM_HD SolveP<T> solve_consts(const Prim<T>& p, T iK3, int K)
+GKM_HD SolveP<T> solve_consts(const Prim<T>& p, const Phys<T>& ph)
 {
     SolveP<T> c;
-    c.z3 = T(K + 3) * p.s;
+    c.z3 = ph.k3 * p.s;
     c.uq = T(0.5) * (p.U[0] * p.U[0] + p.U[1] * p.U[1] + p.U[2] * p.U[2] + c.z3);
-    c.hf = (T(1.0 / kPrandtl) * iK3) * (p.is * p.is);
+    c.hf = ph.iPrK3 * (p.is * p.is);
     return c;
 }
 
@@ -986,6 +1020,14 @@ GKM_HD SlopeP<T> face_slope(const Prov& in, int v, const Prim<T>& p, const Solve
         return solve_lab<T>(in.DW(v, 0), in.DW(v, 1), in.DW(v, 2), in.DW(v, 3), in.DW(v, 4), T(1), p, c);
 }
 
+// the factor of a one-sided difference over half a cell, 2 / dx
+template <class T, class Prov>
+GKM_HD T normal_scale(const Prov& in, T dx)
+{
+    if constexpr (has_raw<Prov>::value) return in.scale(0);
+    else return T(2) / dx;
+}
+
 // The time integrals the peculiar form needs, from src/GKMflux.cpp:162-167,197-204 with
 // gm0 = dt - tau (1 - e), e = exp(-dt/tau), multiplied out: the slope of the equilibrium is solved
 // from gm0 B_, so the coefficients are
@@ -1021,7 +1063,7 @@ GKM_HD RelaxCoefs<T> relax_coefs(wide_t<T> tau, wide_t<T> dt)
     c.dte = T(dte);
     c.h = T((P - dt) + (P - dte));
     c.p0 = T(gm0);
-    c.p1g = T(D(0.5) * dt * dt / gm0 - tau);
+    c.p1g = T((D(0.5) * dt) * (dt * recip<D>(gm0)) - tau);
     return c;
 }
 
@@ -1031,8 +1073,6 @@ GKM_HD RelaxCoefs<T> relax_coefs(wide_t<T> tau, wide_t<T> dt)
 template <class T, class Prov>
 GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, T F[5])
 {
-    const int K = ph.K;
-    const T iK3 = ph.iK3;
     Prim<T> st[2];
     T inv_psum;
     {
@@ -1057,7 +1097,7 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
         half_space<T>(p, j == 0 ? +1 : -1, J0[j], g[j]);
         const T m = p.den * J0[j], mu = p.den * (p.U[0] * J0[j] + g[j]);   // rho <1>, rho <u>
         const T o2 = m * p.U[1], o3 = m * p.U[2];
-        const T o4 = T(0.5) * (mu * p.U[0] + o2 * p.U[1] + o3 * p.U[2] + T(K + 3) * (p.P * J0[j]));
+        const T o4 = T(0.5) * (mu * p.U[0] + o2 * p.U[1] + o3 * p.U[2] + ph.k3 * (p.P * J0[j]));
         if (j == 0) {
             We[0] = m; We[1] = mu; We[2] = o2; We[3] = o3; We[4] = o4;
         } else {
@@ -1074,8 +1114,8 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
     for (int side = 0; side < 2; side++) {
         const Prim<T> p = side == 0 ? st[0] : st[1];
         const T s = p.s, U = p.U[0];
-        const T z1 = T(K + 2) * s, k4 = T(K + 4) * s;
-        const SolveP<T> sv = solve_consts<T>(p, iK3, K);
+        const T z1 = ph.k2 * s, k4 = ph.k4 * s;
+        const SolveP<T> sv = solve_consts<T>(p, ph);
         const T d[3] = {U - e.U[0], p.U[1] - e.U[1], p.U[2] - e.U[2]};
         const T d2[3] = {d[0] + d[0], d[1] + d[1], d[2] + d[2]};
         const T dd = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
@@ -1094,9 +1134,9 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
         half_G<T>(o, q, J, A, an, ay, az, s, U, z1, k4);
         // this side's time slope (src/GKMflux.cpp:145-151) with its sign changed: the slopes of
         // <psi G> over the full space
-        const T S = an.a1 + ay.a2 + az.a3, k5 = T(K + 5) * s;
+        const T S = an.a1 + ay.a2 + az.a3, k5 = ph.k5 * s;
         SlopeP<T> at;
-        at.h = T(1.0 / kPrandtl) * (A.h + iK3 * S);
+        at.h = T(1.0 / kPrandtl) * A.h + ph.iPrK3 * S;
         at.a1 = (A.a1 + an.a0) + an.h * k5;
         at.a2 = (A.a2 + ay.a0) + ay.h * k5;
         at.a3 = (A.a3 + az.a0) + az.h * k5;
@@ -1123,12 +1163,12 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
 
     // ---------------- equilibrium part, in its own frame
     const T s = e.s, U = e.U[0];
-    const T z1 = T(K + 2) * s, k5 = T(K + 5) * s, k7 = T(K + 7) * s;
-    const SolveP<T> sv = solve_consts<T>(e, iK3, K);
+    const T z1 = ph.k2 * s, k5 = ph.k5 * s, k7 = ph.k7 * s;
+    const SolveP<T> sv = solve_consts<T>(e, ph);
     const T h = rc.h, p2 = rc.tau * h;
     // normal slopes from the cell averages (src/GKMflux.cpp:115-116), left minus right and right:
     // <P_l>_{u>0} + <P_r>_{u<0} = <P_l - P_r>_{u>0} + <P_r>
-    const T idx2 = T(2) / dx;
+    const T idx2 = normal_scale<T>(in, dx);
     T br[5], bd[5];
 #pragma unroll
     for (int i = 0; i < 5; i++) {
@@ -1185,7 +1225,7 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
         const T r = rc.p0 * e.P;
         Fe[0] += rc.p0 * We[1];
         Fe[1] += r;
-        Fe[4] += (T(K + 3) * U) * r;
+        Fe[4] += (ph.k3 * U) * r;
     }
     // to the laboratory frame
     F[0] = Fe[0];

@@ -118,6 +118,22 @@ __device__ __forceinline__ double step_dt(const SweepArgs& a)
     return cfl_dt(a.fc, a.clock, a.parity, a.dt_fixed_mode, a.dt_fixed);
 }
 
+// the flux's constants from the launch's: dimensional for double, non-dimensional for float
+template <class T>
+__device__ __forceinline__ Phys<T> sweep_phys(const FieldConst& fc)
+{
+    Phys<T> ph{T(fc.gam), T(fc.gm1), sizeof(T) == 4 ? T(1) : T(kR), fc.K};
+    ph.k2 = T(fc.k2);
+    ph.k3 = T(fc.k3);
+    ph.k4 = T(fc.k4);
+    ph.k5 = T(fc.k5);
+    ph.k7 = T(fc.k7);
+    ph.iK3 = T(fc.iK3);
+    ph.iPrK3 = T(fc.iPrK3);
+    if (sizeof(T) == 8) ph.dK2 = T(fc.dK2);   // the float's own rounding of gamma - 1 enters the mixed one
+    return ph;
+}
+
 __device__ __forceinline__ double block_max(double v, double* red)
 {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -394,13 +410,12 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
     const T dtw = kMixed ? T(dt * fc.u_s * fc.inv_dx) : T(dt);
     const T dxw = kMixed ? T(1) : T(fc.dx);
     const T inv_dxw = kMixed ? T(1) : T(fc.inv_dx);
-    const Phys<T> ph{T(fc.gam), T(fc.gm1), kMixed ? T(1) : T(kR), fc.K};
+    const Phys<T> ph = sweep_phys<T>(fc);
     const float cv_mixed = float(1.0 / fc.gm1);   // R / (gamma - 1) in the non-dimensional units (R = 1)
     const T eps_r = kMixed ? T(fc.eps_rho) : T(kWenoEps);
     const T eps_m = kMixed ? T(fc.eps_m) : T(kWenoEps);
     const T eps_T = kMixed ? T(fc.eps_T) : T(kWenoEps);
     const double* __restrict__ W = a.W;
-    const double suth_c = fc.mu0 * (fc.T0 + 110.4) * kR / ((kR * fc.T0) * sqrt(kR * fc.T0));
     // mixed form: tau' = tau us / dx = tc_a x^(3/2) / ((x + tc_b) p') (Sutherland) or tc_a x^0.76 / p'
     // (power law), x = T / T0, p' = p / p0
     const float tc_a = kMixed ? float(fc.visc == 1 ? fc.mu0 * fc.u_s * fc.inv_dx / fc.p0
@@ -711,7 +726,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                         // indicators' own size before it can overflow
                         constexpr T k24 = T(1.0 / 16777216.0);
                         const T p01 = k24 * (pq[0] * pq[1]), p23 = k24 * (pq[2] * pq[3]);
-                        const T inv = T(1.0 / 6.0 / 16777216.0) / (p01 * p23);
+                        const T inv = T(1.0 / 6.0 / 16777216.0) * recip<T>(p01 * p23);
                         const T i01 = p23 * inv, i23 = p01 * inv;   // 1 / (6 p01), 1 / (6 p23)
                         const T iq[4] = {pq[1] * i01, pq[0] * i01, pq[3] * i23, pq[2] * i23};
 #pragma unroll
@@ -721,7 +736,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                         }
                     }
                     const T pT = D[4][0] * D[4][1], plr = l[0] * r[0];
-                    const T inv2 = T(1) / (pT * plr);
+                    const T inv2 = recip<T>(pT * plr);
                     const T iT = T(1.0 / 6.0) * (plr * inv2), ilr = pT * inv2;   // 1 / (6 pT), 1 / (rho_l rho_r)
                     const T Tc = s2[5 * kWC + c];
                     const T Tl = Tc + N[4][0] * (D[4][1] * iT), Tr = Tc + N[4][1] * (D[4][0] * iT);
@@ -813,7 +828,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                 // mu(T) / p = C sqrt(pd) / (pd + 110.4 R rho^2), C = mu0 (T0 + 110.4) R / (R T0)^(3/2)
                 const double d = wl[cc], m1 = wl[kWC + cc], m2 = wl[2 * kWC + cc], m3 = wl[3 * kWC + cc];
                 const double pd = fc.gm1 * (wl[4 * kWC + cc] * d - 0.5 * (m1 * m1 + m2 * m2 + m3 * m3));
-                tau0 = suth_c * sqrt(pd) / (pd + (110.4 * kR) * (d * d));
+                tau0 = fc.suth_c * (pd * rsqrt_t<double>(pd)) * recip<double>(pd + (110.4 * kR) * (d * d));
             }
             const long long ci = cell0 + (long long)(f + 3) * st.sn;
             // the accumulator of this cell (y, z sweeps) travels to shared memory while the flux

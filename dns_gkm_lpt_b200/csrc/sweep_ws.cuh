@@ -117,9 +117,8 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
     const int f_begin = a.f0 + bz * a.seg_len;
     const int f_end = min(f_begin + a.seg_len, a.f1 > 0 ? a.f1 : n);
     const double dt = step_dt(a);
-    const Phys<T> ph{fc.gam, fc.gm1, kR, fc.K};
+    const Phys<T> ph = sweep_phys<T>(fc);
     const double* __restrict__ W = a.W;
-    const double suth_c = fc.mu0 * (fc.T0 + 110.4) * kR / ((kR * fc.T0) * sqrt(kR * fc.T0));
 
     if (DIR == 0 && bx == 0 && by == 0 && bz == 0 && tid == 0 && !a.skip_clock_init) {
         a.clock->wave[a.parity ^ 1] = 0ull;   // the z sweep of this step reduces into it
@@ -229,7 +228,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                         // indicators' own size before it can overflow
                         constexpr T k24 = T(1.0 / 16777216.0);
                         const T p01 = k24 * (pq[0] * pq[1]), p23 = k24 * (pq[2] * pq[3]);
-                        const T inv = T(1.0 / 6.0 / 16777216.0) / (p01 * p23);
+                        const T inv = T(1.0 / 6.0 / 16777216.0) * recip<T>(p01 * p23);
                         const T i01 = p23 * inv, i23 = p01 * inv;
                         const T iq[4] = {pq[1] * i01, pq[0] * i01, pq[3] * i23, pq[2] * i23};
 #pragma unroll
@@ -239,7 +238,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                         }
                     }
                     const T pT = D[4][0] * D[4][1], plr = l[0] * r[0];
-                    const T inv2 = T(1) / (pT * plr);
+                    const T inv2 = recip<T>(pT * plr);
                     const T iT = T(1.0 / 6.0) * (plr * inv2), ilr = pT * inv2;
                     const T Tc = s2[5 * kWC + c];
                     const T Tl = Tc + N[4][0] * (D[4][1] * iT), Tr = Tc + N[4][1] * (D[4][0] * iT);
@@ -304,7 +303,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                 } else {
                     const double d = wl[cc], m1 = wl[kWC + cc], m2 = wl[2 * kWC + cc], m3 = wl[3 * kWC + cc];
                     const double pd = fc.gm1 * (wl[4 * kWC + cc] * d - 0.5 * (m1 * m1 + m2 * m2 + m3 * m3));
-                    tau0 = suth_c * sqrt(pd) / (pd + (110.4 * kR) * (d * d));
+                    tau0 = fc.suth_c * (pd * rsqrt_t<double>(pd)) * recip<double>(pd + (110.4 * kR) * (d * d));
                 }
                 const long long ci = cell0 + (long long)(f + 3) * st.sn;
                 constexpr bool kFetchA = DIR != 0;
