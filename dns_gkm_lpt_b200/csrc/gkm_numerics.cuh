@@ -154,7 +154,7 @@ GKM_HD void weno_scalar(T a3, T a2, T a1, T b1, T b2, T b3, T eps, T& fl, T& fr)
 // candidate k and the right-biased candidate 3-k are the same polynomial of the same three
 // cells, and so are the second differences of their indicators, so four of each serve both
 // sides; a candidate is a1 + delta/6.  The indicators are taken four times over, 4 (eps + IS) =
-// (13/3 d^2 + 4 eps) + e^2, which leaves the weights as they are: 70 operations for both sides
+// (13/3 d^2 + 4 eps) + e^2, which leaves the weights as they are: 64 operations for both sides
 // where candidates and indicators of the cell values took 112.
 // Measured at 256^3 (a step, default shapes): FP64 13.97 -> 13.00 ms, mixed 8.26 -> 8.05 ms; the
 // reconstructed values' error against extended precision is a tenth (FP64) and a third (FP32) of
@@ -181,7 +181,8 @@ GKM_HD double imax<double>(double a, double b)
 
 template <class T>
 struct WenoParts {
-    T d0, d1, d2, d3;        // six times (candidate - a1): the left side's 0..3, the right side's 3..0
+    T d0, d1, d2, d3;        // six times (candidate - a1), 9 times that for the middle two (their linear
+                             // weight against the outer two's): the left side's 0..3, the right side's 3..0
     T l0, l1, l2, l3;        // 4 (eps + IS) of the left side
     T r0, r1, r2, r3;        // and of the right side
 };
@@ -194,21 +195,22 @@ GKM_HD WenoParts<T> weno_parts(T a3, T a2, T a1, T b1, T b2, T b3, T eps)
     const T dA = f2 - f1, dB = f3 - f2, dC = f4 - f3, dD = f5 - f4;
     const T qA = c * dA * dA + e4, qB = c * dB * dB + e4, qC = c * dC * dC + e4, qD = c * dD * dD + e4;
     WenoParts<T> w;
+    const T el = T(3) * f2 - f1, er = T(3) * f4 - f5;
     T e;
-    e = T(3) * f2 - f1;          w.l0 = qA + e * e;
+    w.l0 = qA + el * el;
     e = f2 + f3;                 w.l1 = qB + e * e;
     e = T(3) * f3 - f4;          w.l2 = qC + e * e;
-    e = T(5) * f4 - T(3) * f5;   w.l3 = qD + e * e;
-    e = T(3) * f4 - f5;          w.r0 = qD + e * e;
+    e = er - T(2) * dD;          w.l3 = qD + e * e;   // 5 f4 - 3 f5
+    w.r0 = qD + er * er;
     e = f3 + f4;                 w.r1 = qC + e * e;
     e = T(3) * f3 - f2;          w.r2 = qB + e * e;
-    e = T(5) * f2 - T(3) * f1;   w.r3 = qA + e * e;
+    e = el + T(2) * dA;          w.r3 = qA + e * e;   // 5 f2 - 3 f1
     w.l3 = imax<T>(imax<T>(w.l0, w.l1), imax<T>(w.l2, w.l3));
     w.r3 = imax<T>(imax<T>(w.r0, w.r1), imax<T>(w.r2, w.r3));
-    w.d0 = T(5) * f2 - T(2) * f1;
-    w.d1 = T(2) * f3 + f2;
-    w.d2 = T(4) * f3 - f4;
-    w.d3 = T(6) * f3 - T(5) * f4 + T(2) * f5;
+    w.d0 = T(2) * el - f2;                       // 5 f2 - 2 f1
+    w.d1 = T(18) * f3 + T(9) * f2;
+    w.d2 = T(36) * f3 - T(9) * f4;
+    w.d3 = T(6) * f3 - T(T(2) * er - f4);        // 6 f3 - 5 f4 + 2 f5
     return w;
 }
 
@@ -220,14 +222,14 @@ GKM_HD void weno_nd(T a3, T a2, T a1, T b1, T b2, T b3, T eps, T& Nl, T& Dl, T& 
     const WenoParts<T> w = weno_parts<T>(a3, a2, a1, b1, b2, b3, eps);
     const T n = T(9);
     {
-        const T p01 = w.l0 * w.l1, p23 = w.l2 * w.l3, g0 = n * w.l0, g3 = n * w.l3;
-        Nl = p23 * (w.l1 * w.d0 + g0 * w.d1) + p01 * (g3 * w.d2 + w.l2 * w.d3);
-        Dl = p23 * (w.l1 + g0) + p01 * (g3 + w.l2);
+        const T p01 = w.l0 * w.l1, p23 = w.l2 * w.l3;
+        Nl = p23 * (w.l1 * w.d0 + w.l0 * w.d1) + p01 * (w.l3 * w.d2 + w.l2 * w.d3);
+        Dl = p23 * (n * w.l0 + w.l1) + p01 * (n * w.l3 + w.l2);
     }
     {
-        const T p01 = w.r0 * w.r1, p23 = w.r2 * w.r3, g0 = n * w.r0, g3 = n * w.r3;
-        Nr = p23 * (w.r1 * w.d3 + g0 * w.d2) + p01 * (g3 * w.d1 + w.r2 * w.d0);
-        Dr = p23 * (w.r1 + g0) + p01 * (g3 + w.r2);
+        const T p01 = w.r0 * w.r1, p23 = w.r2 * w.r3;
+        Nr = p23 * (w.r1 * w.d3 + w.r0 * w.d2) + p01 * (w.r3 * w.d1 + w.r2 * w.d0);
+        Dr = p23 * (n * w.r0 + w.r1) + p01 * (n * w.r3 + w.r2);
     }
 }
 
@@ -241,15 +243,15 @@ GKM_HD void weno_scalar(T a3, T a2, T a1, T b1, T b2, T b3, T eps, T& fl, T& fr)
         const WenoParts<T> w = weno_parts<T>(a3, a2, a1, b1, b2, b3, eps);
         const T n = T(9), c16 = T(1.0 / 6.0);
         {
-            const T t = (w.l0 * w.l1) / (w.l2 * w.l3), g0 = n * w.l0, g3 = n * w.l3;
-            const T x = w.l1 * w.d0 + g0 * w.d1, y = g3 * w.d2 + w.l2 * w.d3;
-            const T u = w.l1 + g0, v = g3 + w.l2;
+            const T t = (w.l0 * w.l1) / (w.l2 * w.l3);
+            const T x = w.l1 * w.d0 + w.l0 * w.d1, y = w.l3 * w.d2 + w.l2 * w.d3;
+            const T u = n * w.l0 + w.l1, v = n * w.l3 + w.l2;
             fl = a1 + c16 * T((x + t * y) / (u + t * v));
         }
         {
-            const T t = (w.r0 * w.r1) / (w.r2 * w.r3), g0 = n * w.r0, g3 = n * w.r3;
-            const T x = w.r1 * w.d3 + g0 * w.d2, y = g3 * w.d1 + w.r2 * w.d0;
-            const T u = w.r1 + g0, v = g3 + w.r2;
+            const T t = (w.r0 * w.r1) / (w.r2 * w.r3);
+            const T x = w.r1 * w.d3 + w.r0 * w.d2, y = w.r3 * w.d1 + w.r2 * w.d0;
+            const T u = n * w.r0 + w.r1, v = n * w.r3 + w.r2;
             fr = a1 + c16 * T((x + t * y) / (u + t * v));
         }
     } else {
@@ -273,7 +275,7 @@ GKM_HD T temperature(T r, T m1, T m2, T m3, T E, const Phys<T>& ph)
     return ph.gm1 * (E * ir - T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) * ir * ir) / ph.Rg;
 #else
     const T ir = recip<T>(r);
-    return (E * ir - T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3) * ir * ir) * (ph.gm1 / ph.Rg);
+    return (E - (T(0.5) * (m1 * m1 + m2 * m2 + m3 * m3)) * ir) * (ir * (ph.gm1 / ph.Rg));
 #endif
 }
 
@@ -700,21 +702,25 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
 // J_k = <c^k>_{u>0}.  Written in psi'' = (1, c, v', w', (c^2 + v'^2 + w'^2 + xi^2)/2),
 //   * the slope solve is diagonal (SlopeP, solve_lab / solve_pec);
 //   * the full-space moments of G = u (psi.a_n) + v (psi.a_y) + w (psi.a_z) are closed forms
-//     of a few products (full_G): with A = U a_n + V a_y + W a_z and D = c P_n + v' P_y + w' P_z,
+//     of a few products: with A = U a_n + V a_y + W a_z and D = c P_n + v' P_y + w' P_z,
 //     G = psi''.A + D;
 //   * the half-space moments of G and of psi.a are sums of four or three J_k per component,
 //     because the tangential average of zeta = v'^2 + w'^2 + xi^2 against a polynomial differs
-//     from <zeta> times its average by one product with s (half_G, half_P).
+//     from <zeta> times its average by one product with s (half_poly, half_P).
 // Every moment, slope and time coefficient is the reference's (src/GKMflux.cpp:11-229); the
 // frames, and so the order of the sums, are not.  Each side's moments go from its own frame to
-// the equilibrium state's by psi_e = T(U - U_e) psi'' (to_frame), where the equilibrium's slopes
+// the equilibrium state's by psi_e = T(U - U_e) psi'' (add_in_frame), where the equilibrium's slopes
 // are solved, and the summed flux to the laboratory frame at the end.  The reference's
 // gamma_1 (moments of the equilibrium) + gamma_3 (its conserved state), gamma_3 = -gamma_1, has
 // an energy component only, gamma_1 p dK2 / 2 (Phys).  About 900 operations per face beside the divisions and
 // the special functions, where the moments in the laboratory frame took about 2,000; the sweeps
-// are bound by the FP64 (mixed: FP32) arithmetic.  Measured at 256^3 with the default shapes: a step
-// 18.00 -> 13.97 ms in FP64, 10.62 -> 8.26 ms in the mixed form; errors against extended precision
-// equal (mass, tangential momentum) or smaller (normal momentum, energy).
+// are bound by the FP64 (mixed: FP32) arithmetic: the FP64 pipe takes a warp instruction every 2.2
+// cycles from independent streams and every 2.5 to 3 from chains of one or two, however many warps
+// there are, so the count of operations decides.  Measured at 256^3 with the default shapes: a step
+// 18.00 -> 13.97 ms in FP64, 10.62 -> 8.26 ms in the mixed form; with the polynomials of a side combined
+// before one contraction per weight, single reciprocals and the shorter WENO sums the x/y/z sweeps went
+// from 2.67/2.74/3.14 to 2.57/2.63/3.02 ms (64- and 48-face segments).  Errors against extended precision
+// are smaller in every component than with the laboratory-frame moments.
 
 // Primitive values of a state: 1/rho, p, s = 1 / (2 lam) = p / rho and 1 / s.
 template <class T>
@@ -722,55 +728,20 @@ struct Prim {
     T den, ir, U[3], P, s, is;
 };
 
-// both face states together, with pd = p rho = (gamma - 1)(E rho - |m|^2 / 2) known before any
-// division: 1/rho_l, 1/rho_r, 1/p_l, 1/p_r and 1/(p_l + p_r) (the collision-time ratio) all
-// from one reciprocal of rho_l rho_r pd_l pd_r S, S = pd_l rho_r + pd_r rho_l = (p_l + p_r) rho_l rho_r
-template <class T>
-GKM_HD void prim_pair(const T wl[5], const T wr[5], T gm1, Prim<T>& l, Prim<T>& r, T& inv_psum)
-{
-    l.den = wl[0];
-    r.den = wr[0];
-    const T pdl = gm1 * (wl[4] * l.den - T(0.5) * (wl[1] * wl[1] + wl[2] * wl[2] + wl[3] * wl[3]));
-    const T pdr = gm1 * (wr[4] * r.den - T(0.5) * (wr[1] * wr[1] + wr[2] * wr[2] + wr[3] * wr[3]));
-    const T dd = l.den * r.den, pp = pdl * pdr;
-    const T S = pdl * r.den + pdr * l.den;
-    const T inv = recip<T>((dd * pp) * S);
-    const T ppS = pp * S * inv;   // 1 / dd
-    l.ir = r.den * ppS;
-    r.ir = l.den * ppS;
-    const T ddS = dd * S * inv;   // 1 / pp
-    const T iPl = l.den * (pdr * ddS), iPr = r.den * (pdl * ddS);   // rho / pd
-    inv_psum = dd * (dd * pp * inv);
-    Prim<T>* st[2] = {&l, &r};
-    const T* w[2] = {wl, wr};
-    const T iP[2] = {iPl, iPr};
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        Prim<T>& p = *st[k];
-        p.U[0] = w[k][1] * p.ir;
-        p.U[1] = w[k][2] * p.ir;
-        p.U[2] = w[k][3] * p.ir;
-        p.P = gm1 * (w[k][4] - T(0.5) * (w[k][1] * p.U[0] + w[k][2] * p.U[1] + w[k][3] * p.U[2]));
-        p.s = p.P * p.ir;
-        p.is = p.den * iP[k];
-    }
-}
-
-// one state with one division: 1/rho = pd / (rho pd), 1/p = rho^2 / (rho pd)
+// 1/rho and 1/p each by a reciprocal of its own (grouping them under one costs more products than the
+// short reciprocal has steps)
 template <class T>
 GKM_HD Prim<T> prim(const T W[5], T gm1)
 {
     Prim<T> p;
     p.den = W[0];
-    const T pd = gm1 * (W[4] * p.den - T(0.5) * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]));
-    const T inv = recip<T>(p.den * pd);
-    p.ir = pd * inv;
+    p.ir = recip<T>(W[0]);
     p.U[0] = W[1] * p.ir;
     p.U[1] = W[2] * p.ir;
     p.U[2] = W[3] * p.ir;
     p.P = gm1 * (W[4] - T(0.5) * (W[1] * p.U[0] + W[2] * p.U[1] + W[3] * p.U[2]));
     p.s = p.P * p.ir;
-    p.is = p.den * (p.den * p.den * inv);
+    p.is = p.den * recip<T>(p.P);
     return p;
 }
 
@@ -973,35 +944,25 @@ GKM_HD SlopeP<T> convect(const T U[3], const SlopeP<T>& n, const SlopeP<T>& y, c
     return A;
 }
 
-// <psi'' G> with weights 1 and u (o and p) over the half space of J
+// A polynomial Q = k G + l P_t (+ m) of the half-space moments, by its tangential averages:
+// <Q> = c0 + c1 c + c2 c^2 + c3 c^3, <zeta Q> = z1 <Q> + 2 s (y0 + y1 c), <v' Q> = s (v0 + v1 c + v2 c^2),
+// <w' Q> likewise
 template <class T>
-GKM_HD void half_G(T o[5], T p[5], const T* J, const SlopeP<T>& A, const SlopeP<T>& n, const SlopeP<T>& y,
-                   const SlopeP<T>& z, T s, T U, T z1, T k4)
+struct HalfPoly {
+    T c0, c1, c2, c3, y0, y1, v0, v1, v2, w0, w1, w2;
+};
+// <psi'' Q> with the normal weight N_k (J: 1; L: u)
+template <class T>
+GKM_HD void half_poly(T o[5], const T* N, const HalfPoly<T>& Q, T s, T z1)
 {
-    // <G>_tan = c0 + c1 c + c2 c^2 + c3 c^3, <zeta G>_tan = z1 <G>_tan + 2 s (y0 + y1 c)
-    const T y0 = A.h * z1 + s * (y.a2 + z.a3), y1 = n.h * z1;
-    const T c0 = A.a0 + y0, c1 = (A.a1 + n.a0) + y1, c2 = A.h + n.a1, c3 = n.h;
-    const T s0 = c0 * J[0] + c1 * J[1] + c2 * J[2] + c3 * J[3];
-    const T s1 = c0 * J[1] + c1 * J[2] + c2 * J[3] + c3 * J[4];
-    const T s2 = c0 * J[2] + c1 * J[3] + c2 * J[4] + c3 * J[5];
-    const T s3 = c0 * J[3] + c1 * J[4] + c2 * J[5] + c3 * J[6];
-    // <v' G>_tan = s (v0 + v1 c + h_y c^2), <w' G>_tan likewise
-    const T v0 = (A.a2 + y.a0) + y.h * k4, v1 = n.a2 + y.a1;
-    const T w0 = (A.a3 + z.a0) + z.h * k4, w1 = n.a3 + z.a1;
-    const T va = v0 * J[0] + v1 * J[1] + y.h * J[2], vb = v0 * J[1] + v1 * J[2] + y.h * J[3];
-    const T wa = w0 * J[0] + w1 * J[1] + z.h * J[2], wb = w0 * J[1] + w1 * J[2] + z.h * J[3];
-    const T ea = y0 * J[0] + y1 * J[1], eb = y0 * J[1] + y1 * J[2];
-    const T ss = s + s;
+    const T s0 = Q.c0 * N[0] + Q.c1 * N[1] + Q.c2 * N[2] + Q.c3 * N[3];
+    const T s1 = Q.c0 * N[1] + Q.c1 * N[2] + Q.c2 * N[3] + Q.c3 * N[4];
+    const T s2 = Q.c0 * N[2] + Q.c1 * N[3] + Q.c2 * N[4] + Q.c3 * N[5];
     o[0] = s0;
     o[1] = s1;
-    o[2] = s * va;
-    o[3] = s * wa;
-    o[4] = z1 * s0 + (s2 + ss * ea);
-    p[0] = s1 + U * s0;
-    p[1] = s2 + U * s1;
-    p[2] = s * (vb + U * va);
-    p[3] = s * (wb + U * wa);
-    p[4] = z1 * p[0] + ((s3 + U * s2) + ss * (eb + U * ea));
+    o[2] = s * (Q.v0 * N[0] + Q.v1 * N[1] + Q.v2 * N[2]);
+    o[3] = s * (Q.w0 * N[0] + Q.w1 * N[1] + Q.w2 * N[2]);
+    o[4] = z1 * s0 + (s2 + (s + s) * (Q.y0 * N[0] + Q.y1 * N[1]));
 }
 
 // a face provider may give raw differences and their common factors instead of slopes:
@@ -1047,13 +1008,17 @@ template <class T, bool EXPM1>
 GKM_HD RelaxCoefs<T> relax_coefs(wide_t<T> tau, wide_t<T> dt)
 {
     using D = wide_t<T>;
-    D e, omx;
-    if constexpr (EXPM1) {
-        omx = -expm1(-dt / tau);
-        e = D(1) - omx;
-    } else {
-        e = exp_t<D>(-dt / tau);
-        omx = D(1) - e;
+    D e = D(0), omx = D(1);
+    // beyond x = dt / tau = 40, e (under 2^-57) is below the rounding of every term it enters
+    const D x = dt / tau;
+    if (!(x > D(40))) {
+        if constexpr (EXPM1) {
+            omx = -expm1(-x);
+            e = D(1) - omx;
+        } else {
+            e = exp_t<D>(-x);
+            omx = D(1) - e;
+        }
     }
     const D P = tau * omx, dte = dt * e, gm0 = dt - P;
     RelaxCoefs<T> c;
@@ -1074,7 +1039,6 @@ template <class T, class Prov>
 GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph, T F[5])
 {
     Prim<T> st[2];
-    T inv_psum;
     {
         T wl[5], wr[5];
 #pragma unroll
@@ -1082,12 +1046,13 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
             wl[q] = in.Wl(q);
             wr[q] = in.Wr(q);
         }
-        prim_pair<T>(wl, wr, ph.gm1, st[0], st[1], inv_psum);
+        st[0] = prim<T>(wl, ph.gm1);
+        st[1] = prim<T>(wr, ph.gm1);
     }
     // collision time with the pressure-jump correction, src/GKMflux.cpp:156-157:
     // |rho_l/lam_l - rho_r/lam_r| / |rho_l/lam_l + rho_r/lam_r| with rho/lam = 2 p (p > 0)
     const RelaxCoefs<T> rc = relax_coefs<T, (sizeof(T) < sizeof(wide_t<T>))>(
-        wide_t<T>(tau0) + wide_t<T>(dt) * wide_t<T>(fabs(st[0].P - st[1].P) * inv_psum), wide_t<T>(dt));
+        wide_t<T>(tau0) + wide_t<T>(dt) * wide_t<T>(fabs(st[0].P - st[1].P) * recip<T>(st[0].P + st[1].P)), wide_t<T>(dt));
 
     // the equilibrium state at the face (src/GKMflux.cpp:73-77), from both half-Maxwellians
     T We[5], J0[2], g[2];
@@ -1131,32 +1096,61 @@ GKM_HD void gks_flux_peculiar(const Prov& in, T tau0, T dt, T dx, const Phys<T>&
         add_in_frame<T>(bz, wy, o, d, d2, dd);
         const SlopeP<T> an = face_slope<T>(in, side, p, sv);
         const SlopeP<T> A = convect<T>(p.U, an, ay, az);
-        half_G<T>(o, q, J, A, an, ay, az, s, U, z1, k4);
+        // <psi G>, averaged over the tangential velocities
+        HalfPoly<T> G;
+        G.y0 = A.h * z1 + s * (ay.a2 + az.a3);
+        G.y1 = an.h * z1;
+        G.c0 = A.a0 + G.y0;
+        G.c1 = (A.a1 + an.a0) + G.y1;
+        G.c2 = A.h + an.a1;
+        G.c3 = an.h;
+        G.v0 = (A.a2 + ay.a0) + ay.h * k4;
+        G.v1 = an.a2 + ay.a1;
+        G.v2 = ay.h;
+        G.w0 = (A.a3 + az.a0) + az.h * k4;
+        G.w1 = an.a3 + az.a1;
+        G.w2 = az.h;
         // this side's time slope (src/GKMflux.cpp:145-151) with its sign changed: the slopes of
-        // <psi G> over the full space
+        // <psi G> over the full space; averaged likewise (its v' and w' parts are t2, t3 alone)
         const T S = an.a1 + ay.a2 + az.a3, k5 = ph.k5 * s;
-        SlopeP<T> at;
-        at.h = T(1.0 / kPrandtl) * A.h + ph.iPrK3 * S;
-        at.a1 = (A.a1 + an.a0) + an.h * k5;
-        at.a2 = (A.a2 + ay.a0) + ay.h * k5;
-        at.a3 = (A.a3 + az.a0) + az.h * k5;
-        at.a0 = (A.a0 + s * S) + (A.h - at.h) * sv.z3;
-        T x[5], y[5];
-        half_P2<T>(x, y, J, at, s, U, z1);
+        const T th = T(1.0 / kPrandtl) * A.h + ph.iPrK3 * S, ty = th * z1;
+        const T t1 = (A.a1 + an.a0) + an.h * k5;
+        const T t2 = (A.a2 + ay.a0) + ay.h * k5;
+        const T t3 = (A.a3 + az.a0) + az.h * k5;
+        const T t0 = ((A.a0 + s * S) + (A.h - th) * sv.z3) + ty;
+        // gm0 B_ takes dt e G - P P_t, the flux p4 u G + p5 u P_t (the time slope's sign is in both) and
+        // the free transport of the initial half-Maxwellian, P rho u
         const T dte = rc.dte, P = rc.P, p5 = rc.tau * P, p4 = rc.tau * dte - (p5 + p5);
+        HalfPoly<T> Q;
+        Q.c0 = dte * G.c0 - P * t0;
+        Q.c1 = dte * G.c1 - P * t1;
+        Q.c2 = dte * G.c2 - P * th;
+        Q.c3 = dte * G.c3;
+        Q.y0 = dte * G.y0 - P * ty;
+        Q.y1 = dte * G.y1;
+        Q.v0 = dte * G.v0 - P * t2;
+        Q.v1 = dte * G.v1;
+        Q.v2 = dte * G.v2;
+        Q.w0 = dte * G.w0 - P * t3;
+        Q.w1 = dte * G.w1;
+        Q.w2 = dte * G.w2;
+        half_poly<T>(o, J, Q, s, z1);
+        Q.c0 = p4 * G.c0 + p5 * t0 + P * p.den;
+        Q.c1 = p4 * G.c1 + p5 * t1;
+        Q.c2 = p4 * G.c2 + p5 * th;
+        Q.c3 = p4 * G.c3;
+        Q.y0 = p4 * G.y0 + p5 * ty;
+        Q.y1 = p4 * G.y1;
+        Q.v0 = p4 * G.v0 + p5 * t2;
+        Q.v1 = p4 * G.v1;
+        Q.v2 = p4 * G.v2;
+        Q.w0 = p4 * G.w0 + p5 * t3;
+        Q.w1 = p4 * G.w1;
+        Q.w2 = p4 * G.w2;
+        T L[6];
 #pragma unroll
-        for (int i = 0; i < 5; i++) {
-            o[i] = dte * o[i] - P * x[i];
-            q[i] = p4 * q[i] + p5 * y[i];
-        }
-        // free transport of the initial half-Maxwellian: rho <u psi''>
-        {
-            const T r = P * p.den;
-            const T m0 = r * (J[1] + U * J[0]), m1 = r * (J[2] + U * J[1]);
-            q[0] += m0;
-            q[1] += m1;
-            q[4] += z1 * m0 + r * (J[3] + U * J[2]);
-        }
+        for (int k = 0; k < 6; k++) L[k] = J[k + 1] + U * J[k];   // <u c^k>
+        half_poly<T>(q, L, Q, s, z1);
         add_in_frame<T>(B, o, d, d2, dd);
         add_in_frame<T>(Fe, q, d, d2, dd);
     }
