@@ -63,10 +63,11 @@ using SweepTile64b = SweepTile<16, 16, 1>;
 // against four: x 1.536 / 11.86 -> 1.522 / 11.30, y 1.688 / 13.14 -> 1.651 / 12.36, z 1.969 / 14.77 -> 2.117 /
 // 15.45 (128 registers without the fourth CTA)
 using SweepTile32a = SweepTile<16, 8, 4>;
+constexpr int kMixedZCtas = 3;
 template <int DIR, class T, class Tile>
 constexpr int sweep_ctas()
 {
-    return sizeof(T) == 4 && DIR == 2 ? 3 : Tile::ctas;
+    return sizeof(T) == 4 && DIR == 2 ? kMixedZCtas : Tile::ctas;
 }
 // variant 2: 16 x 16 windows, warp-specialized (a producer warpgroup reconstructs face f+1 while
 // two consumer warpgroups compute the fluxes of face f; sweep_ws.cuh); ensembles: its persistent
