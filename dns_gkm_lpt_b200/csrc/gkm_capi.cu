@@ -236,11 +236,12 @@ cudaError_t enqueue_splines(gkm_handle* h, const double* W)
     }
     if (h->d_self && (W == h->buf[0] || W == h->buf[1])) {
         gkm::EnsembleWork w{};
-        w.line0 = h->d_self_off;
-        w.line1 = h->d_self_off + 2;
-        w.warp2 = h->d_self_off + 4;
+        w.group0 = h->d_self_off;
+        w.group1 = h->d_self_off + 2;
+        w.group2 = h->d_self_off + 4;
         h->launches += 3;
-        return gkm::launch_ensemble_splines(h->d_self, w, h->self_totals, 1, W == h->buf[0] ? 0 : 1, h->stream);
+        return gkm::launch_ensemble_splines(h->d_self, w, h->self_totals, 1, h->grid.npts, W == h->buf[0] ? 0 : 1,
+                                            h->stream);
     }
     h->launches += kSplinePasses;
     return gkm::launch_spline_build(W, h->fc, h->grid, device_tables(h), h->coef[0], h->coef[1], h->coef[2],
@@ -276,7 +277,9 @@ cudaError_t setup_batched_splines(gkm_handle* h)
     md.scratch[0] = h->scratch;
     md.scratch[1] = h->scratch_extra[0];
     md.scratch[2] = h->scratch_extra[1];
-    const long long off[6] = {0, 3 * N * N, 0, 3 * M * N, 0, 3 * ((M * M + 31) / 32)};
+    const int pad = h->grid.pad;
+    const long long off[6] = {0, 3 * gkm::spline_groups(0, N, pad), 0, 3 * gkm::spline_groups(1, N, pad),
+                              0, 3 * gkm::spline_groups(2, N, pad)};
     h->self_totals[0] = off[1];
     h->self_totals[1] = off[3];
     h->self_totals[2] = off[5];
@@ -623,6 +626,7 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     if (e != cudaSuccess) return bail(e, "cudaMalloc(stats)");
     e = gkm::sweep_prepare();
     if (e == cudaSuccess) e = gkm::sweep_mixed_prepare();
+    if (e == cudaSuccess) e = gkm::spline_prepare();
     if (e != cudaSuccess) return bail(e, "sweep_prepare");
     e = setup_batched_splines(h);
     if (e != cudaSuccess) return bail(e, "batched spline build");

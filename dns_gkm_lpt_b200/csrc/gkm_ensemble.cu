@@ -29,7 +29,7 @@ namespace {
 
 // offset arrays in d_off, each nm + 1 long longs
 // kOrderX..Z hold, per sweep direction, the member at each position of the work list
-enum OffsetSet { kItemX = 0, kItemY, kItemZ, kGhost, kLine0, kLine1, kWarp2, kPart, kOrderX, kOrderY, kOrderZ,
+enum OffsetSet { kItemX = 0, kItemY, kItemZ, kGhost, kGroup0, kGroup1, kGroup2, kPart, kOrderX, kOrderY, kOrderZ,
                  kNumSets };
 
 }  // namespace
@@ -132,16 +132,17 @@ gkm_status refresh(gkm_ensemble* E, bool need_state)
         for (int c = 0; c < 6; c++) md.P[c] = h->P[c];
         md.np = h->np;
         md.tmaps = h->d_tmaps;
-        const long long N = h->grid.npts, M = N + h->grid.pad;
+        const long long N = h->grid.npts;
+        const int pad = h->grid.pad;
         const long long nt = h->fc.nt;
         const bool parts = h->np > 0;   // members without particles skip the spline work
         const long long count[kPart + 1] = {0,
                                             0,
                                             0,
                                             nt * nt * nt - n * n * n,
-                                            parts ? 3 * N * N : 0,
-                                            parts ? 3 * M * N : 0,
-                                            parts ? 3 * ((M * M + 31) / 32) : 0,
+                                            parts ? 3 * gkm::spline_groups(0, N, pad) : 0,
+                                            parts ? 3 * gkm::spline_groups(1, N, pad) : 0,
+                                            parts ? 3 * gkm::spline_groups(2, N, pad) : 0,
                                             h->np};
         for (int s = kGhost; s <= kPart; s++) at(s, m + 1) = at(s, m) + count[s];
     }
@@ -188,17 +189,20 @@ cudaError_t launch_halo_all(gkm_ensemble* E, int parity)
 
 cudaError_t launch_splines_all(gkm_ensemble* E, int parity)
 {
-    if (E->total[kLine0] == 0) return cudaSuccess;
+    if (E->total[kGroup0] == 0) return cudaSuccess;
     gkm::EnsembleWork w{};
     for (int d = 0; d < 3; d++) w.item[d] = off_ptr(E, kItemX + d);
     w.ghost = off_ptr(E, kGhost);
-    w.line0 = off_ptr(E, kLine0);
-    w.line1 = off_ptr(E, kLine1);
-    w.warp2 = off_ptr(E, kWarp2);
+    w.group0 = off_ptr(E, kGroup0);
+    w.group1 = off_ptr(E, kGroup1);
+    w.group2 = off_ptr(E, kGroup2);
     w.part = off_ptr(E, kPart);
-    const long long totals[3] = {E->total[kLine0], E->total[kLine1], E->total[kWarp2]};
+    const long long totals[3] = {E->total[kGroup0], E->total[kGroup1], E->total[kGroup2]};
+    int max_npts = 0;
+    for (const gkm_handle* h : E->mem)
+        if (h->np > 0) max_npts = std::max(max_npts, h->grid.npts);
     E->launches += 3;
-    return gkm::launch_ensemble_splines(E->d_mem, w, totals, nm_of(E), parity ^ 1, E->stream);
+    return gkm::launch_ensemble_splines(E->d_mem, w, totals, nm_of(E), max_npts, parity ^ 1, E->stream);
 }
 
 cudaError_t launch_particles_all(gkm_ensemble* E)

@@ -39,7 +39,7 @@ struct gkm_handle {
     // left out when the device lacks the memory (large grids), then one component at a time
     double* scratch_extra[2] = {nullptr, nullptr};
     gkm::MemberDev* d_self = nullptr;
-    long long* d_self_off = nullptr;   // line0 | line1 | warp2 prefix offsets, 2 each
+    long long* d_self_off = nullptr;   // prefix offsets of the three passes' line groups, 2 each
     long long self_totals[3] = {0, 0, 0};
     bool splines_valid = false;
     int64_t np = 0, cap = 0;

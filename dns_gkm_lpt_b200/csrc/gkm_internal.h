@@ -154,6 +154,13 @@ struct SplineTables {
     double denom;        // periodic Sherman-Morrison denominator
 };
 
+// groups of 32 lines of one component in spline pass 0, 1 or 2
+__host__ __device__ inline long long spline_groups(int pass, long long N, int pad)
+{
+    const long long M = N + pad, lines = pass == 0 ? N * N : (pass == 1 ? M * N : M * M);
+    return (lines + 31) / 32;
+}
+cudaError_t spline_prepare();   // the line kernels' shared-memory limit, on the current device
 cudaError_t launch_spline_build(const double* W, const FieldConst& fc, const SplineGrid& g, const SplineTables& tb,
                                 double* coef_u, double* coef_v, double* coef_w, double* scratch, cudaStream_t s);
 cudaError_t launch_spline_component(const double* W, const FieldConst& fc, const SplineGrid& g, const SplineTables& tb,
@@ -231,9 +238,9 @@ struct MemberDev {
 struct EnsembleWork {           // prefix offsets, nm + 1 entries each, in device memory
     const long long* item[3];   // sweep work items per direction
     const long long* ghost;     // ghost cells
-    const long long* line0;     // spline pass-0 lines of the 3 components
-    const long long* line1;     // spline pass-1 lines of the 3 components
-    const long long* warp2;     // spline pass-2 groups of 32 lines, 3 components
+    const long long* group0;    // groups of 32 spline lines of the 3 components, pass 0
+    const long long* group1;    // pass 1
+    const long long* group2;    // pass 2
     const long long* part;      // particles
 };
 
@@ -261,7 +268,7 @@ cudaError_t launch_ensemble_sweep32(int dir, int variant, const MemberDev* mem, 
 cudaError_t launch_ensemble_halo(const MemberDev* mem, const long long* off, int nm, long long total, int buf,
                                  int finish_step, cudaStream_t s);
 cudaError_t launch_ensemble_splines(const MemberDev* mem, const EnsembleWork& w, const long long totals[3], int nm,
-                                    int buf, cudaStream_t s);
+                                    int max_npts, int buf, cudaStream_t s);
 cudaError_t launch_ensemble_heun(const MemberDev* mem, const long long* off, int nm, long long total, cudaStream_t s);
 
 // Thomas tables of the spline line solves (gkm_capi.cu)

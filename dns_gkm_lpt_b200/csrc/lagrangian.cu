@@ -13,8 +13,13 @@
 //   periodic:       the n interior cell centres, cyclic rows, stored N+3 per
 //                   axis with wrapped copies so a 4-point window never wraps.
 // The line solve and the evaluation use rounding-explicit intrinsics in the
-// order of the CPU oracle, so both produce the same bits.
+// order of the CPU oracle, so both produce the same bits.  A solve's divisions
+// by the pivots are multiplications by their reciprocals with a correction that
+// rounds as the division does (pivot_div.cuh).  Lines short enough for a few
+// warps of them per SM are solved in shared memory (resident_*), longer ones
+// streamed through global memory (line_solve, pass2_group).
 #include "gkm_internal.h"
+#include "pivot_div.cuh"
 
 namespace gkm {
 namespace {
@@ -35,17 +40,52 @@ constexpr int kLineBatchBatched = 8, kLineBatchSingle = 4;
 // where eight (64 registers) spill the fetch-ahead values
 constexpr int kPassCtasPerSm = 6;
 
+// The pivots and multipliers of the line solves reach the fixed point of d = 4 - 1/d to the last
+// bit within 17 rows, whatever the number of points and the ends; from this row on (but for the
+// last pivot of periodic lines) they are held in registers.
+constexpr int kPivotRows = 24;
+
+// x_i = (cv_u - x_{i+1}) / dp_i, i = i0 - u: the U rows of a back substitution down from i0
+// (below the line's last row), solutions into cv.  False, with x as it was, where a numerator is
+// out of pivot_quotient's range: the caller repeats the rows with divisions.
+template <int U>
+__device__ __forceinline__ bool back_rows(double (&cv)[U], int i0, const SplineTables& tb, double d_inf, double r_inf,
+                                          double& x)
+{
+    const bool fixed = i0 - U + 1 >= kPivotRows;
+    double y = x;
+    bool ok = true;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const double d = fixed ? d_inf : tb.dp[i0 - u], r = fixed ? r_inf : tb.mt[i0 - u + 1];
+        const double a = sub(cv[u], y);
+        ok = ok && pivot_in_range(a);
+        y = pivot_quotient(a, d, r);
+        cv[u] = y;
+    }
+    if (ok) x = y;
+    return ok;
+}
+// the fixed point: row kPivotRows where the line has it before its last row, else unused
+__device__ __forceinline__ void fixed_pivots(int N, const SplineTables& tb, double& d_inf, double& r_inf)
+{
+    d_inf = N > kPivotRows + 4 ? tb.dp[kPivotRows] : 0.0;
+    r_inf = N > kPivotRows + 4 ? tb.mt[kPivotRows + 1] : 0.0;
+}
+
 template <int U, class Src>
 __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables& tb, double* c, long long cs)
 {
+    double d_inf, r_inf;
+    fixed_pivots(N, tb, d_inf, r_inf);
     if (!periodic) {
         const double c0 = f(0), cl = f(N - 1);
         double rp = 0.0;
-        auto fwd = [&](int i, double fi) {
+        auto fwd = [&](int i, double fi, double m) {
             double r = mul(6.0, fi);
             if (i == 1) r = sub(r, c0);
             if (i == N - 2) r = sub(r, cl);
-            rp = (i == 1) ? r : sub(r, mul(tb.mt[i], rp));
+            rp = (i == 1) ? r : sub(r, mul(m, rp));
             c[(long long)(i + 1) * cs] = rp;
         };
         int i = 1;
@@ -54,9 +94,9 @@ __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables
 #pragma unroll
             for (int u = 0; u < U; u++) fv[u] = f(i + u);
 #pragma unroll
-            for (int u = 0; u < U; u++) fwd(i + u, fv[u]);
+            for (int u = 0; u < U; u++) fwd(i + u, fv[u], i > kPivotRows ? r_inf : tb.mt[i + u]);
         }
-        for (; i <= N - 2; i++) fwd(i, f(i));
+        for (; i <= N - 2; i++) fwd(i, f(i), tb.mt[i]);
         double x = __ddiv_rn(c[(long long)(N - 1) * cs], tb.dp[N - 2]);
         c[(long long)(N - 1) * cs] = x;
         i = N - 3;
@@ -64,12 +104,18 @@ __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables
             double cv[U];
 #pragma unroll
             for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u + 1) * cs];
+            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                x = __ddiv_rn(sub(cv[u], x), tb.dp[i - u]);
-                c[(long long)(i - u + 1) * cs] = x;
+                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
+            } else {
+#pragma unroll 1
+                for (int k = i; k > i - U; k--) {
+                    x = __ddiv_rn(sub(c[(long long)(k + 1) * cs], x), tb.dp[k]);
+                    c[(long long)(k + 1) * cs] = x;
+                }
             }
         }
+#pragma unroll 1
         for (; i >= 1; i--) {
             x = __ddiv_rn(sub(c[(long long)(i + 1) * cs], x), tb.dp[i]);
             c[(long long)(i + 1) * cs] = x;
@@ -92,7 +138,7 @@ __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables
             for (int u = 0; u < U; u++) fv[u] = f(i + u);
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                rp = sub(mul(6.0, fv[u]), mul(tb.mt[i + u], rp));
+                rp = sub(mul(6.0, fv[u]), mul(i > kPivotRows ? r_inf : tb.mt[i + u], rp));
                 c[(long long)(i + u + 1) * cs] = rp;
             }
         }
@@ -107,12 +153,18 @@ __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables
             double cv[U];
 #pragma unroll
             for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u + 1) * cs];
+            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                x = __ddiv_rn(sub(cv[u], x), tb.dp[i - u]);
-                c[(long long)(i - u + 1) * cs] = x;
+                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
+            } else {
+#pragma unroll 1
+                for (int k = i; k > i - U; k--) {
+                    x = __ddiv_rn(sub(c[(long long)(k + 1) * cs], x), tb.dp[k]);
+                    c[(long long)(k + 1) * cs] = x;
+                }
             }
         }
+#pragma unroll 1
         for (; i >= 0; i--) {
             x = __ddiv_rn(sub(c[(long long)(i + 1) * cs], x), tb.dp[i]);
             c[(long long)(i + 1) * cs] = x;
@@ -132,14 +184,16 @@ __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables
 template <int U, class Src>
 __device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTables& tb, double* c, long long cs)
 {
+    double d_inf, r_inf;
+    fixed_pivots(N, tb, d_inf, r_inf);
     if (!periodic) {
         const double c0 = f(0), cl = f(N - 1);
         double rp = 0.0;
-        auto fwd = [&](int i, double fi) {
+        auto fwd = [&](int i, double fi, double m) {
             double r = mul(6.0, fi);
             if (i == 1) r = sub(r, c0);
             if (i == N - 2) r = sub(r, cl);
-            rp = (i == 1) ? r : sub(r, mul(tb.mt[i], rp));
+            rp = (i == 1) ? r : sub(r, mul(m, rp));
             c[(long long)i * cs] = rp;
         };
         int i = 1;
@@ -148,9 +202,9 @@ __device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTab
 #pragma unroll
             for (int u = 0; u < U; u++) fv[u] = f(i + u);
 #pragma unroll
-            for (int u = 0; u < U; u++) fwd(i + u, fv[u]);
+            for (int u = 0; u < U; u++) fwd(i + u, fv[u], i > kPivotRows ? r_inf : tb.mt[i + u]);
         }
-        for (; i <= N - 2; i++) fwd(i, f(i));
+        for (; i <= N - 2; i++) fwd(i, f(i), tb.mt[i]);
         double x = __ddiv_rn(c[(long long)(N - 2) * cs], tb.dp[N - 2]);
         c[(long long)(N - 1) * cs] = x;
         i = N - 3;
@@ -158,12 +212,18 @@ __device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTab
             double cv[U];
 #pragma unroll
             for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u) * cs];
+            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                x = __ddiv_rn(sub(cv[u], x), tb.dp[i - u]);
-                c[(long long)(i - u + 1) * cs] = x;
+                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
+            } else {
+#pragma unroll 1
+                for (int k = i; k > i - U; k--) {
+                    x = __ddiv_rn(sub(c[(long long)(k) * cs], x), tb.dp[k]);
+                    c[(long long)(k + 1) * cs] = x;
+                }
             }
         }
+#pragma unroll 1
         for (; i >= 1; i--) {
             x = __ddiv_rn(sub(c[(long long)i * cs], x), tb.dp[i]);
             c[(long long)(i + 1) * cs] = x;
@@ -184,7 +244,7 @@ __device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTab
             for (int u = 0; u < U; u++) fv[u] = f(i + u);
 #pragma unroll
             for (int u = 0; u < U; u++) {
-                rp = sub(mul(6.0, fv[u]), mul(tb.mt[i + u], rp));
+                rp = sub(mul(6.0, fv[u]), mul(i > kPivotRows ? r_inf : tb.mt[i + u], rp));
                 c[(long long)(i + u) * cs] = rp;
             }
         }
@@ -199,12 +259,18 @@ __device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTab
             double cv[U];
 #pragma unroll
             for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u) * cs];
+            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
 #pragma unroll
-            for (int u = 0; u < U; u++) {
-                x = __ddiv_rn(sub(cv[u], x), tb.dp[i - u]);
-                c[(long long)(i - u + 1) * cs] = x;
+                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
+            } else {
+#pragma unroll 1
+                for (int k = i; k > i - U; k--) {
+                    x = __ddiv_rn(sub(c[(long long)(k) * cs], x), tb.dp[k]);
+                    c[(long long)(k + 1) * cs] = x;
+                }
             }
         }
+#pragma unroll 1
         for (; i >= 0; i--) {
             x = __ddiv_rn(sub(c[(long long)i * cs], x), tb.dp[i]);
             c[(long long)(i + 1) * cs] = x;
@@ -233,8 +299,9 @@ __device__ __forceinline__ double spline_source(const double* __restrict__ W, lo
     return mul(mul(d, gm1), sub(__ddiv_rn(W[4 * nt3 + idx], d), mul(0.5, vs)));
 }
 
-// pass 0: the data of source q along axis 0 (y) -> out [M0][N1][N2]; one line (i, k)
-template <int U>
+// pass 0: the data of source q along axis 0 (y) -> out [M0][N1][N2]; one line (i, k).  VEL: q is a
+// velocity (1..3), whose source alone is compiled in.
+template <int U, bool VEL>
 __device__ __forceinline__ void pass0_line(const double* __restrict__ W, const FieldConst& fc, const SplineGrid& g,
                                            const SplineTables& tb, int q, double* __restrict__ out, long long L,
                                            long long stride = 0)
@@ -247,16 +314,21 @@ __device__ __forceinline__ void pass0_line(const double* __restrict__ W, const F
     const int i = (int)(L / N), k = (int)(L - (long long)i * N);
     const long long base = (long long)(i + off) * nt + (k + off);
     const long long sj = (long long)nt * nt;
-    auto f = [&](int j) { return spline_source(W, nt3, fc.gm1, q, (long long)(j + off) * sj + base); };
+    auto f = [&](int j) {
+        const long long idx = (long long)(j + off) * sj + base;
+        if constexpr (VEL) return __ddiv_rn(W[q * nt3 + idx], W[idx]);
+        else return spline_source(W, nt3, fc.gm1, q, idx);
+    };
     line_solve<U>(f, N, g.periodic, tb, out + L, lines);
 }
 
+template <bool VEL>
 __global__ void spline_pass0(const double* __restrict__ W, FieldConst fc, SplineGrid g, SplineTables tb, int q,
                              double* __restrict__ out)
 {
     const long long lines = (long long)g.npts * g.npts;
     for (long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x; L < lines; L += (long long)gridDim.x * blockDim.x)
-        pass0_line<kLineBatchSingle>(W, fc, g, tb, q, out, L);
+        pass0_line<kLineBatchSingle, VEL>(W, fc, g, tb, q, out, L);
 }
 
 // pass 1: [M0][N1][N2] along axis 1 -> [M0][M1][N2]; one line (a, k)
@@ -286,6 +358,57 @@ __global__ void spline_pass1(const double* __restrict__ in, SplineGrid g, Spline
 // same order, so the coefficients are identical.
 constexpr int kLineChunk = 32;
 constexpr int kPass2Warps = 4;
+
+// Rows of one line staged in shared memory: row[t] holds point i0 + t.  Forward elimination of the
+// points [i_lo, i_hi] in that chunk, and back substitution of the same points downwards (the
+// line's last row, whose pivot has no tabled reciprocal, divided first).
+__device__ __forceinline__ void chunk_forward(double* row, int i0, int i_lo, int i_hi, int N, int periodic,
+                                              const SplineTables& tb, double c0, double cl, double r_inf, double& rp)
+{
+    const int a = max(i_lo, i0), b = min(i_hi, i0 + kLineChunk - 1);
+#pragma unroll 8
+    for (int i = a; i <= b; i++) {
+        double r = mul(6.0, row[i - i0]);
+        if (!periodic) {
+            if (i == 1) r = sub(r, c0);
+            if (i == N - 2) r = sub(r, cl);
+        }
+        rp = (i == i_lo) ? r : sub(r, mul(i > kPivotRows ? r_inf : tb.mt[i], rp));
+        row[i - i0] = rp;
+    }
+}
+__device__ __forceinline__ void chunk_back(double* row, int i0, int i_lo, int i_hi, const SplineTables& tb, double d_inf,
+                                           double r_inf, double& x)
+{
+    const int a = max(i_lo, i0);
+    int i = min(i_hi, i0 + kLineChunk - 1);
+    if (i == i_hi && i >= a) {
+        x = __ddiv_rn(row[i - i0], tb.dp[i]);
+        row[i - i0] = x;
+        i--;
+    }
+    constexpr int U = 8;
+    for (; i - U + 1 >= a; i -= U) {
+        double cv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) cv[u] = row[i - u - i0];
+        if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
+#pragma unroll
+            for (int u = 0; u < U; u++) row[i - u - i0] = cv[u];
+        } else {
+#pragma unroll 1
+            for (int k = i; k > i - U; k--) {
+                x = __ddiv_rn(sub(row[k - i0], x), tb.dp[k]);
+                row[k - i0] = x;
+            }
+        }
+    }
+#pragma unroll 1
+    for (; i >= a; i--) {
+        x = __ddiv_rn(sub(row[i - i0], x), tb.dp[i]);
+        row[i - i0] = x;
+    }
+}
 
 // lines [L0, L0 + 32) of a pass-2 input (lines total), by one warp with its staging rows sm.
 // Chunks are 32 output slots [s0, s0 + 32), holding values s0 - 1 .. s0 + 30 of the line (value i
@@ -323,6 +446,8 @@ __device__ __forceinline__ void pass2_group(const double* __restrict__ in, const
         __syncwarp();
     };
     const int s_last = (N / kLineChunk) * kLineChunk;   // the chunk holding slot N
+    double d_inf, r_inf;
+    fixed_pivots(N, tb, d_inf, r_inf);
     const double* src = in + myL * N;
     double* dst = out + myL * M;
     if (!g.periodic) {
@@ -331,31 +456,18 @@ __device__ __forceinline__ void pass2_group(const double* __restrict__ in, const
         double rp = 0.0;
         for (int s0 = 0; s0 <= s_last; s0 += kLineChunk) {
             load_in(s0);
-            if (mine)
-                for (int t = 0; t < kLineChunk; t++) {
-                    const int i = s0 - 1 + t;
-                    if (i < 1 || i > N - 2) continue;
-                    double r = mul(6.0, sm[lane][t]);
-                    if (i == 1) r = sub(r, c0);
-                    if (i == N - 2) r = sub(r, cl);
-                    rp = (i == 1) ? r : sub(r, mul(tb.mt[i], rp));
-                    sm[lane][t] = rp;
-                }
+            if (mine) chunk_forward(sm[lane], s0 - 1, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
             store_out(s0);
         }
         // back substitution, chunks in descending order
         double x = 0.0, x1 = 0.0, xl2 = 0.0;
         for (int s0 = s_last; s0 >= 0; s0 -= kLineChunk) {
             load_out(s0);
-            if (mine)
-                for (int t = kLineChunk - 1; t >= 0; t--) {
-                    const int i = s0 - 1 + t;
-                    if (i < 1 || i > N - 2) continue;
-                    x = (i == N - 2) ? __ddiv_rn(sm[lane][t], tb.dp[N - 2]) : __ddiv_rn(sub(sm[lane][t], x), tb.dp[i]);
-                    sm[lane][t] = x;
-                    if (i == N - 2) xl2 = x;
-                    if (i == 1) x1 = x;
-                }
+            if (mine) {
+                chunk_back(sm[lane], s0 - 1, 1, N - 2, tb, d_inf, r_inf, x);
+                if (s0 - 1 <= N - 2 && N - 2 < s0 - 1 + kLineChunk) xl2 = sm[lane][N - 2 - (s0 - 1)];
+                x1 = x;   // the last chunk's last value is the solution of point 1
+            }
             store_out(s0);
         }
         if (mine) {
@@ -368,27 +480,17 @@ __device__ __forceinline__ void pass2_group(const double* __restrict__ in, const
         double rp = 0.0;
         for (int s0 = 0; s0 <= s_last; s0 += kLineChunk) {
             load_in(s0);
-            if (mine)
-                for (int t = 0; t < kLineChunk; t++) {
-                    const int i = s0 - 1 + t;
-                    if (i < 0 || i > N - 1) continue;
-                    rp = (i == 0) ? mul(6.0, sm[lane][t]) : sub(mul(6.0, sm[lane][t]), mul(tb.mt[i], rp));
-                    sm[lane][t] = rp;
-                }
+            if (mine) chunk_forward(sm[lane], s0 - 1, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
             store_out(s0);
         }
         double x = 0.0, x0 = 0.0, xl = 0.0;
         for (int s0 = s_last; s0 >= 0; s0 -= kLineChunk) {
             load_out(s0);
-            if (mine)
-                for (int t = kLineChunk - 1; t >= 0; t--) {
-                    const int i = s0 - 1 + t;
-                    if (i < 0 || i > N - 1) continue;
-                    x = (i == N - 1) ? __ddiv_rn(sm[lane][t], tb.dp[N - 1]) : __ddiv_rn(sub(sm[lane][t], x), tb.dp[i]);
-                    sm[lane][t] = x;
-                    if (i == N - 1) xl = x;
-                    if (i == 0) x0 = x;
-                }
+            if (mine) {
+                chunk_back(sm[lane], s0 - 1, 0, N - 1, tb, d_inf, r_inf, x);
+                if (s0 - 1 <= N - 1 && N - 1 < s0 - 1 + kLineChunk) xl = sm[lane][N - 1 - (s0 - 1)];
+                x0 = x;   // the last chunk's last value is the solution of point 0
+            }
             store_out(s0);
         }
         const double fac = mine ? __ddiv_rn(add(x0, mul(-0.25, xl)), tb.denom) : 0.0;
@@ -438,7 +540,7 @@ __global__ void spline_pass0_room(const double* __restrict__ W, FieldConst fc, S
     const long long lines = (long long)g.npts * g.npts;
     const long long stride = (long long)(g.npts + g.pad) * g.npts;
     for (long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x; L < lines; L += (long long)gridDim.x * blockDim.x)
-        pass0_line<kLineBatchSingle>(W, fc, g, tb, q, out, L, stride);
+        pass0_line<kLineBatchSingle, true>(W, fc, g, tb, q, out, L, stride);
 }
 
 // pass 1 in place on [M0][M1][N2]: line (a, k) reads rows 0..N-1 and writes rows 0..M-1
@@ -496,35 +598,24 @@ __device__ __forceinline__ void pass2_group_f32(double* in, const SplineGrid& g,
     const double* src = in + myL * N;
     float* dst = out + myL * M;
     const int top = ((N - 1) / kLineChunk) * kLineChunk;
+    double d_inf, r_inf;
+    fixed_pivots(N, tb, d_inf, r_inf);
     if (!g.periodic) {
         const double c0 = mine ? src[0] : 0.0, cl = mine ? src[N - 1] : 0.0;
         double rp = 0.0;
         for (int k0 = 0; k0 < N; k0 += kLineChunk) {
             load(k0);
-            if (mine)
-                for (int t = 0; t < kLineChunk && k0 + t < N; t++) {
-                    const int i = k0 + t;
-                    if (i < 1 || i > N - 2) continue;
-                    double r = mul(6.0, sm[lane][t]);
-                    if (i == 1) r = sub(r, c0);
-                    if (i == N - 2) r = sub(r, cl);
-                    rp = (i == 1) ? r : sub(r, mul(tb.mt[i], rp));
-                    sm[lane][t] = rp;
-                }
+            if (mine) chunk_forward(sm[lane], k0, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
             store(k0, 0, N);
         }
         double x = 0.0, x1 = 0.0, xl2 = 0.0;
         for (int k0 = top; k0 >= 0; k0 -= kLineChunk) {
             load(k0);
-            if (mine)
-                for (int t = kLineChunk - 1; t >= 0; t--) {
-                    const int i = k0 + t;
-                    if (i < 1 || i > N - 2) continue;
-                    x = (i == N - 2) ? __ddiv_rn(sm[lane][t], tb.dp[N - 2]) : __ddiv_rn(sub(sm[lane][t], x), tb.dp[i]);
-                    sm[lane][t] = x;
-                    if (i == N - 2) xl2 = x;
-                    if (i == 1) x1 = x;
-                }
+            if (mine) {
+                chunk_back(sm[lane], k0, 1, N - 2, tb, d_inf, r_inf, x);
+                if (k0 <= N - 2 && N - 2 < k0 + kLineChunk) xl2 = sm[lane][N - 2 - k0];
+                x1 = x;
+            }
             emit(k0, 1, N - 1, 1);   // the solution of point i is coefficient i + 1 (1 <= i <= N-2)
         }
         if (mine) {
@@ -537,26 +628,17 @@ __device__ __forceinline__ void pass2_group_f32(double* in, const SplineGrid& g,
         double rp = 0.0;
         for (int k0 = 0; k0 < N; k0 += kLineChunk) {
             load(k0);
-            if (mine)
-                for (int t = 0; t < kLineChunk && k0 + t < N; t++) {
-                    const int i = k0 + t;
-                    rp = (i == 0) ? mul(6.0, sm[lane][t]) : sub(mul(6.0, sm[lane][t]), mul(tb.mt[i], rp));
-                    sm[lane][t] = rp;
-                }
+            if (mine) chunk_forward(sm[lane], k0, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
             store(k0, 0, N);
         }
         double x = 0.0, x0 = 0.0, xl = 0.0;
         for (int k0 = top; k0 >= 0; k0 -= kLineChunk) {
             load(k0);
-            if (mine)
-                for (int t = kLineChunk - 1; t >= 0; t--) {
-                    const int i = k0 + t;
-                    if (i > N - 1) continue;
-                    x = (i == N - 1) ? __ddiv_rn(sm[lane][t], tb.dp[N - 1]) : __ddiv_rn(sub(sm[lane][t], x), tb.dp[i]);
-                    sm[lane][t] = x;
-                    if (i == N - 1) xl = x;
-                    if (i == 0) x0 = x;
-                }
+            if (mine) {
+                chunk_back(sm[lane], k0, 0, N - 1, tb, d_inf, r_inf, x);
+                if (k0 <= N - 1 && N - 1 < k0 + kLineChunk) xl = sm[lane][N - 1 - k0];
+                x0 = x;
+            }
             store(k0, 1, N - 1);
         }
         const double fac = mine ? __ddiv_rn(add(x0, mul(-0.25, xl)), tb.denom) : 0.0;
@@ -594,6 +676,281 @@ __global__ void __launch_bounds__(32 * kPass2Warps) spline_pass2_f32(double* in,
     const long long nwarps = (long long)gridDim.x * kPass2Warps;
     for (long long L0 = ((long long)blockIdx.x * kPass2Warps + warp) * 32; L0 < lines; L0 += nwarps * 32)
         pass2_group_f32(in, g, tb, out, L0, lines, stage[warp]);
+}
+
+// ---- lines resident in shared memory.  A warp (one CTA) takes 32 lines: their values come in at
+// once, all loads in flight, each lane solves its line in place, and the coefficients go out, so a
+// pass reads and writes global memory once.  The forward values of the kernels above make the round
+// through global memory instead, and their loads wait on one another 4 or 8 at a time.  What
+// remains is the lanes' serial chain, which pivot_quotient keeps short.
+// How many warps of such lines an SM holds decides where it pays.  Velocity splines, ms, streaming
+// kernels against these: three components per launch 64^3 0.099 -> 0.048, 128^3 0.270 -> 0.157, 160^3 0.390 ->
+// 0.338, 192^3 0.817 -> 0.640, 224^3 1.08 -> 1.16, 256^3 1.42 -> 1.65; one component per launch (coefficients in
+// FP32) 128^3 0.511 -> 0.198, 224^3 1.28 -> 1.09, 256^3 1.65 -> 1.50, 282^3 1.80 -> 1.90.
+constexpr int kResidentBatched = 200, kResidentSingle = 264;
+constexpr int kTableRows = kPivotRows + 2;   // rows of the tables a warp keeps beside its lines
+inline size_t resident_bytes(int npts) { return sizeof(double) * (2 * kTableRows + 32 * (size_t)(npts | 1)); }
+
+// 8-byte asynchronous copies, a thread's own (its wait covers them)
+__device__ __forceinline__ void copy8_async(double* dst, const double* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait()
+{
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+}
+
+// the first rows of the pivot tables in shared memory (mt, then dp), the later ones' fixed point
+struct LineTables {
+    const double *mt, *dp;
+    double d_inf, r_inf, d_last;
+    __device__ __forceinline__ double m(int i) const { return i < kTableRows ? mt[i] : r_inf; }
+    __device__ __forceinline__ double d(int i) const { return i < kTableRows ? dp[i] : d_inf; }
+};
+// issued with the lines' own copies; the caller waits and synchronises the warp
+__device__ __forceinline__ LineTables line_tables(const SplineTables& tb, int N, int periodic, double* smem)
+{
+    const int lane = threadIdx.x;
+    if (lane < kTableRows && lane <= N) {
+        copy8_async(smem + lane, tb.mt + lane);
+        copy8_async(smem + kTableRows + lane, tb.dp + lane);
+    }
+    LineTables T;
+    T.mt = smem;
+    T.dp = smem + kTableRows;
+    fixed_pivots(N, tb, T.d_inf, T.r_inf);
+    T.d_last = tb.dp[periodic ? N - 1 : N - 2];
+    return T;
+}
+
+// one line in place in shared memory, point i at s[i * st]: on return s holds the coefficients of points
+// 0..N-1 (natural ends: lo and hi the ones outside).  The arithmetic and its order are line_solve's.
+__device__ __forceinline__ void resident_solve(double* s, int st, int N, int periodic, const LineTables& T,
+                                               const SplineTables& tb, double& lo, double& hi)
+{
+    const int i_lo = periodic ? 0 : 1, i_hi = periodic ? N - 1 : N - 2;
+    const double c0 = s[0], cl = s[(N - 1) * st];
+    double rp = 0.0;
+    constexpr int U = 8;
+    auto fwd = [&](int i, double fi) {
+        double r = mul(6.0, fi);
+        if (!periodic) {
+            if (i == 1) r = sub(r, c0);
+            if (i == N - 2) r = sub(r, cl);
+        }
+        rp = (i == i_lo) ? r : sub(r, mul(T.m(i), rp));
+        s[i * st] = rp;
+    };
+    int i = i_lo;
+    for (; i + U - 1 <= i_hi; i += U) {
+        double fv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) fv[u] = s[(i + u) * st];
+        if (i > kPivotRows && i + U - 1 < N - 2) {   // the inner rows
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                rp = sub(mul(6.0, fv[u]), mul(T.r_inf, rp));
+                s[(i + u) * st] = rp;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < U; u++) fwd(i + u, fv[u]);
+        }
+    }
+#pragma unroll 1
+    for (; i <= i_hi; i++) fwd(i, s[i * st]);
+    double x = __ddiv_rn(rp, T.d_last);
+    s[i_hi * st] = x;
+    const double x_hi = x;
+    i = i_hi - 1;
+    auto back = [&](int k) {
+        const double a = sub(s[k * st], x), d = T.d(k);
+        x = pivot_in_range(a) ? pivot_quotient(a, d, T.m(k + 1)) : __ddiv_rn(a, d);
+        s[k * st] = x;
+    };
+    for (; i - U + 1 >= i_lo; i -= U) {
+        const bool fixed = i - U + 1 >= kPivotRows;
+        double cv[U], y = x;
+        bool ok = true;
+#pragma unroll
+        for (int u = 0; u < U; u++) cv[u] = s[(i - u) * st];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const double d = fixed ? T.d_inf : T.d(i - u), r = fixed ? T.r_inf : T.m(i - u + 1);
+            const double a = sub(cv[u], y);
+            ok = ok && pivot_in_range(a);
+            y = pivot_quotient(a, d, r);
+            cv[u] = y;
+        }
+        if (ok) {
+            x = y;
+#pragma unroll
+            for (int u = 0; u < U; u++) s[(i - u) * st] = cv[u];
+        } else {
+#pragma unroll 1
+            for (int k = i; k > i - U; k--) back(k);
+        }
+    }
+#pragma unroll 1
+    for (; i >= i_lo; i--) back(i);
+    if (!periodic) {
+        // x is the solution of point 1 (N >= 4)
+        lo = sub(2.0 * c0, x);
+        hi = sub(2.0 * cl, x_hi);
+    } else {
+        const double fac = __ddiv_rn(add(x, mul(-0.25, x_hi)), tb.denom);
+#pragma unroll 8
+        for (int k = 0; k < N; k++) s[k * st] = sub(s[k * st], mul(fac, tb.z[k]));
+        lo = hi = 0.0;
+    }
+}
+
+// strided lines (passes 0 and 1): lane's column of s to c, stride cs
+__device__ __forceinline__ void resident_store(const double* s, int N, int periodic, double lo, double hi, double* c,
+                                               long long cs)
+{
+#pragma unroll 8
+    for (int i = 0; i < N; i++) c[(long long)(i + 1) * cs] = s[i * 32];
+    if (!periodic) {
+        c[0] = lo;
+        c[(long long)(N + 1) * cs] = hi;
+    } else {
+        c[0] = s[(N - 1) * 32];
+        c[(long long)(N + 1) * cs] = s[0];
+        c[(long long)(N + 2) * cs] = s[32];
+    }
+}
+
+// pass 0, lines [32 group, 32 group + 32) of source q along axis 0 -> out, `stride` apart along axis 0
+template <bool VEL>
+__device__ __forceinline__ void resident_pass0(const double* __restrict__ W, const FieldConst& fc, const SplineGrid& g,
+                                               const SplineTables& tb, int q, double* __restrict__ out, long long stride,
+                                               long long group, double* smem)
+{
+    const int N = g.npts, lane = threadIdx.x;
+    const LineTables T = line_tables(tb, N, g.periodic, smem);
+    const bool mine = group * 32 + lane < (long long)N * N;
+    const long long L = mine ? group * 32 + lane : (long long)N * N - 1;   // a lane beyond the lines repeats the last
+    const int off = g.periodic ? 3 : 0, nt = fc.nt;
+    const int i = (int)(L / N), k = (int)(L - (long long)i * N);
+    const long long sj = (long long)nt * nt, base = off * sj + (long long)(i + off) * nt + (k + off), nt3 = fc.nt3;
+    double* s = smem + 2 * kTableRows + lane;
+    if constexpr (VEL) {   // the next rows' loads are issued before this batch's divisions
+        constexpr int U = 8;
+        const double* pd = W + base;
+        const double* pm = pd + q * nt3;
+        double d[U], m[U], dn[U], mn[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long o = min(u, N - 1) * sj;
+            d[u] = pd[o];
+            m[u] = pm[o];
+        }
+        for (int j = 0; j < N; j += U) {
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const long long o = min(j + U + u, N - 1) * sj;
+                dn[u] = pd[o];
+                mn[u] = pm[o];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (j + u < N) s[(j + u) * 32] = __ddiv_rn(m[u], d[u]);
+                d[u] = dn[u];
+                m[u] = mn[u];
+            }
+        }
+    } else {
+#pragma unroll 4
+        for (int j = 0; j < N; j++) s[j * 32] = spline_source(W, nt3, fc.gm1, q, base + j * sj);
+    }
+    copy_async_wait();
+    __syncwarp();
+    if (!mine) return;
+    double lo, hi;
+    resident_solve(s, 32, N, g.periodic, T, tb, lo, hi);
+    resident_store(s, N, g.periodic, lo, hi, out + L, stride);
+}
+
+// pass 1, lines of [M0][in_rows][N2] along axis 1 -> [M0][M1][N2] (in place where in == out and in_rows = M)
+__device__ __forceinline__ void resident_pass1(const double* in, int in_rows, const SplineGrid& g, const SplineTables& tb,
+                                               double* out, long long group, double* smem)
+{
+    const int N = g.npts, M = N + g.pad, lane = threadIdx.x;
+    const LineTables T = line_tables(tb, N, g.periodic, smem);
+    const bool mine = group * 32 + lane < (long long)M * N;
+    const long long L = mine ? group * 32 + lane : (long long)M * N - 1;
+    const int a = (int)(L / N), k = (int)(L - (long long)a * N);
+    const double* src = in + (long long)a * in_rows * N + k;
+    double* s = smem + 2 * kTableRows + lane;
+    if (mine) {
+#pragma unroll 8
+        for (int i = 0; i < N; i++) copy8_async(s + i * 32, src + (long long)i * N);
+    }
+    copy_async_wait();
+    __syncwarp();
+    if (!mine) return;
+    double lo, hi;
+    resident_solve(s, 32, N, g.periodic, T, tb, lo, hi);
+    resident_store(s, N, g.periodic, lo, hi, out + (long long)a * M * N + k, N);
+}
+
+// pass 2, the contiguous lines of [M0][M1][N2] -> [M0][M1][M2]: rows move coalesced, lane j solves row j
+// (rows an odd number of doubles apart: no bank conflicts); the stores start on the output's sectors
+template <class OutT>
+__device__ __forceinline__ void resident_pass2(const double* __restrict__ in, const SplineGrid& g, const SplineTables& tb,
+                                               OutT* __restrict__ out, long long group, double* smem)
+{
+    const int N = g.npts, M = N + g.pad, S = N | 1, lane = threadIdx.x;
+    const long long lines = (long long)M * M, L0 = group * 32;
+    const int nl = (int)min(32LL, lines - L0);
+    const LineTables T = line_tables(tb, N, g.periodic, smem);
+    smem += 2 * kTableRows;
+    for (int j = 0; j < nl; j++)
+        for (int k = lane; k < N; k += 32) copy8_async(smem + j * S + k, in + (L0 + j) * N + k);
+    copy_async_wait();
+    __syncwarp();
+    if (lane < nl) {
+        double lo, hi;
+        double* s = smem + lane * S;
+        resident_solve(s, 1, N, g.periodic, T, tb, lo, hi);
+        OutT* dst = out + (L0 + lane) * M;
+        if (!g.periodic) {
+            dst[0] = (OutT)lo;
+            dst[N + 1] = (OutT)hi;
+        } else {
+            dst[0] = (OutT)s[N - 1];
+            dst[N + 1] = (OutT)s[0];
+            dst[N + 2] = (OutT)s[1];
+        }
+    }
+    __syncwarp();
+    for (int j = 0; j < nl; j++)
+        for (int sl = lane; sl <= N; sl += 32)
+            if (sl > 0) out[(L0 + j) * M + sl] = (OutT)smem[j * S + sl - 1];
+}
+
+template <bool VEL>
+__global__ void __launch_bounds__(32) spline_resident0(const double* __restrict__ W, FieldConst fc, SplineGrid g,
+                                                       SplineTables tb, int q, double* __restrict__ out, long long stride)
+{
+    extern __shared__ double line_smem[];
+    resident_pass0<VEL>(W, fc, g, tb, q, out, stride, blockIdx.x, line_smem);
+}
+__global__ void __launch_bounds__(32) spline_resident1(const double* in, int in_rows, SplineGrid g, SplineTables tb,
+                                                       double* out)
+{
+    extern __shared__ double line_smem[];
+    resident_pass1(in, in_rows, g, tb, out, blockIdx.x, line_smem);
+}
+template <class OutT>
+__global__ void __launch_bounds__(32) spline_resident2(const double* __restrict__ in, SplineGrid g, SplineTables tb,
+                                                       OutT* __restrict__ out)
+{
+    extern __shared__ double line_smem[];
+    resident_pass2<OutT>(in, g, tb, out, blockIdx.x, line_smem);
 }
 
 struct Basis {
@@ -1151,31 +1508,75 @@ cudaError_t grid_launch(K kernel, long long work, int threads, cudaStream_t s, A
     return cudaGetLastError();
 }
 
-// ---- ensemble forms: one launch per pass over every member's lines / particles
+// ---- ensemble forms: one launch per pass over every member's lines / particles; the lines in groups of
+// 32, one warp each, off[] the members' groups of all three components
+__device__ __forceinline__ const MemberDev& ensemble_group(const MemberDev* __restrict__ mem,
+                                                           const long long* __restrict__ off, int nm, long long w,
+                                                           int pass, int& q, long long& group)
+{
+    const int m = find_member(off, nm, w);
+    const MemberDev& md = mem[m];
+    const long long local = w - off[m], groups = spline_groups(pass, md.grid.npts, md.grid.pad);
+    q = (int)(local / groups);
+    group = local - q * groups;
+    return md;
+}
+
+__global__ void __launch_bounds__(32) ensemble_resident0(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
+                                                         int nm, int buf)
+{
+    extern __shared__ double line_smem[];
+    int q;
+    long long group;
+    const MemberDev& md = ensemble_group(mem, off, nm, blockIdx.x, 0, q, group);
+    resident_pass0<true>(md.buf[buf], md.fc, md.grid, md.tb, q + 1, md.coef[q], (long long)md.grid.npts * md.grid.npts,
+                         group, line_smem);
+}
+__global__ void __launch_bounds__(32) ensemble_resident1(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
+                                                         int nm)
+{
+    extern __shared__ double line_smem[];
+    int q;
+    long long group;
+    const MemberDev& md = ensemble_group(mem, off, nm, blockIdx.x, 1, q, group);
+    resident_pass1(md.coef[q], md.grid.npts, md.grid, md.tb, md.scratch[q], group, line_smem);
+}
+__global__ void __launch_bounds__(32) ensemble_resident2(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
+                                                         int nm)
+{
+    extern __shared__ double line_smem[];
+    int q;
+    long long group;
+    const MemberDev& md = ensemble_group(mem, off, nm, blockIdx.x, 2, q, group);
+    resident_pass2<double>(md.scratch[q], md.grid, md.tb, md.coef[q], group, line_smem);
+}
+
 __global__ void __launch_bounds__(128, kPassCtasPerSm) ensemble_pass0_kernel(const MemberDev* __restrict__ mem, const long long* __restrict__ off, int nm,
                                       int buf)
 {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long total = off[nm];
-    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-        const int m = find_member(off, nm, x);
-        const MemberDev& md = mem[m];
-        const long long local = x - off[m];
-        const long long lines = (long long)md.grid.npts * md.grid.npts;
-        const int q = (int)(local / lines);
-        pass0_line<kLineBatchBatched>(md.buf[buf], md.fc, md.grid, md.tb, q + 1, md.coef[q], local - q * lines);
+    for (long long w = (long long)blockIdx.x * 4 + warp; w < total; w += (long long)gridDim.x * 4) {
+        int q;
+        long long group;
+        const MemberDev& md = ensemble_group(mem, off, nm, w, 0, q, group);
+        const long long L = group * 32 + lane;
+        if (L < (long long)md.grid.npts * md.grid.npts)
+            pass0_line<kLineBatchBatched, true>(md.buf[buf], md.fc, md.grid, md.tb, q + 1, md.coef[q], L);
     }
 }
 
 __global__ void __launch_bounds__(128, kPassCtasPerSm) ensemble_pass1_kernel(const MemberDev* __restrict__ mem, const long long* __restrict__ off, int nm)
 {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long total = off[nm];
-    for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-        const int m = find_member(off, nm, x);
-        const MemberDev& md = mem[m];
-        const long long local = x - off[m];
-        const long long lines = (long long)(md.grid.npts + md.grid.pad) * md.grid.npts;
-        const int q = (int)(local / lines);
-        pass1_line<kLineBatchBatched>(md.coef[q], md.grid, md.tb, md.scratch[q], local - q * lines);
+    for (long long w = (long long)blockIdx.x * 4 + warp; w < total; w += (long long)gridDim.x * 4) {
+        int q;
+        long long group;
+        const MemberDev& md = ensemble_group(mem, off, nm, w, 1, q, group);
+        const long long L = group * 32 + lane;
+        if (L < (long long)(md.grid.npts + md.grid.pad) * md.grid.npts)
+            pass1_line<kLineBatchBatched>(md.coef[q], md.grid, md.tb, md.scratch[q], L);
     }
 }
 
@@ -1186,13 +1587,11 @@ __global__ void __launch_bounds__(32 * kPass2Warps, kPassCtasPerSm)
     const int warp = threadIdx.x >> 5;
     const long long total = off[nm];
     for (long long w = (long long)blockIdx.x * kPass2Warps + warp; w < total; w += (long long)gridDim.x * kPass2Warps) {
-        const int m = find_member(off, nm, w);
-        const MemberDev& md = mem[m];
-        const long long local = w - off[m];
+        int q;
+        long long group;
+        const MemberDev& md = ensemble_group(mem, off, nm, w, 2, q, group);
         const long long M = md.grid.npts + md.grid.pad;
-        const long long lines = M * M, groups = (lines + 31) / 32;
-        const int q = (int)(local / groups);
-        pass2_group(md.scratch[q], md.grid, md.tb, md.coef[q], (local - q * groups) * 32, lines, stage[warp]);
+        pass2_group(md.scratch[q], md.grid, md.tb, md.coef[q], group * 32, M * M, stage[warp]);
     }
 }
 
@@ -1208,6 +1607,41 @@ __global__ void ensemble_heun_kernel(const MemberDev* __restrict__ mem, const lo
     }
 }
 
+// the line kernels' shared-memory limit, on the current device
+cudaError_t resident_prepare()
+{
+    const int bytes = (int)resident_bytes(kResidentSingle > kResidentBatched ? kResidentSingle : kResidentBatched);
+    const void* kernels[] = {(const void*)spline_resident0<true>,    (const void*)spline_resident0<false>,
+                             (const void*)spline_resident1,          (const void*)spline_resident2<double>,
+                             (const void*)spline_resident2<float>,   (const void*)ensemble_resident0,
+                             (const void*)ensemble_resident1,        (const void*)ensemble_resident2};
+    for (const void* k : kernels) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// one component (kind q) through resident lines: pass 0 to `mid` (stride0 along axis 0), pass 1 to `buf`
+// (from in_rows rows per plane), pass 2 to out
+template <class OutT>
+cudaError_t resident_component(const double* W, const FieldConst& fc, const SplineGrid& g, const SplineTables& tb, int q,
+                               double* mid, long long stride0, int in_rows, double* buf, OutT* out, cudaStream_t s)
+{
+    const size_t smem = resident_bytes(g.npts);
+    const unsigned g0 = (unsigned)spline_groups(0, g.npts, g.pad), g1 = (unsigned)spline_groups(1, g.npts, g.pad),
+                   g2 = (unsigned)spline_groups(2, g.npts, g.pad);
+    if (q >= 1 && q <= 3) spline_resident0<true><<<g0, 32, smem, s>>>(W, fc, g, tb, q, mid, stride0);
+    else spline_resident0<false><<<g0, 32, smem, s>>>(W, fc, g, tb, q, mid, stride0);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    spline_resident1<<<g1, 32, smem, s>>>(mid, in_rows, g, tb, buf);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    spline_resident2<OutT><<<g2, 32, smem, s>>>(buf, g, tb, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_pass2(const double* in, const SplineGrid& g, const SplineTables& tb, double* out, cudaStream_t s)
 {
     const long long M = g.npts + g.pad;
@@ -1220,17 +1654,14 @@ cudaError_t launch_pass2(const double* in, const SplineGrid& g, const SplineTabl
 
 }  // namespace
 
+cudaError_t spline_prepare() { return resident_prepare(); }
+
 cudaError_t launch_spline_build(const double* W, const FieldConst& fc, const SplineGrid& g, const SplineTables& tb,
                                 double* coef_u, double* coef_v, double* coef_w, double* scratch, cudaStream_t s)
 {
     double* outs[3] = {coef_u, coef_v, coef_w};
-    const long long N = g.npts, M = N + g.pad;
     for (int f = 0; f < 3; f++) {
-        cudaError_t e = grid_launch(spline_pass0, N * N, 128, s, W, fc, g, tb, f + 1, outs[f]);
-        if (e != cudaSuccess) return e;
-        e = grid_launch(spline_pass1, M * N, 128, s, (const double*)outs[f], g, tb, scratch);
-        if (e != cudaSuccess) return e;
-        e = launch_pass2((const double*)scratch, g, tb, outs[f], s);
+        cudaError_t e = launch_spline_component(W, fc, g, tb, f + 1, outs[f], scratch, s);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1241,7 +1672,10 @@ cudaError_t launch_spline_component(const double* W, const FieldConst& fc, const
                                     int component, double* coef, double* scratch, cudaStream_t s)
 {
     const long long N = g.npts, M = N + g.pad;
-    cudaError_t e = grid_launch(spline_pass0, N * N, 128, s, W, fc, g, tb, component, coef);
+    if (N <= kResidentSingle) return resident_component(W, fc, g, tb, component, coef, N * N, (int)N, scratch, coef, s);
+    const bool vel = component >= 1 && component <= 3;
+    cudaError_t e = vel ? grid_launch(spline_pass0<true>, N * N, 128, s, W, fc, g, tb, component, coef)
+                        : grid_launch(spline_pass0<false>, N * N, 128, s, W, fc, g, tb, component, coef);
     if (e != cudaSuccess) return e;
     e = grid_launch(spline_pass1, M * N, 128, s, (const double*)coef, g, tb, scratch);
     if (e != cudaSuccess) return e;
@@ -1249,16 +1683,27 @@ cudaError_t launch_spline_component(const double* W, const FieldConst& fc, const
 }
 
 cudaError_t launch_ensemble_splines(const MemberDev* mem, const EnsembleWork& w, const long long totals[3], int nm,
-                                    int buf, cudaStream_t s)
+                                    int max_npts, int buf, cudaStream_t s)
 {
-    cudaError_t e = grid_launch(ensemble_pass0_kernel, totals[0], 128, s, mem, w.line0, nm, buf);
+    if (max_npts <= kResidentBatched) {
+        const size_t smem = resident_bytes(max_npts);
+        ensemble_resident0<<<(unsigned)totals[0], 32, smem, s>>>(mem, w.group0, nm, buf);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        ensemble_resident1<<<(unsigned)totals[1], 32, smem, s>>>(mem, w.group1, nm);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        ensemble_resident2<<<(unsigned)totals[2], 32, smem, s>>>(mem, w.group2, nm);
+        return cudaGetLastError();
+    }
+    cudaError_t e = grid_launch(ensemble_pass0_kernel, totals[0] * 32, 128, s, mem, w.group0, nm, buf);
     if (e != cudaSuccess) return e;
-    e = grid_launch(ensemble_pass1_kernel, totals[1], 128, s, mem, w.line1, nm);
+    e = grid_launch(ensemble_pass1_kernel, totals[1] * 32, 128, s, mem, w.group1, nm);
     if (e != cudaSuccess) return e;
     long long b = (totals[2] + kPass2Warps - 1) / kPass2Warps;
     if (b < 1) b = 1;
     if (b > 148 * 16) b = 148 * 16;
-    ensemble_pass2_kernel<<<(unsigned)b, 32 * kPass2Warps, 0, s>>>(mem, w.warp2, nm);
+    ensemble_pass2_kernel<<<(unsigned)b, 32 * kPass2Warps, 0, s>>>(mem, w.group2, nm);
     return cudaGetLastError();
 }
 
@@ -1426,6 +1871,11 @@ cudaError_t launch_spline_build_f32(const double* W, const FieldConst& fc, const
     float* outs[3] = {coef_u, coef_v, coef_w};
     const long long N = g.npts, M = N + g.pad;
     for (int f = 0; f < 3; f++) {
+        if (N <= kResidentSingle) {
+            cudaError_t e = resident_component(W, fc, g, tb, f + 1, buf, M * N, (int)M, buf, outs[f], s);
+            if (e != cudaSuccess) return e;
+            continue;
+        }
         cudaError_t e = grid_launch(spline_pass0_room, N * N, 128, s, W, fc, g, tb, f + 1, buf);
         if (e != cudaSuccess) return e;
         e = grid_launch(spline_pass1_inplace, M * N, 128, s, buf, g, tb);

@@ -137,6 +137,8 @@ extern "C" gkm_status gkm_spline_build_noalloc(const double* W, int32_t n, int32
         gkm::spline_line_tables((int)N, periodic, mt.data(), dp.data(), z.data(), &denom);
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    e = gkm::spline_prepare();
+    if (e != cudaSuccess) return GKM_ERR_CUDA;
     line_tables_kernel<<<1, 1, 0, s>>>((int)N, periodic, sym.tables);
     e = cudaGetLastError();
     if (e != cudaSuccess) return GKM_ERR_CUDA;
