@@ -66,11 +66,13 @@ __device__ __forceinline__ bool back_rows(double (&cv)[U], int i0, const SplineT
     if (ok) x = y;
     return ok;
 }
-// the fixed point: row kPivotRows where the line has it before its last row, else unused
+// the fixed point, taken at row kPivotRows; shorter lines (last row N - 2, periodic N - 1) have no row
+// that uses it
 __device__ __forceinline__ void fixed_pivots(int N, const SplineTables& tb, double& d_inf, double& r_inf)
 {
-    d_inf = N > kPivotRows + 4 ? tb.dp[kPivotRows] : 0.0;
-    r_inf = N > kPivotRows + 4 ? tb.mt[kPivotRows + 1] : 0.0;
+    const bool reached = N - 2 >= kPivotRows;
+    d_inf = reached ? tb.dp[kPivotRows] : 0.0;
+    r_inf = reached ? tb.mt[kPivotRows] : 0.0;
 }
 
 template <int U, class Src>

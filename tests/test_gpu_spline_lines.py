@@ -11,7 +11,7 @@ from dns_gkm_lpt_b200.solver import Solver
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N,build", [(4, 2), (10, 1), (24, 2), (25, 1), (26, 2), (27, 1), (34, 2), (200, 2), (201, 2),
+@pytest.mark.parametrize("N,build", [(4, 2), (10, 1), (24, 2), (25, 1), (26, 2), (27, 1), (28, 2), (34, 2), (200, 2), (201, 2),
                                      (264, 1), (265, 1)])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_coefficients_at_the_edges_of_the_line_kernels(oracle, mode, N, build):
