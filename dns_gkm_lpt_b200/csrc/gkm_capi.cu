@@ -392,6 +392,7 @@ gkm_status read_clock(gkm_handle* h, DevClock* c)
     CK(h, cudaMemcpyAsync(c, h->clock, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     if (c->status & 2) return fail(h, GKM_ERR_CUDA, "a bulk tensor copy of a sweep did not complete in time");
+    if (c->status & gkm::kStatusTags) return fail(h, GKM_ERR_STATE, "particle tags corrupted");
     if (c->status & 1) return fail(h, GKM_ERR_NONFINITE, "state holds a non-finite value or non-positive density");
     return GKM_OK;
 }
@@ -404,15 +405,23 @@ gkm_status ensure_splines(gkm_handle* h)
     return GKM_OK;
 }
 
-// upload index of the particle in each device slot (the arrays are kept in spline-cell order)
-gkm_status host_tags(gkm_handle* h, std::vector<long long>& tags)
+// np x 3 values in upload order from particle arrays a[0..2], through the sorted copy s[0..2]
+gkm_status download_triples(gkm_handle* h, double* const a[3], double* const s[3], double* out)
 {
-    tags.resize((size_t)h->np);
-    if (h->np == 0) return GKM_OK;
-    CK(h, cudaMemcpyAsync(tags.data(), h->tag, sizeof(long long) * (size_t)h->np, cudaMemcpyDeviceToHost, h->stream));
-    CK(h, cudaStreamSynchronize(h->stream));
-    for (long long t : tags)
-        if (t < 0 || t >= h->np) return fail(h, GKM_ERR_STATE, "particle tags corrupted");
+    CK(h, gkm::launch_particle_export(h->np, h->tag, a, s, h->clock, h->stream));
+    h->launches += 1;
+    for (int k = 0; k < 3; k++)
+        CK(h, cudaMemcpyAsync(out + (size_t)k * h->np, s[k], sizeof(double) * (size_t)h->np, cudaMemcpyDeviceToHost,
+                              h->stream));
+    return GKM_OK;
+}
+gkm_status upload_triples(gkm_handle* h, int64_t np, const double* in, double* const s[3], double* const a[3],
+                          long long* tag)
+{
+    for (int k = 0; k < 3; k++)
+        CK(h, cudaMemcpyAsync(s[k], in + (size_t)k * np, sizeof(double) * (size_t)np, cudaMemcpyHostToDevice, h->stream));
+    CK(h, gkm::launch_particle_import(np, s, a, tag, h->stream));
+    h->launches += 1;
     return GKM_OK;
 }
 
@@ -445,7 +454,8 @@ gkm_status compute_props(gkm_handle* h)
     if (h->np > 0) {
         const double* c8[8] = {h->prop_coef[0], h->coef[0], h->coef[1], h->coef[2],
                                h->prop_coef[1], h->prop_coef[2], h->prop_coef[3], h->prop_coef[4]};
-        CK(h, gkm::launch_particle_props(c8, h->grid, h->np, h->P[0], h->P[1], h->P[2], h->props, h->stream));
+        CK(h, gkm::launch_particle_props(c8, h->grid, h->np, h->P[0], h->P[1], h->P[2], h->tag, h->props, h->clock,
+                                          h->stream));
         h->launches += 1;
     }
     return GKM_OK;
@@ -458,15 +468,12 @@ gkm_status gkm_host_props(gkm_handle* h, double* out)
 {
     gkm_status s = compute_props(h);
     if (s != GKM_OK || h->np == 0) return s;
-    std::vector<double> tmp((size_t)gkm::kPropCount * (size_t)h->np);
-    CK(h, cudaMemcpyAsync(tmp.data(), h->props, sizeof(double) * tmp.size(), cudaMemcpyDeviceToHost, h->stream));
+    int status = 0;
+    CK(h, cudaMemcpyAsync(&status, &h->clock->status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(h, cudaMemcpyAsync(out, h->props, sizeof(double) * gkm::kPropCount * (size_t)h->np, cudaMemcpyDeviceToHost,
+                          h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
-    std::vector<long long> tags;
-    s = host_tags(h, tags);
-    if (s != GKM_OK) return s;
-    const size_t np = (size_t)h->np;
-    for (size_t p = 0; p < np; p++)
-        for (int q = 0; q < gkm::kPropCount; q++) out[(size_t)tags[p] * gkm::kPropCount + q] = tmp[(size_t)q * np + p];
+    if (status & gkm::kStatusTags) return fail(h, GKM_ERR_STATE, "particle tags corrupted");
     return GKM_OK;
 }
 
@@ -1143,19 +1150,11 @@ gkm_status gkm_particles_upload(gkm_handle* h, int64_t np, const double* pos, co
 {
     if (!h || (np > 0 && !pos)) return GKM_ERR_ARG;
     if (np < 0 || np > h->cap) return fail(h, GKM_ERR_ARG, "particle count exceeds max_particles");
-    std::vector<double> tmp((size_t)np);
-    for (int c = 0; c < 6; c++) {
-        const double* src = c < 3 ? pos : U;
-        if (!src) continue;
-        for (int64_t p = 0; p < np; p++) tmp[(size_t)p] = src[3 * p + (c % 3)];
-        CK(h, cudaMemcpyAsync(h->P[c], tmp.data(), sizeof(double) * (size_t)np, cudaMemcpyHostToDevice, h->stream));
-        CK(h, cudaStreamSynchronize(h->stream));
-    }
     if (np > 0) {   // tags: the upload order, restored by every download
-        std::vector<long long> tags((size_t)np);
-        for (int64_t p = 0; p < np; p++) tags[(size_t)p] = p;
-        CK(h, cudaMemcpyAsync(h->tag, tags.data(), sizeof(long long) * (size_t)np, cudaMemcpyHostToDevice, h->stream));
-        CK(h, cudaStreamSynchronize(h->stream));
+        gkm_status s = upload_triples(h, np, pos, h->P_sorted, h->P, h->tag);
+        if (s == GKM_OK && U) s = upload_triples(h, np, U, h->P_sorted + 3, h->P + 3, nullptr);
+        if (s != GKM_OK) return s;
+        CK(h, cudaStreamSynchronize(h->stream));   // the caller's arrays have been read
     }
     h->np = np;
     if (!U && np > 0) {
@@ -1178,16 +1177,10 @@ gkm_status gkm_particles_upload(gkm_handle* h, int64_t np, const double* pos, co
 gkm_status gkm_particles_download(gkm_handle* h, double* pos, double* U)
 {
     if (!h) return GKM_ERR_ARG;
-    std::vector<double> tmp((size_t)h->np);
-    std::vector<long long> tags;
-    gkm_status s = host_tags(h, tags);
-    if (s != GKM_OK) return s;
-    for (int c = 0; c < 6; c++) {
-        double* dst = c < 3 ? pos : U;
-        if (!dst) continue;
-        CK(h, cudaMemcpyAsync(tmp.data(), h->P[c], sizeof(double) * (size_t)h->np, cudaMemcpyDeviceToHost, h->stream));
-        CK(h, cudaStreamSynchronize(h->stream));
-        for (int64_t p = 0; p < h->np; p++) dst[3 * tags[(size_t)p] + (c % 3)] = tmp[(size_t)p];
+    if (h->np > 0) {
+        gkm_status s = pos ? download_triples(h, h->P, h->P_sorted, pos) : GKM_OK;
+        if (s == GKM_OK && U) s = download_triples(h, h->P + 3, h->P_sorted + 3, U);
+        if (s != GKM_OK) return s;
     }
     DevClock c;
     return read_clock(h, &c);

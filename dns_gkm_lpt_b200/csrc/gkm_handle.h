@@ -53,7 +53,7 @@ struct gkm_handle {
     unsigned* sort_temp = nullptr;
     double* prop_coef[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // rho, p, lap u, lap v, lap w
     double* lap_nodes = nullptr;     // nt^3 Laplacian node values (one velocity component at a time)
-    double* props = nullptr;         // [kPropCount][cap] particle properties
+    double* props = nullptr;         // [cap][kPropCount] particle properties, in upload order
     gkm::StatsPartial* partials = nullptr;
     double* stats_out = nullptr;
     cudaGraphExec_t graph[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};

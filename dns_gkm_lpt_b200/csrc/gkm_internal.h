@@ -17,9 +17,11 @@ struct DevClock {
                                  // timestep(W); t += dt)
     long long iter;              // completed steps
     unsigned long long wave[2];  // max(|u|+c) of the current/next state, as double bits
-    int status;                  // bit 0: non-finite state detected
+    int status;                  // bit 0: non-finite state; bit 1: a bulk copy timed out; bit 2: particle tags corrupted
     int pad;
 };
+
+constexpr int kStatusTags = 4;
 
 // Physical and grid constants of one field (reference globals of src/param.h:11-27).
 struct FieldConst {
@@ -203,7 +205,14 @@ cudaError_t launch_spline_source(const double* src, const FieldConst& fc, const 
                                  int kind, double* coef, double* scratch, cudaStream_t s);
 cudaError_t launch_lap_nodes(const double* coef, const SplineGrid& g, const FieldConst& fc, double* out, cudaStream_t s);
 cudaError_t launch_particle_props(const double* const coefs[8], const SplineGrid& g, long long np, const double* py,
-                                  const double* px, const double* pz, double* props, cudaStream_t s);
+                                  const double* px, const double* pz, const long long* tag, double* props,
+                                  DevClock* clock, cudaStream_t s);
+// np x 3 host values through three device arrays of np (value e of them in array e / np): the particle
+// arrays' triples in upload order, and back with fresh tags (tag may be null)
+cudaError_t launch_particle_export(long long np, const long long* tag, double* const src[3], double* const dst[3],
+                                   DevClock* clock, cudaStream_t s);
+cudaError_t launch_particle_import(long long np, double* const src[3], double* const dst[3], long long* tag,
+                                   cudaStream_t s);
 cudaError_t launch_particle_stats(const double* props, long long np, StatsPartial* partials, int nblocks, double* out6,
                                   cudaStream_t s);
 cudaError_t launch_stats(const double* W, const FieldConst& fc, const SplineGrid& g, const double* const coefs[3],
