@@ -91,17 +91,21 @@ __device__ __forceinline__ double collision_time(const FieldConst& fc, double T,
     return fc.mu0 * (x * sqrt(x)) * (fc.T0 + 110.4) / ((T + 110.4) * p);
 }
 
-// |u| + c of a conserved state in FP64: with one reciprocal of rho (the z sweeps' reduction
-// for the next step's dt, within an ulp or two of the reference's), and with the reference's
-// divisions (src/update.cpp:1039-1046 via c2p; the stand-alone timestep, whose dt equals the
-// reference's bit for bit).
-__device__ __forceinline__ double wave_speed_recip(const double w[5], double gam, double gm1)
+// |u| + c of a conserved state in FP64: its square |u|^2 + c^2 + 2 |u| c with one reciprocal of rho and
+// one inverse root (the z sweeps' reduction for the next step's dt, whose square root is taken
+// once per thread: within an ulp or two of the reference's; NaN where p < 0), and with the
+// reference's divisions and roots (src/update.cpp:1039-1046 via c2p; the stand-alone timestep,
+// whose dt equals the reference's bit for bit).
+__device__ __forceinline__ double wave_speed_sq(const double w[5], double gam, double gm1)
 {
-    const double d = w[0], id = 1.0 / d;
+    const double id = recip<double>(w[0]);
     const double u = w[1] * id, v = w[2] * id, x = w[3] * id;
     const double vs = u * u + v * v + x * x;
-    const double p = (d * gm1) * (w[4] * id - 0.5 * vs);
-    return sqrt(vs) + sqrt(gam * p * id);
+    const double cs = (gam * gm1) * (w[4] * id - 0.5 * vs);
+    const double q = vs * cs;
+    // below 1e-280 the product's root adds nothing to c^2 (and its inverse root is not defined at 0)
+    const double root = q > 1e-280 ? q * rsqrt_t<double>(q) : (cs >= 0.0 ? 0.0 : nan(""));
+    return vs + cs + 2.0 * root;
 }
 
 __device__ __forceinline__ double wave_speed(const double w[5], double gam, double gm1)
@@ -750,11 +754,22 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                 }
             }
             // the window's cells beyond one per thread: one WENO scalar per work item (5 per cell,
-            // T into the energy slots), then their face energies
+            // T into the energy slots), then their face energies, one side per item.  The two corners
+            // of the last row, which no face's slopes read, are left out where that saves a round of
+            // items (16 x 8: 50 cells make two rounds, 52 three; there the sweeps' 2.57 / 2.63 / 3.17 ms
+            // at 256^3 became 2.50 / 2.56 / 3.07)
             if constexpr (kSplit) {
-                constexpr int kRest = kWC - kSweepThreads;
+                constexpr int kAll = kWC - kSweepThreads, kLastRow = kWC - kWB;
+                constexpr bool kSkip = kSweepThreads <= kLastRow &&
+                                       (5 * (kAll - 2) + kSweepThreads - 1) / kSweepThreads <
+                                           (5 * kAll + kSweepThreads - 1) / kSweepThreads;
+                constexpr int kRest = kSkip ? kAll - 2 : kAll;
+                auto rest_cell = [](int r) {
+                    const int c = kSweepThreads + r;
+                    return kSkip && c >= kLastRow ? c + 1 : c;
+                };
                 for (int it = tid; it < 5 * kRest; it += kSweepThreads) {
-                    const int q = it / kRest, c = kSweepThreads + (it - q * kRest);
+                    const int q = it / kRest, c = rest_cell(it - q * kRest);
                     const int aa = c / kWB, bb = c - aa * kWB;
                     if (a0 + aa - 1 > n || b0 + bb - 1 > n) continue;
                     const int o = (q < 4 ? q : 5) * kWC + c;
@@ -765,13 +780,12 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                     rec[(5 + q) * kWC + c] = fr;
                 }
                 __syncthreads();
-                for (int c = kSweepThreads + tid; c < kWC; c += kSweepThreads) {
+                for (int it = tid; it < 2 * kRest; it += kSweepThreads) {
+                    const int sd = it / kRest, c = rest_cell(it - sd * kRest);
                     const int aa = c / kWB, bb = c - aa * kWB;
                     if (a0 + aa - 1 > n || b0 + bb - 1 > n) continue;
-                    T* lc = rec + c;
-                    T* rc = rec + 5 * kWC + c;
-                    lc[4 * kWC] = face_energy<T>(lc[0], lc[kWC], lc[2 * kWC], lc[3 * kWC], lc[4 * kWC], ph);
-                    rc[4 * kWC] = face_energy<T>(rc[0], rc[kWC], rc[2 * kWC], rc[3 * kWC], rc[4 * kWC], ph);
+                    T* x = rec + 5 * sd * kWC + c;
+                    x[4 * kWC] = face_energy<T>(x[0], x[kWC], x[2 * kWC], x[3 * kWC], x[4 * kWC], ph);
                 }
             }
         }
@@ -883,7 +897,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
                         else a.A[q * nt3 + ci] = wn[q];
                     }
                     if (zp && !first_of_pair(f)) fence_async_shared();   // the brick's copy out reads it
-                    const double ws = wave_speed_recip(wn, fc.gam, fc.gm1);
+                    const double ws = wave_speed_sq(wn, fc.gam, fc.gm1);
                     if (!isfinite(ws) || !(wn[0] > 0.0)) bad = true;
                     else wmax = ws > wmax ? ws : wmax;
                 }
@@ -906,7 +920,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
         }
     }
     if (DIR == 2) {
-        double m = block_max(wmax, reinterpret_cast<double*>(rec));
+        double m = block_max(sqrt(wmax), reinterpret_cast<double*>(rec));
         if (tid == 0 && m > 0.0) atomicMax(&a.clock->wave[a.parity ^ 1], (unsigned long long)__double_as_longlong(m));
         if (bad) atomicOr(&a.clock->status, 1);
     }

@@ -337,7 +337,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                             wn[q] = __dsub_rn((double)wl[q * kWC + cc], __dmul_rn(fc.inv_dx, s));
                             a.A[q * nt3 + ci] = wn[q];
                         }
-                        const double ws = wave_speed_recip(wn, fc.gam, fc.gm1);
+                        const double ws = wave_speed_sq(wn, fc.gam, fc.gm1);
                         if (!isfinite(ws) || !(wn[0] > 0.0)) bad = true;
                         else wmax = ws > wmax ? ws : wmax;
                     }
@@ -348,7 +348,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
             mbar_arrive(bar_empty0 + 8 * (k & 1));
         }
         if (DIR == 2) {   // max |u| + c over the consumers: warp shuffles, then the warp maxima in order
-            double v = wmax;
+            double v = sqrt(wmax);
             for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
             double* red = stage;   // every consumer has read its staged accumulator
             consumer_sync();
