@@ -124,11 +124,10 @@ const void* sweep_tmap_wb(const gkm_handle* h, const double* W, int dir, int var
 // boxes (WB, 1, WA, 5) for the x sweep's slabs (window j x k at one i), (WB, WA, 1, 5) for the y
 // sweep's (window i x k at one j), (2, TB, TA, 5) for the z sweep's accumulator bricks (two k-cells
 // of the window i x j) and (2, WB, WA, 5) for its slabs (two k-planes of the window and its halo).
-// The row strides must be multiples of 16 bytes, so nt must be even; otherwise (or without the
-// driver entry point) the sweeps move every value with cp.async and plain loads and stores.
+// The row strides must be multiples of 16 bytes, which the even pitch gives.  Without the driver
+// entry point the sweeps move every value with cp.async and plain loads and stores.
 cudaError_t setup_tensor_maps(gkm_handle* h)
 {
-    if (h->fc.nt % 2) return cudaSuccess;
     const bool mixed = h->cfg.precision == GKM_PREC_MIXED;
     using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -143,7 +142,7 @@ cudaError_t setup_tensor_maps(gkm_handle* h)
     const Encode encode = reinterpret_cast<Encode>(fn);
     const cuuint64_t nt = (cuuint64_t)h->fc.nt;
     const cuuint64_t dims[4] = {nt, nt, nt, 5};
-    const cuuint64_t strides[3] = {nt * 8, nt * nt * 8, nt * nt * nt * 8};
+    const cuuint64_t pitch = (cuuint64_t)h->fc.pitch, strides[3] = {pitch * 8, nt * pitch * 8, nt * nt * pitch * 8};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const int nmaps = 2 * gkm::kSweepVariants64 * 4;
     std::vector<CUtensorMap> maps((size_t)nmaps);
@@ -437,7 +436,7 @@ gkm_status compute_props(gkm_handle* h)
     const long long M = h->grid.npts + h->grid.pad;
     for (int c = 0; c < 5; c++)
         if (!h->prop_coef[c]) CK(h, cudaMalloc(&h->prop_coef[c], sizeof(double) * (size_t)(M * M * M)));
-    if (!h->lap_nodes) CK(h, cudaMalloc(&h->lap_nodes, sizeof(double) * (size_t)h->fc.nt3));
+    if (!h->lap_nodes) CK(h, cudaMalloc(&h->lap_nodes, sizeof(double) * (size_t)h->fc.comp));
     if (!h->props && h->cap > 0) CK(h, cudaMalloc(&h->props, sizeof(double) * gkm::kPropCount * (size_t)h->cap));
     const gkm::SplineTables tb = device_tables(h);
     const double* W = h->buf[h->parity];
@@ -462,6 +461,17 @@ gkm_status compute_props(gkm_handle* h)
 }
 
 }  // namespace
+
+gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
+{
+    *dense = h->buf[h->parity];
+    if (h->fc.pitch == h->fc.nt) return GKM_OK;
+    double* out = h->buf[h->parity ^ 1];
+    CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->stream));
+    h->launches += 1;
+    *dense = out;
+    return GKM_OK;
+}
 
 // host copy of the property table, particle-major (np x kPropCount); used by the writers too
 gkm_status gkm_host_props(gkm_handle* h, double* out)
@@ -521,6 +531,8 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     fc.n = P.n;
     fc.nt = P.n + 6;
     fc.nt3 = (long long)fc.nt * fc.nt * fc.nt;
+    fc.pitch = fc.nt + fc.nt % 2;
+    fc.comp = (long long)fc.nt * fc.nt * fc.pitch;
     fc.K = K;
     fc.visc = cfg->visc_law;
     fc.gam = P.gam;
@@ -567,7 +579,7 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     if (e != cudaSuccess) return bail(e, "cudaStreamCreate");
     h->stream = h->own_stream;
     for (int b = 0; b < 2; b++) {
-        e = cudaMalloc(&h->buf[b], sizeof(double) * 5 * (size_t)fc.nt3);
+        e = cudaMalloc(&h->buf[b], sizeof(double) * 5 * (size_t)fc.comp);
         if (e != cudaSuccess) return bail(e, "cudaMalloc(state)");
     }
     e = cudaMalloc(&h->clock, sizeof(DevClock));
@@ -673,6 +685,7 @@ gkm_status gkm_destroy(gkm_handle* h)
     for (int c = 0; c < 5; c++) cudaFree(h->prop_coef[c]);
     cudaFree(h->lap_nodes);
     cudaFree(h->props);
+    cudaFree(h->pipe_dense);
     for (cudaEvent_t e : h->pipe_ev) cudaEventDestroy(e);
     for (cudaStream_t s : {h->pipe_in, h->pipe_out, h->pipe_comp[0], h->pipe_comp[1], h->pipe_comp[2], h->pipe_comp[3],
                            h->pipe_halo})
@@ -691,8 +704,14 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
         if (!W[q]) return fail(h, GKM_ERR_ARG, "W[q] is NULL");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
     double* dst = h->buf[h->parity];
+    // odd grids: dense rows through the accumulator buffer, free between steps, then to their pitch
+    double* land = h->fc.pitch == h->fc.nt ? dst : h->buf[h->parity ^ 1];
     for (int q = 0; q < 5; q++)
-        CK(h, cudaMemcpyAsync(dst + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
+        CK(h, cudaMemcpyAsync(land + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
+    if (land != dst) {
+        CK(h, gkm::launch_rows_expand(land, dst, h->fc, h->stream));
+        h->launches += 1;
+    }
     h->launches += 1;
     CK(h, gkm::launch_halo(dst, h->fc, h->clock, 0, h->parity, 0, 0.0, h->stream));
     CK(h, cudaMemsetAsync(&h->clock->status, 0, sizeof(int), h->stream));
@@ -708,7 +727,9 @@ gkm_status gkm_download_state(gkm_handle* h, double* const W[5])
     if (!h || !W) return GKM_ERR_ARG;
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
-    const double* src = h->buf[h->parity];
+    const double* src = nullptr;
+    gkm_status s = gkm_host::dense_state(h, &src);
+    if (s != GKM_OK) return s;
     for (int q = 0; q < 5; q++) {
         if (!W[q]) return fail(h, GKM_ERR_ARG, "W[q] is NULL");
         CK(h, cudaMemcpyAsync(W[q], src + (size_t)q * h->fc.nt3, bytes, cudaMemcpyDefault, h->stream));
@@ -995,10 +1016,16 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
                            h->pipe_halo})
         CK(h, cudaStreamWaitEvent(s, ev_start, 0));
 
+    // odd grids: the copies go to and from dense planes, which the halo launches read and write (a 2-D
+    // copy between dense and pitched rows takes the bus four times as long).  Chunk c's result overwrites
+    // planes whose input was spread before chunk c's sweeps began.
+    double* const dense = fc.pitch == fc.nt ? nullptr : h->pipe_dense;
+    double* const in = dense ? dense : Wd;
+    const double* const out = dense ? dense : A;
     auto copy_in = [&](int J0, int J1) -> cudaError_t {
         for (int q = 0; q < 5; q++) {
             const size_t off = (size_t)q * nt3 + (size_t)J0 * plane;
-            cudaError_t e = cudaMemcpyAsync(Wd + off, W[q] + (size_t)J0 * plane, sizeof(double) * (J1 - J0) * plane,
+            cudaError_t e = cudaMemcpyAsync(in + off, W[q] + (size_t)J0 * plane, sizeof(double) * (J1 - J0) * plane,
                                             cudaMemcpyDefault, h->pipe_in);
             if (e != cudaSuccess) return e;
         }
@@ -1007,7 +1034,7 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
     auto copy_out = [&](int J0, int J1, cudaStream_t s) -> cudaError_t {
         for (int q = 0; q < 5; q++) {
             const size_t off = (size_t)q * nt3 + (size_t)J0 * plane;
-            cudaError_t e = cudaMemcpyAsync(W[q] + (size_t)J0 * plane, A + off, sizeof(double) * (J1 - J0) * plane,
+            cudaError_t e = cudaMemcpyAsync(W[q] + (size_t)J0 * plane, out + off, sizeof(double) * (J1 - J0) * plane,
                                             cudaMemcpyDefault, s);
             if (e != cudaSuccess) return e;
         }
@@ -1033,12 +1060,12 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
         const int P0 = c == 0 ? 3 : part_end(c - 1), P1 = part_end(c);
         CK(h, cudaStreamWaitEvent(h->pipe_halo, ev_cp[c], 0));
         if (c == 0) {   // the y-ghost planes: images of planes n..n+2 (copied first) and of planes 3..5
-            CK(h, gkm::launch_halo_planes(Wd, fc, 0, 3, h->pipe_halo));
-            CK(h, gkm::launch_halo_planes(Wd, fc, n + 3, n + 6, h->pipe_halo));
+            CK(h, gkm::launch_halo_planes(Wd, fc, 0, 3, dense, nullptr, h->pipe_halo));
+            CK(h, gkm::launch_halo_planes(Wd, fc, n + 3, n + 6, dense, nullptr, h->pipe_halo));
             h->launches += 2;
         }
         if (P1 > P0) {
-            CK(h, gkm::launch_halo_planes(Wd, fc, P0, P1, h->pipe_halo));
+            CK(h, gkm::launch_halo_planes(Wd, fc, P0, P1, dense, nullptr, h->pipe_halo));
             h->launches += 1;
         }
         CK(h, cudaEventRecord(ev_in[c], h->pipe_halo));
@@ -1070,7 +1097,7 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
             ad.tmap_wb = sweep_tmap_wb(h, ad.W, d, v);
             CK(h, mixed ? gkm::launch_sweep_mixed_rows(d, v, ad, j0, j1, s) : gkm::launch_sweep_rows(d, v, ad, j0, j1, s));
         }
-        CK(h, gkm::launch_halo_planes(A, fc, 3 + j0, 3 + j1, s));
+        CK(h, gkm::launch_halo_planes(A, fc, 3 + j0, 3 + j1, nullptr, dense, s));
         h->launches += 4;
         CK(h, cudaEventRecord(ev_out[c], s));
         CK(h, cudaStreamWaitEvent(h->pipe_out, ev_out[c], 0));
@@ -1080,8 +1107,8 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
 
     // the y-ghost planes of the new state, the clock, the last copies
     for (int c = 0; c < K; c++) CK(h, cudaStreamWaitEvent(h->stream, ev_out[c], 0));
-    CK(h, gkm::launch_halo_planes(A, fc, 0, 3, h->stream));
-    CK(h, gkm::launch_halo_planes(A, fc, n + 3, n + 6, h->stream));
+    CK(h, gkm::launch_halo_planes(A, fc, 0, 3, nullptr, dense, h->stream));
+    CK(h, gkm::launch_halo_planes(A, fc, n + 3, n + 6, nullptr, dense, h->stream));
     CK(h, gkm::launch_clock_finish(ck, dt, h->stream));
     h->launches += 3;
     CK(h, copy_out(0, 3, h->stream));
@@ -1112,6 +1139,12 @@ gkm_status gkm_evolve(gkm_handle* h, double* const W[5], double dt)
     if (!(dt > 0.0)) return fail(h, GKM_ERR_ARG, "dt must be > 0");
     bool pipelined = true;
     for (int q = 0; q < 5; q++) pipelined = pipelined && W[q] && async_capable(W[q]);
+    if (pipelined && h->fc.pitch != h->fc.nt && !h->pipe_dense &&
+        cudaMalloc(&h->pipe_dense, sizeof(double) * 5 * (size_t)h->fc.nt3) != cudaSuccess) {
+        cudaGetLastError();   // no room for the dense planes: the one-shot path needs none
+        h->pipe_dense = nullptr;
+        pipelined = false;
+    }
     if (pipelined) return evolve_pipelined(h, W, dt);
     gkm_status s = gkm_upload_state(h, (const double* const*)W);
     if (s != GKM_OK) return s;

@@ -63,6 +63,7 @@ struct gkm_handle {
     // plug-point pipeline (gkm_evolve with pinned or device buffers): copy-in, copy-out and
     // two compute streams, and per-chunk events, created on first use
     cudaStream_t pipe_in = nullptr, pipe_out = nullptr, pipe_comp[4] = {nullptr, nullptr, nullptr, nullptr};
+    double* pipe_dense = nullptr;       // odd grids: the pipeline's dense planes, 5 x nt^3 (on first use)
     cudaStream_t pipe_halo = nullptr;   // ghost wrap of each part as it lands, off the copy-in stream
     std::vector<cudaEvent_t> pipe_ev;
     int pipe_chunk = 0;      // y-planes per chunk (multiple of 16); 0: about n/8
@@ -96,5 +97,9 @@ inline gkm_status cuda_fail(gkm_handle* h, cudaError_t e, const char* where)
         cudaError_t e_ = (expr);                            \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, #expr); \
     } while (0)
+
+// the current state as dense rows (5 components of nt^3, device memory): the state itself, or on odd
+// grids a copy in the accumulator buffer, which is free between steps
+gkm_status dense_state(gkm_handle* h, const double** dense);
 
 }  // namespace gkm_host

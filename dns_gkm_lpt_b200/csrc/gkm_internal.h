@@ -28,6 +28,12 @@ struct FieldConst {
     int n;          // interior cells per side
     int nt;         // n + 6
     long long nt3;  // nt^3
+    // The state arrays on the device: cell (j, i, k) of component q at q comp + (j nt + i) pitch + k.  The
+    // pitch is nt rounded up to even: bulk tensor copies want row strides of 16 bytes, and without them the
+    // z sweep of odd grids gathered 8 bytes of a line per cell and plane (255^3 z: 5.89 -> 2.96 ms FP64,
+    // 6.40 -> 1.95 mixed).  Host arrays are dense (the reference's layout).
+    int pitch;
+    long long comp;   // nt^2 pitch
     int K;
     int visc;       // 0 Sutherland, 1 power law 0.76
     double gam, gm1, dx, inv_dx, mu0, T0, cfl;
@@ -87,7 +93,7 @@ constexpr int kRing = 6;            // slabs held: the 6-cell WENO stencil
 constexpr int kSlabComps = 6;       // rho, rho u, rho v, rho w, rho E, T
 
 struct SweepArgs {
-    const double* __restrict__ W;   // current state, 5 components of nt^3 (reference layout)
+    const double* __restrict__ W;   // current state, 5 components (FieldConst: pitch, comp)
     double* __restrict__ A;         // accumulator; the z sweep overwrites it with the new state
     FieldConst fc;
     DevClock* clock;
@@ -115,8 +121,14 @@ cudaError_t launch_sweep(int dir, int variant, const SweepArgs& a, int nseg, cud
 // The cells updated are exactly those of planes [j0, j1).
 cudaError_t launch_sweep_rows(int dir, int variant, SweepArgs a, int j0, int j1, cudaStream_t s);
 cudaError_t launch_sweep_mixed_rows(int dir, int variant, SweepArgs a, int j0, int j1, cudaStream_t s);
-// Ghost cells of the ghost-layout y-planes [J0, J1) (0 <= J0 < J1 <= nt) from their periodic images
-cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, cudaStream_t s);
+// The state between the device's pitched rows and dense rows (dense: 5 components of nt^3 in device memory)
+cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, cudaStream_t s);
+cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, cudaStream_t s);
+// Ghost cells of the ghost-layout y-planes [J0, J1) (0 <= J0 < J1 <= nt) from their periodic images;
+// odd grids' plug point: with `from` every cell of those planes from the dense state, with `to` the planes
+// written to it as well
+cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, const double* from, double* to,
+                               cudaStream_t s);
 // the clock update that closes a step with a given dt: t += dt, iter += 1
 cudaError_t launch_clock_finish(DevClock* clock, double dt, cudaStream_t s);
 // the same sweeps with the reconstruction and the flux in single precision (sweep_mixed.cu)

@@ -290,15 +290,15 @@ __device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTab
 // (rho (gam-1)) (rho E / rho - |u|^2 / 2); q = kSrcPlain the array itself (one nt^3 component).
 constexpr int kSrcDensity = 0, kSrcPressure = 4, kSrcPlain = 5;
 
-__device__ __forceinline__ double spline_source(const double* __restrict__ W, long long nt3, double gm1, int q,
+__device__ __forceinline__ double spline_source(const double* __restrict__ W, long long comp, double gm1, int q,
                                                 long long idx)
 {
     if (q == kSrcDensity || q == kSrcPlain) return W[idx];
     const double d = W[idx];
-    if (q != kSrcPressure) return __ddiv_rn(W[q * nt3 + idx], d);
-    const double u = __ddiv_rn(W[nt3 + idx], d), v = __ddiv_rn(W[2 * nt3 + idx], d), w = __ddiv_rn(W[3 * nt3 + idx], d);
+    if (q != kSrcPressure) return __ddiv_rn(W[q * comp + idx], d);
+    const double u = __ddiv_rn(W[comp + idx], d), v = __ddiv_rn(W[2 * comp + idx], d), w = __ddiv_rn(W[3 * comp + idx], d);
     const double vs = add(add(mul(u, u), mul(v, v)), mul(w, w));
-    return mul(mul(d, gm1), sub(__ddiv_rn(W[4 * nt3 + idx], d), mul(0.5, vs)));
+    return mul(mul(d, gm1), sub(__ddiv_rn(W[4 * comp + idx], d), mul(0.5, vs)));
 }
 
 // pass 0: the data of source q along axis 0 (y) -> out [M0][N1][N2]; one line (i, k).  VEL: q is a
@@ -310,16 +310,15 @@ __device__ __forceinline__ void pass0_line(const double* __restrict__ W, const F
 {
     const int N = g.npts;
     const long long lines = stride ? stride : (long long)N * N;   // output stride along axis 0
-    const long long nt3 = fc.nt3;
-    const int nt = fc.nt;
+    const long long comp = fc.comp;
     const int off = g.periodic ? 3 : 0;
     const int i = (int)(L / N), k = (int)(L - (long long)i * N);
-    const long long base = (long long)(i + off) * nt + (k + off);
-    const long long sj = (long long)nt * nt;
+    const long long base = (long long)(i + off) * fc.pitch + (k + off);
+    const long long sj = (long long)fc.nt * fc.pitch;
     auto f = [&](int j) {
         const long long idx = (long long)(j + off) * sj + base;
-        if constexpr (VEL) return __ddiv_rn(W[q * nt3 + idx], W[idx]);
-        else return spline_source(W, nt3, fc.gm1, q, idx);
+        if constexpr (VEL) return __ddiv_rn(W[q * comp + idx], W[idx]);
+        else return spline_source(W, comp, fc.gm1, q, idx);
     };
     line_solve<U>(f, N, g.periodic, tb, out + L, lines);
 }
@@ -835,14 +834,15 @@ __device__ __forceinline__ void resident_pass0(const double* __restrict__ W, con
     const LineTables T = line_tables(tb, N, g.periodic, smem);
     const bool mine = group * 32 + lane < (long long)N * N;
     const long long L = mine ? group * 32 + lane : (long long)N * N - 1;   // a lane beyond the lines repeats the last
-    const int off = g.periodic ? 3 : 0, nt = fc.nt;
+    const int off = g.periodic ? 3 : 0;
     const int i = (int)(L / N), k = (int)(L - (long long)i * N);
-    const long long sj = (long long)nt * nt, base = off * sj + (long long)(i + off) * nt + (k + off), nt3 = fc.nt3;
+    const long long sj = (long long)fc.nt * fc.pitch, base = off * sj + (long long)(i + off) * fc.pitch + (k + off),
+                    comp = fc.comp;
     double* s = smem + 2 * kTableRows + lane;
     if constexpr (VEL) {   // the next rows' loads are issued before this batch's divisions
         constexpr int U = 8;
         const double* pd = W + base;
-        const double* pm = pd + q * nt3;
+        const double* pm = pd + q * comp;
         double d[U], m[U], dn[U], mn[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -866,7 +866,7 @@ __device__ __forceinline__ void resident_pass0(const double* __restrict__ W, con
         }
     } else {
 #pragma unroll 4
-        for (int j = 0; j < N; j++) s[j * 32] = spline_source(W, nt3, fc.gm1, q, base + j * sj);
+        for (int j = 0; j < N; j++) s[j * 32] = spline_source(W, comp, fc.gm1, q, base + j * sj);
     }
     copy_async_wait();
     __syncwarp();
@@ -1139,7 +1139,7 @@ __global__ void lap_nodes_kernel(const double* __restrict__ C, SplineGrid g, Fie
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(e / ((long long)N * N)), i = (int)((e / N) % N), k = (int)(e % N);
         const int J = j + off, I = i + off, K = k + off;
-        const long long o = ((long long)J * nt + I) * nt + K;
+        const long long o = ((long long)J * nt + I) * fc.pitch + K;
         if (J < 3 || J >= nt - 3 || I < 3 || I >= nt - 3 || K < 3 || K >= nt - 3) {
             out[o] = 0.0;
             continue;
@@ -1462,15 +1462,15 @@ __device__ __forceinline__ double visc(const FieldConst& fc, double T)
     return fc.mu0 * pow(x, 1.5) * (fc.T0 + 110.4) / (T + 110.4);
 }
 
-__device__ __forceinline__ void cell_c2p(const double* W, long long nt3, long long idx, double gm1, double& d, double& u,
+__device__ __forceinline__ void cell_c2p(const double* W, long long comp, long long idx, double gm1, double& d, double& u,
                                          double& v, double& w, double& P, double& T)
 {
     d = W[idx];
-    u = W[nt3 + idx] / d;
-    v = W[2 * nt3 + idx] / d;
-    w = W[3 * nt3 + idx] / d;
+    u = W[comp + idx] / d;
+    v = W[2 * comp + idx] / d;
+    w = W[3 * comp + idx] / d;
     const double vs = u * u + v * v + w * w;
-    P = (d * gm1) * (W[4 * nt3 + idx] / d - 0.5 * vs);
+    P = (d * gm1) * (W[4 * comp + idx] / d - 0.5 * vs);
     T = P / (287.0 * d);
 }
 
@@ -1480,7 +1480,7 @@ __global__ void stats_kernel(const double* __restrict__ W, FieldConst fc, Spline
 {
     __shared__ double red[16][32];
     const int n = fc.n, nt = fc.nt;
-    const long long nt3 = fc.nt3, total = (long long)n * n * n;
+    const long long comp = fc.comp, total = (long long)n * n * n;
     const long long M = g.npts + g.pad;
     const int off = g.periodic ? 0 : 3;   // coefficient window start of interior cell m
     double acc[16];
@@ -1488,9 +1488,9 @@ __global__ void stats_kernel(const double* __restrict__ W, FieldConst fc, Spline
     for (int s = 0; s < 16; s++) acc[s] = 0.0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(e / ((long long)n * n)), i = (int)((e / n) % n), k = (int)(e % n);
-        const long long idx = ((long long)(j + 3) * nt + (i + 3)) * nt + (k + 3);
+        const long long idx = ((long long)(j + 3) * nt + (i + 3)) * fc.pitch + (k + 3);
         double d, u, v, w, P, T;
-        cell_c2p(W, nt3, idx, fc.gm1, d, u, v, w, P, T);
+        cell_c2p(W, comp, idx, fc.gm1, d, u, v, w, P, T);
         if (PASS == 0) {
             double gu[3], gv[3], gw[3];
             node_grad<CT>(cf.c[0], M, j + off, i + off, k + off, g.dinv, gu);

@@ -146,7 +146,8 @@ extern "C" gkm_status gkm_spline_build_noalloc(const double* W, int32_t n, int32
     gkm::FieldConst fc{};
     fc.n = n;
     fc.nt = (int)nt;
-    fc.nt3 = nt * nt * nt;
+    fc.nt3 = fc.comp = nt * nt * nt;   // the caller's dense array
+    fc.pitch = (int)nt;
     gkm::SplineGrid g{};
     g.npts = (int)N;
     g.pad = periodic ? 3 : 2;

@@ -30,7 +30,9 @@ gkm_status download_state(gkm_handle* h, std::vector<double>& W)
 {
     const size_t nt3 = (size_t)h->fc.nt3;
     W.resize(5 * nt3);
-    const double* src = h->buf[h->parity];
+    const double* src = nullptr;
+    gkm_status s = gkm_host::dense_state(h, &src);
+    if (s != GKM_OK) return s;
     CK(h, cudaMemcpyAsync(W.data(), src, sizeof(double) * 5 * nt3, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
     return GKM_OK;

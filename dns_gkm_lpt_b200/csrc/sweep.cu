@@ -38,11 +38,14 @@ __global__ void halo_kernel(double* __restrict__ W, FieldConst fc, DevClock* clo
 }
 
 // ghost cells of the y-planes [J0, J1): every cell with a coordinate outside the interior takes the
-// value of its periodic image, which is interior in all three coordinates
-__global__ void halo_planes_kernel(double* __restrict__ W, FieldConst fc, int J0, int J1)
+// value of its periodic image, which is interior in all three coordinates.  FROM: all cells, from the
+// dense state; TO: the planes into the dense state too (odd grids, whose rows have a pitch here)
+template <bool FROM, bool TO>
+__global__ void halo_planes_kernel(double* W, FieldConst fc, int J0, int J1, const double* __restrict__ from,
+                                   double* __restrict__ to)
 {
     const int n = fc.n, nt = fc.nt;
-    const long long nt2 = (long long)nt * nt, nt3 = fc.nt3;
+    const long long nt2 = (long long)nt * nt, comp = fc.comp;
     const long long total = (long long)(J1 - J0) * nt2;
     auto wrap = [n](int x) { return x < 3 ? x + n : (x >= n + 3 ? x - n : x); };
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
@@ -51,11 +54,31 @@ __global__ void halo_planes_kernel(double* __restrict__ W, FieldConst fc, int J0
         const long long rem = e - (long long)(j - J0) * nt2;
         const int i = (int)(rem / nt), k = (int)(rem - (long long)i * nt);
         const int wj = wrap(j), wi = wrap(i), wk = wrap(k);
-        if (wj == j && wi == i && wk == k) continue;   // interior cell
-        const long long dst = ((long long)j * nt + i) * nt + k;
-        const long long src = ((long long)wj * nt + wi) * nt + wk;
+        const bool ghost = wj != j || wi != i || wk != k;
+        if (!FROM && !TO && !ghost) continue;
+        const long long dst = ((long long)j * nt + i) * fc.pitch + k;
+        const long long src = ((long long)wj * nt + wi) * (FROM ? nt : fc.pitch) + wk;
+        double v[5];
 #pragma unroll
-        for (int q = 0; q < 5; q++) W[q * nt3 + dst] = W[q * nt3 + src];
+        for (int q = 0; q < 5; q++) v[q] = FROM ? from[q * fc.nt3 + src] : W[q * comp + src];
+#pragma unroll
+        for (int q = 0; q < 5; q++) {
+            if (FROM || ghost) W[q * comp + dst] = v[q];
+            if (TO) to[q * fc.nt3 + ((long long)j * nt + i) * nt + k] = v[q];
+        }
+    }
+}
+
+// rows of odd grids between the pitched layout and dense staging: a warp per row, bound by memory
+template <bool EXPAND>
+__global__ void rows_kernel(const double* __restrict__ src, double* __restrict__ dst, long long rows, int nt, int pitch)
+{
+    const int lane = threadIdx.x & 31;
+    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows;
+         r += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const double* s = src + r * (EXPAND ? nt : pitch);
+        double* d = dst + r * (EXPAND ? pitch : nt);
+        for (int k = lane; k < nt; k += 32) d[k] = s[k];
     }
 }
 
@@ -69,16 +92,16 @@ __global__ void wave_reduce_kernel(const double* __restrict__ W, FieldConst fc, 
 {
     __shared__ double red[32];
     const int n = fc.n, nt = fc.nt;
-    const long long nt3 = fc.nt3, total = (long long)n * n * n;
+    const long long comp = fc.comp, total = (long long)n * n * n;
     double m = 0.0;
     bool bad = false;
     for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
          g += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(g / ((long long)n * n)), i = (int)((g / n) % n), k = (int)(g % n);
-        const long long idx = ((long long)(j + 3) * nt + (i + 3)) * nt + (k + 3);
+        const long long idx = ((long long)(j + 3) * nt + (i + 3)) * fc.pitch + (k + 3);
         double w[5];
 #pragma unroll
-        for (int q = 0; q < 5; q++) w[q] = W[q * nt3 + idx];
+        for (int q = 0; q < 5; q++) w[q] = W[q * comp + idx];
         double ws = wave_speed(w, fc.gam, fc.gm1);
         if (!isfinite(ws) || !(w[0] > 0.0)) bad = true;
         else m = ws > m ? ws : m;
@@ -310,14 +333,35 @@ cudaError_t launch_sweep_rows(int dir, int variant, SweepArgs a, int j0, int j1,
     return launch_sweep_rows_t<double, SweepTile64a>(dir, a, j0, j1, s);
 }
 
-cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, cudaStream_t s)
+cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, const double* from, double* to,
+                               cudaStream_t s)
 {
     if (J0 < 0 || J1 > fc.nt || J0 >= J1) return cudaErrorInvalidValue;
     const long long total = (long long)(J1 - J0) * fc.nt * fc.nt;
     long long blocks = (total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    halo_planes_kernel<<<(unsigned)blocks, 256, 0, s>>>(W, fc, J0, J1);
+    if (from) halo_planes_kernel<true, false><<<(unsigned)blocks, 256, 0, s>>>(W, fc, J0, J1, from, to);
+    else if (to) halo_planes_kernel<false, true><<<(unsigned)blocks, 256, 0, s>>>(W, fc, J0, J1, from, to);
+    else halo_planes_kernel<false, false><<<(unsigned)blocks, 256, 0, s>>>(W, fc, J0, J1, from, to);
     return cudaGetLastError();
+}
+
+template <bool EXPAND>
+static cudaError_t rows_t(const double* src, double* dst, const FieldConst& fc, cudaStream_t s)
+{
+    const long long rows = 5LL * fc.nt * fc.nt;   // the components follow one another in both layouts
+    long long blocks = (rows + 7) / 8;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    rows_kernel<EXPAND><<<(unsigned)blocks, 256, 0, s>>>(src, dst, rows, fc.nt, fc.pitch);
+    return cudaGetLastError();
+}
+cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, cudaStream_t s)
+{
+    return rows_t<true>(dense, W, fc, s);
+}
+cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, cudaStream_t s)
+{
+    return rows_t<false>(W, dense, fc, s);
 }
 
 cudaError_t launch_clock_finish(DevClock* clock, double dt, cudaStream_t s)

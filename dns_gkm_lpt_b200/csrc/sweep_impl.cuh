@@ -33,12 +33,12 @@ struct Strides {
 };
 
 template <int DIR>
-__device__ __forceinline__ Strides strides(int nt)
+__device__ __forceinline__ Strides strides(const FieldConst& fc)
 {
-    const long long nt2 = (long long)nt * nt;
-    if (DIR == 0) return {nt, nt2, 1};   // normal i; window (j, k)
-    if (DIR == 1) return {nt2, nt, 1};   // normal j; window (i, k)
-    return {1, nt2, nt};                 // normal k; window (j, i)
+    const long long row = fc.pitch, plane = fc.nt * row;
+    if (DIR == 0) return {row, plane, 1};   // normal i; window (j, k)
+    if (DIR == 1) return {plane, row, 1};   // normal j; window (i, k)
+    return {1, plane, row};                 // normal k; window (j, i)
 }
 
 // Tangential neighbour faces in window coordinates (da, db): "N/S" feed the y-slot slope and
@@ -326,7 +326,7 @@ constexpr int kProbePolls = 256;
 __device__ __forceinline__ void halo_cell(double* __restrict__ W, const FieldConst& fc, long long g)
 {
     const int n = fc.n, nt = fc.nt;
-    const long long nt2 = (long long)nt * nt, nt3 = fc.nt3;
+    const long long nt2 = (long long)nt * nt, comp = fc.comp;
     const long long r1 = 6 * nt2, r2 = (long long)n * 6 * nt;
     int j, i, k;
     if (g < r1) {
@@ -352,14 +352,14 @@ __device__ __forceinline__ void halo_cell(double* __restrict__ W, const FieldCon
         k = m < 3 ? m : n + m;
     }
     auto wrap = [n](int x) { return x < 3 ? x + n : (x >= n + 3 ? x - n : x); };
-    const long long dst = ((long long)j * nt + i) * nt + k;
-    const long long src = ((long long)wrap(j) * nt + wrap(i)) * nt + wrap(k);
+    const long long dst = ((long long)j * nt + i) * fc.pitch + k;
+    const long long src = ((long long)wrap(j) * nt + wrap(i)) * fc.pitch + wrap(k);
 #pragma unroll
-    for (int q = 0; q < 5; q++) W[q * nt3 + dst] = W[q * nt3 + src];
+    for (int q = 0; q < 5; q++) W[q * comp + dst] = W[q * comp + src];
 }
 
 // Which data movement a sweep kernel is compiled for: tensor copies (the handle has tensor maps)
-// or per-element copies (odd nt).  The single-cube launches pick the form by the maps a launch
+// or per-element copies (no driver entry point for them).  The single-cube launches pick the form by the maps a launch
 // carries, so each kernel holds only its own path; the ensemble's persistent kernel serves
 // members with and without maps and decides per item.
 constexpr int kMapsRuntime = 0, kMapsOn = 1, kMapsOff = 2;
@@ -402,9 +402,9 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(
         kZPairs ? land + zland_elems<Tile>() : (kMLand ? mland + 5 * kWC : stage + 5 * kSweepThreads));
     const FieldConst& fc = a.fc;
-    const int n = fc.n, nt = fc.nt;
-    const long long nt3 = fc.nt3;
-    const Strides st = strides<DIR>(nt);
+    const int n = fc.n;
+    const long long comp = fc.comp;
+    const Strides st = strides<DIR>(fc);
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTB + tx;
     const int b0 = bx * kTB, a0 = by * kTA;
     const int f_begin = a.f0 + bz * a.seg_len;
@@ -478,7 +478,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
             const int A = a0 + aa - 1, B = b0 + bb - 1;
             if (A > n || B > n) continue;
             const long long idx = (A + 3) * st.sA + (B + 3) * st.sB + (long long)(f + 3) * st.sn;
-            store_cell(s, c, W[idx], W[nt3 + idx], W[2 * nt3 + idx], W[3 * nt3 + idx], W[4 * nt3 + idx]);
+            store_cell(s, c, W[idx], W[comp + idx], W[2 * comp + idx], W[3 * comp + idx], W[4 * comp + idx]);
         }
     };
 
@@ -494,7 +494,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
             if (A > n || B > n) continue;
             const long long idx = (A + 3) * st.sA + (B + 3) * st.sB + (long long)(f + 3) * st.sn;
 #pragma unroll
-            for (int q = 0; q < 5; q++) cp_async8(&dst[q * kWC + c], &W[q * nt3 + idx]);
+            for (int q = 0; q < 5; q++) cp_async8(&dst[q * kWC + c], &W[q * comp + idx]);
         }
         cp_async_commit();
     };
@@ -523,7 +523,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
         tma_phase ^= 1u;
         for (int f = f_begin - 3; f < f_begin + 3; f++) finish_slab(f);
     } else if (!kMixed) {
-        // FP64 otherwise (the z sweep, odd nt): the first six slabs by cp.async, one wait for all
+        // FP64 otherwise (the z sweep, or no maps): the first six slabs by cp.async, one wait for all
         for (int f = f_begin - 3; f < f_begin + 3; f++) issue_slab(f);
         cp_async_wait_all();
         for (int f = f_begin - 3; f < f_begin + 3; f++) finish_slab(f);
@@ -538,7 +538,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
 #pragma unroll
             for (int p = 0; p < 6; p++)
 #pragma unroll
-                for (int q = 0; q < 5; q++) v[p][q] = W[q * nt3 + idx0 + (long long)(f_begin + p) * st.sn];
+                for (int q = 0; q < 5; q++) v[p][q] = W[q * comp + idx0 + (long long)(f_begin + p) * st.sn];
 #pragma unroll
             for (int p = 0; p < 6; p++) store_cell(slot(f_begin - 3 + p), c, v[p][0], v[p][1], v[p][2], v[p][3], v[p][4]);
         }
@@ -852,7 +852,7 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
             const bool fetch_a = kFetchA && f >= f_begin && !zpair;
             if (fetch_a) {
 #pragma unroll
-                for (int q = 0; q < 5; q++) cp_async8(&stage[q * kSweepThreads + tid], &a.A[q * nt3 + ci]);
+                for (int q = 0; q < 5; q++) cp_async8(&stage[q * kSweepThreads + tid], &a.A[q * comp + ci]);
                 cp_async_commit();
             }
             T Fr[5];
@@ -867,12 +867,12 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
             if (f >= f_begin) {
                 if (DIR == 0) {
 #pragma unroll
-                    for (int q = 0; q < 5; q++) a.A[q * nt3 + ci] = __dsub_rn(F[q], Fprev[q]);
+                    for (int q = 0; q < 5; q++) a.A[q * comp + ci] = __dsub_rn(F[q], Fprev[q]);
                 } else if (DIR == 1) {
 #pragma unroll
                     for (int q = 0; q < 5; q++) {
                         double acc = stage[q * kSweepThreads + tid];
-                        a.A[q * nt3 + ci] = __dsub_rn(__dadd_rn(acc, F[q]), Fprev[q]);
+                        a.A[q * comp + ci] = __dsub_rn(__dadd_rn(acc, F[q]), Fprev[q]);
                     }
                 } else {
                     double wn[5];
@@ -885,16 +885,16 @@ __device__ __forceinline__ void sweep_block(const SweepArgs& a, int bx, int by, 
 #pragma unroll
                     for (int q = 0; q < 5; q++) {
                         double acc = zp ? zc[q * 2 * kTA * kTB]
-                                        : ((kFetchA && !zpair) ? stage[q * kSweepThreads + tid] : a.A[q * nt3 + ci]);
+                                        : ((kFetchA && !zpair) ? stage[q * kSweepThreads + tid] : a.A[q * comp + ci]);
                         double s = __dsub_rn(__dadd_rn(acc, F[q]), Fprev[q]);
                         // the cell's FP64 state (the FP64 ring holds it; the mixed ring has FP32 copies, so
                         // the mixed form reads it from the pair's state brick, or directly)
                         const double wq = kMixed ? ((sweep_state_bricks<T>() && zp) ? zc[(wbr - stage) + q * 2 * kTA * kTB]
-                                                                                    : W[q * nt3 + ci])
+                                                                                    : W[q * comp + ci])
                                                  : (double)wl[q * kWC + cc];
                         wn[q] = __dsub_rn(wq, __dmul_rn(fc.inv_dx, s));
                         if (zp) zc[q * 2 * kTA * kTB] = wn[q];
-                        else a.A[q * nt3 + ci] = wn[q];
+                        else a.A[q * comp + ci] = wn[q];
                     }
                     if (zp && !first_of_pair(f)) fence_async_shared();   // the brick's copy out reads it
                     const double ws = wave_speed_sq(wn, fc.gam, fc.gm1);

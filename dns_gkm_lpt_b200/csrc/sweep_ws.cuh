@@ -109,9 +109,9 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
     const unsigned bar_tma = smem_u32(bars);
     const unsigned bar_full0 = smem_u32(bars + 1), bar_empty0 = smem_u32(bars + 3);   // [2] each
     const FieldConst& fc = a.fc;
-    const int n = fc.n, nt = fc.nt;
-    const long long nt3 = fc.nt3;
-    const Strides st = strides<DIR>(nt);
+    const int n = fc.n;
+    const long long comp = fc.comp;
+    const Strides st = strides<DIR>(fc);
     const int tid = threadIdx.x;
     const int b0 = bx * kTB, a0 = by * Tile::TA;
     const int f_begin = a.f0 + bz * a.seg_len;
@@ -152,7 +152,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                 if (A > n || B > n) continue;
                 const long long idx = (A + 3) * st.sA + (B + 3) * st.sB + (long long)(f + 3) * st.sn;
 #pragma unroll
-                for (int q = 0; q < 5; q++) cp_async8(&dst[q * kWC + c], &W[q * nt3 + idx]);
+                for (int q = 0; q < 5; q++) cp_async8(&dst[q * kWC + c], &W[q * comp + idx]);
             }
             cp_async_commit();
         };
@@ -310,7 +310,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                 const bool fetch_a = kFetchA && f >= f_begin;
                 if (fetch_a) {
 #pragma unroll
-                    for (int q = 0; q < 5; q++) cp_async8(&stage[q * kConsumers + tid], &a.A[q * nt3 + ci]);
+                    for (int q = 0; q < 5; q++) cp_async8(&stage[q * kConsumers + tid], &a.A[q * comp + ci]);
                     cp_async_commit();
                 }
                 T F[5], Fr[5];
@@ -321,12 +321,12 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                 if (f >= f_begin) {
                     if (DIR == 0) {
 #pragma unroll
-                        for (int q = 0; q < 5; q++) a.A[q * nt3 + ci] = __dsub_rn(F[q], Fprev[q]);
+                        for (int q = 0; q < 5; q++) a.A[q * comp + ci] = __dsub_rn(F[q], Fprev[q]);
                     } else if (DIR == 1) {
 #pragma unroll
                         for (int q = 0; q < 5; q++) {
                             const double acc = stage[q * kConsumers + tid];
-                            a.A[q * nt3 + ci] = __dsub_rn(__dadd_rn(acc, F[q]), Fprev[q]);
+                            a.A[q * comp + ci] = __dsub_rn(__dadd_rn(acc, F[q]), Fprev[q]);
                         }
                     } else {
                         double wn[5];
@@ -335,7 +335,7 @@ __device__ __forceinline__ void sweep_block_ws(const SweepArgs& a, int bx, int b
                             const double acc = stage[q * kConsumers + tid];
                             const double s = __dsub_rn(__dadd_rn(acc, F[q]), Fprev[q]);
                             wn[q] = __dsub_rn((double)wl[q * kWC + cc], __dmul_rn(fc.inv_dx, s));
-                            a.A[q * nt3 + ci] = wn[q];
+                            a.A[q * comp + ci] = wn[q];
                         }
                         const double ws = wave_speed_sq(wn, fc.gam, fc.gm1);
                         if (!isfinite(ws) || !(wn[0] > 0.0)) bad = true;
