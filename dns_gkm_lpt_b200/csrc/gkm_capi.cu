@@ -178,32 +178,54 @@ cudaError_t launch_sweep_any(gkm_handle* h, int dir, gkm::SweepArgs a)
     return gkm::launch_sweep(dir, c.variant, a, c.nseg, h->stream);
 }
 
-// Segments along the sweep normal, from a model of the launch: a segment of L faces takes L + 1 face planes
-// (it recomputes its first face) and about one plane's time for its six-slab prologue, and a launch as many
-// rounds of segments as its CTAs fill the SMs' places, so the length with the smallest
-// rounds x (L + 2) is taken, the longest of equals.  Small cubes leave SMs idle and get short segments: measured
-// per sweep in FP64, 64^3 0.104 ms with 16 faces, 0.071 with 8; 16^3 0.094 ms with 16 and 0.053 with 8 faces; 256^3
-// 2.70 ms with 86 faces, 2.60 with 64.
-SweepChoice default_choice(const FieldConst& fc, bool mixed, int variant, int dir)
+// Default sweep shapes, from a model of the launch.  A segment of L faces takes L + p units of time (it
+// recomputes its first face, and its six-slab prologue is latency), p from short segments; with r the
+// launch's CTAs over the SMs' places, one CTA per SM runs in ceil(r) rounds.  Several per SM fill in for one
+// another: r + 0.3 rounds if that is less, at least 1.7 for a second one; a single round starts all CTAs
+// in step and takes 1.1, or 0.93 while no SM holds more than half of its places.  CTAs of several rounds
+// drift apart by some 0.15 L.  In z, several CTAs per SM, odd lengths split pairs of cells.  The units' cost is
+// relative to the 16 x 8 windows of the same direction.  Candidates: x, y the 16 x 8 windows and the warp-specialized ones; z (whose
+// bricks those do without) the 16 x 8 and 16 x 16 windows.  The least cost, of equals the longest segments.
+// Measured against the model with 16 x 8 windows only and whole rounds: x at 96^3 0.159 -> 0.148 ms
+// (warp-specialized, one round), at 128^3 0.395 -> 0.368, at 512^3 19.75 -> 19.40 (256 faces for 512), z at 128^3
+// 0.452 -> 0.436, at 64^3 0.083 -> 0.076 (16 x 16), mixed x at 128^3 0.217 -> 0.197, mixed z at 256^3 1.97 -> 1.89.
+SweepChoice default_choice(const FieldConst& fc, bool mixed, int dir)
 {
-    const gkm::SweepShape sh = gkm::sweep_shape(mixed, variant);
-    const long long tiles = (long long)((fc.n + sh.TB - 1) / sh.TB) * ((fc.n + sh.TA - 1) / sh.TA);
-    const long long places = 148LL * (mixed && dir == 2 ? gkm::kMixedZCtas : sh.ctas);
-    SweepChoice c;
-    c.variant = variant;
-    long long best = -1;
-    for (int nseg = 1; nseg <= fc.n; nseg++) {
-        const int L = (fc.n + nseg - 1) / nseg;
-        if (nseg > 1 && L == c.seg_len) continue;   // the same segments
-        const long long ctas = tiles * ((fc.n + L - 1) / L);
-        const long long cost = (ctas + places - 1) / places * (L + 2);
-        if (best < 0 || cost < best) {
-            best = cost;
-            c.seg_len = L;
+    struct Form {
+        int variant;
+        double cost, extra;
+    };
+    const Form forms[2][2] = {{{0, 1.0, 2.6}, {2, 1.025, 3.1}}, {{0, 1.0, 4.5}, {1, 1.05, 4.0}}};   // x and y; z
+    const Form mixed_forms[2] = {{0, 1.0, 2.6}, {0, 1.0, 6.0}};
+    SweepChoice best;
+    double least = -1.0;
+    for (int k = 0; k < (mixed ? 1 : 2); k++) {
+        const Form& form = mixed ? mixed_forms[dir == 2] : forms[dir == 2][k];
+        if (!mixed && form.variant == 2 && !gkm::ws_ready()) continue;
+        const gkm::SweepShape sh = gkm::sweep_shape(mixed, form.variant);
+        const int per_sm = mixed && dir == 2 ? gkm::kMixedZCtas : (form.variant == 2 ? 1 : sh.ctas);
+        const long long tiles = (long long)((fc.n + sh.TB - 1) / sh.TB) * ((fc.n + sh.TA - 1) / sh.TA);
+        int last = 0;
+        for (int nseg = 1; nseg <= fc.n; nseg++) {
+            const int L = (fc.n + nseg - 1) / nseg;
+            if (L == last) continue;   // the same segments
+            last = L;
+            const double r = (double)(tiles * ((fc.n + L - 1) / L)) / (148.0 * per_sm);
+            const double rounds = per_sm == 1 ? std::ceil(r)
+                                  : r <= 0.5  ? 0.93
+                                  : r <= 1.0  ? 1.1
+                                              : std::max(std::min(r + 0.3, std::ceil(r)), 1.7);
+            const double split = dir == 2 && per_sm > 1 && L > 1 && L % 2 ? 0.8 : 0.0;
+            const double cost = rounds * (L + form.extra + split) * form.cost + (r > 1.0 ? 0.15 * L : 0.0);
+            if (least < 0.0 || cost < least) {
+                least = cost;
+                best.variant = form.variant;
+                best.seg_len = L;
+            }
         }
     }
-    c.nseg = (fc.n + c.seg_len - 1) / c.seg_len;
-    return c;
+    best.nseg = (fc.n + best.seg_len - 1) / best.seg_len;
+    return best;
 }
 
 // enqueue one Eulerian step on h->stream (no host synchronisation)
@@ -565,7 +587,6 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     fc.dK2 = (K + 3) - 2.0 / fc.gm1;
     fc.suth_c = fc.mu0 * (fc.T0 + 110.4) * gkm::kR / ((gkm::kR * fc.T0) * std::sqrt(gkm::kR * fc.T0));
 
-    for (int d = 0; d < 3; d++) h->sweep[d] = default_choice(fc, cfg->precision == GKM_PREC_MIXED, 0, d);
 
     auto bail = [&](cudaError_t e, const char* where) {
         gkm_status s = cuda_fail(h, e, where);
@@ -647,6 +668,7 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     if (e == cudaSuccess) e = gkm::sweep_mixed_prepare();
     if (e == cudaSuccess) e = gkm::spline_prepare();
     if (e != cudaSuccess) return bail(e, "sweep_prepare");
+    for (int d = 0; d < 3; d++) h->sweep[d] = default_choice(fc, cfg->precision == GKM_PREC_MIXED, d);
     e = setup_batched_splines(h);
     if (e != cudaSuccess) return bail(e, "batched spline build");
     e = setup_tensor_maps(h);
@@ -880,6 +902,7 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
         }
         h->sweep[d] = best;
     }
+    h->sweep_chosen = true;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaMemcpyAsync(h->clock, &saved, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream);
@@ -918,6 +941,7 @@ gkm_status gkm_set_sweep_config(gkm_handle* h, const int32_t in[6])
         h->sweep[d].seg_len = in[2 * d + 1] < h->fc.n ? in[2 * d + 1] : h->fc.n;
         h->sweep[d].nseg = (h->fc.n + h->sweep[d].seg_len - 1) / h->sweep[d].seg_len;
     }
+    h->sweep_chosen = true;
     destroy_graphs(h);
     return GKM_OK;
 }
@@ -1091,7 +1115,7 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
             // launch has enough CTAs to fill the SMs beside the other stream's (measured: 256^3
             // -2.5 %, 512^3 -8 % per pinned step against the whole-cube segment lengths)
             ad.seg_len = (d == 1) ? j1 - j0 : std::min(h->sweep[d].seg_len, C);
-            const int v = h->sweep[d].variant;
+            const int v = h->sweep_chosen ? h->sweep[d].variant : 0;   // the defaults are for whole-cube launches
             ad.tmap = sweep_tmap(h, ad.W, d, v);
             ad.tmap_acc = sweep_tmap_acc(h, ad.A, d, v);
             ad.tmap_wb = sweep_tmap_wb(h, ad.W, d, v);

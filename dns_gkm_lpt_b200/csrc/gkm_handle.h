@@ -20,6 +20,7 @@ struct gkm_handle {
     gkm_config cfg{};
     gkm::FieldConst fc{};
     SweepChoice sweep[3];
+    bool sweep_chosen = false;   // by autotune or the caller, not the defaults
     cudaStream_t own_stream = nullptr, stream = nullptr;
     double* buf[2] = {nullptr, nullptr};
     int parity = 0;
