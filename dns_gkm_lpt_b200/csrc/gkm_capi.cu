@@ -367,6 +367,11 @@ gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
     if (!h) return GKM_ERR_ARG;
     if (nsteps < 0) return fail(h, GKM_ERR_ARG, "nsteps < 0");
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
+    if (nsteps > 0) {
+        gkm_status s = gkm_host::take_view(h);
+        if (s != GKM_OK) return s;
+        if (kind != kGraphParticles) h->view_live = false;
+    }
     for (int s = 0; s < nsteps; s++) {
         const int p = h->parity;
         if (h->cfg.use_graphs) {
@@ -421,6 +426,8 @@ gkm_status read_clock(gkm_handle* h, DevClock* c)
 gkm_status ensure_splines(gkm_handle* h)
 {
     if (h->splines_valid) return GKM_OK;
+    gkm_status s = gkm_host::take_view(h);
+    if (s != GKM_OK) return s;
     CK(h, enqueue_splines(h, h->buf[h->parity]));
     h->splines_valid = true;
     return GKM_OK;
@@ -453,7 +460,8 @@ gkm_status compute_props(gkm_handle* h)
 {
     if (h->spline_f32)
         return fail(h, GKM_ERR_CONFIG, "particle properties need FP64 velocity-spline coefficients");
-    gkm_status s = ensure_splines(h);
+    gkm_status s = gkm_host::take_view(h);
+    if (s == GKM_OK) s = ensure_splines(h);
     if (s != GKM_OK) return s;
     const long long M = h->grid.npts + h->grid.pad;
     for (int c = 0; c < 5; c++)
@@ -488,10 +496,22 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 {
     *dense = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
+    if (h->view_live) {
+        *dense = h->view;
+        return GKM_OK;
+    }
     double* out = h->buf[h->parity ^ 1];
     CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->stream));
     h->launches += 1;
     *dense = out;
+    return GKM_OK;
+}
+
+gkm_status gkm_host::take_view(gkm_handle* h)
+{
+    if (!h->view_live) return GKM_OK;
+    CK(h, gkm::launch_rows_expand(h->view, h->buf[h->parity], h->fc, h->stream));
+    h->launches += 1;
     return GKM_OK;
 }
 
@@ -708,6 +728,7 @@ gkm_status gkm_destroy(gkm_handle* h)
     cudaFree(h->lap_nodes);
     cudaFree(h->props);
     cudaFree(h->pipe_dense);
+    cudaFree(h->view);
     for (cudaEvent_t e : h->pipe_ev) cudaEventDestroy(e);
     for (cudaStream_t s : {h->pipe_in, h->pipe_out, h->pipe_comp[0], h->pipe_comp[1], h->pipe_comp[2], h->pipe_comp[3],
                            h->pipe_halo})
@@ -726,8 +747,8 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
         if (!W[q]) return fail(h, GKM_ERR_ARG, "W[q] is NULL");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
     double* dst = h->buf[h->parity];
-    // odd grids: dense rows through the accumulator buffer, free between steps, then to their pitch
-    double* land = h->fc.pitch == h->fc.nt ? dst : h->buf[h->parity ^ 1];
+    // odd grids: dense rows through the view or the accumulator buffer, free between steps, then to their pitch
+    double* land = h->fc.pitch == h->fc.nt ? dst : (h->view_live ? h->view : h->buf[h->parity ^ 1]);
     for (int q = 0; q < 5; q++)
         CK(h, cudaMemcpyAsync(land + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
     if (land != dst) {
@@ -764,7 +785,8 @@ gkm_status gkm_timestep(gkm_handle* h, double* dt_out)
 {
     if (!h) return GKM_ERR_ARG;
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
-    gkm_status s = reduce_wave(h);
+    gkm_status s = gkm_host::take_view(h);
+    if (s == GKM_OK) s = reduce_wave(h);
     if (s != GKM_OK) return s;
     DevClock c;
     s = read_clock(h, &c);
@@ -798,6 +820,11 @@ gkm_status gkm_step_timed(gkm_handle* h, int32_t nsteps, int32_t with_particles,
 {
     if (!h || !ms || nsteps < 0) return GKM_ERR_ARG;
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
+    if (nsteps > 0) {
+        gkm_status s = gkm_host::take_view(h);
+        if (s != GKM_OK) return s;
+        h->view_live = false;
+    }
     for (int k = 0; k < 7; k++) ms[k] = 0.0;
     cudaEvent_t ev[7];
     for (int k = 0; k < 7; k++) CK(h, cudaEventCreate(&ev[k]));
@@ -849,6 +876,10 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
 {
     if (!h || reps < 1) return GKM_ERR_ARG;
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
+    {
+        gkm_status s = gkm_host::take_view(h);
+        if (s != GKM_OK) return s;
+    }
     const bool mixed = h->cfg.precision == GKM_PREC_MIXED;
     const int nvar = mixed ? gkm::kSweepVariants32 : gkm::kSweepVariants64;
     // the sweeps leave W untouched (they write the accumulator A only); the clock
@@ -1139,6 +1170,7 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
     CK(h, copy_out(n + 3, n + 6, h->stream));
     CK(h, cudaStreamWaitEvent(h->stream, ev_done_out, 0));
     h->parity ^= 1;
+    h->view_live = false;
     h->state_loaded = true;
     h->splines_valid = false;
     DevClock c;
@@ -1177,6 +1209,7 @@ gkm_status gkm_evolve(gkm_handle* h, double* const W[5], double dt)
     h->dt_fixed_mode = 1;
     h->dt_fixed = dt;
     cudaError_t e = enqueue_eulerian(h);
+    h->view_live = false;
     h->dt_fixed_mode = mode;
     h->dt_fixed = val;
     if (e != cudaSuccess) return cuda_fail(h, e, "evolve");
@@ -1273,7 +1306,8 @@ gkm_status gkm_stats_compute(gkm_handle* h, gkm_stats* out)
 {
     if (!h || !out) return GKM_ERR_ARG;
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
-    gkm_status s = ensure_splines(h);
+    gkm_status s = gkm_host::take_view(h);
+    if (s == GKM_OK) s = ensure_splines(h);
     if (s != GKM_OK) return s;
     const double* c[3] = {h->coef[0], h->coef[1], h->coef[2]};
     const float* c32[3] = {h->coef32[0], h->coef32[1], h->coef32[2]};
@@ -1388,6 +1422,18 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
 {
     if (!h || !W) return GKM_ERR_ARG;
     *W = h->buf[h->parity];
+    if (h->fc.pitch == h->fc.nt) return GKM_OK;
+    if (!h->view) CK(h, cudaMalloc(&h->view, sizeof(double) * 5 * (size_t)h->fc.nt3));
+    if (!h->view_live) {
+        CK(h, gkm::launch_rows_compact(*W, h->view, h->fc, h->stream));
+        h->launches += 1;
+        // the caller may read it on any stream, as it may the state of an idle handle
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        CK(h, cudaStreamIsCapturing(h->stream, &capture));
+        if (capture == cudaStreamCaptureStatusNone) CK(h, cudaStreamSynchronize(h->stream));
+        h->view_live = true;
+    }
+    *W = h->view;
     return GKM_OK;
 }
 

@@ -93,10 +93,14 @@ gkm_status refresh(gkm_ensemble* E, bool need_state)
     const int nm = nm_of(E);
     const int parity = E->mem[0]->parity;
     for (int m = 0; m < nm; m++) {
-        const gkm_handle* h = E->mem[m];
+        gkm_handle* h = E->mem[m];
         if (need_state && !h->state_loaded) return efail(E, GKM_ERR_STATE, "member " + std::to_string(m) + ": no state uploaded");
         if (h->parity != parity)
             return efail(E, GKM_ERR_STATE, "member " + std::to_string(m) + " was stepped outside the ensemble");
+    }
+    for (int m = 0; need_state && m < nm; m++) {
+        gkm_status s = gkm_host::take_view(E->mem[m]);
+        if (s != GKM_OK) return efail(E, s, E->mem[m]->err);
     }
     std::vector<MemberDev> hm((size_t)nm);
     std::vector<long long> off((size_t)kNumSets * (nm + 1), 0);
@@ -230,6 +234,7 @@ void finish_step(gkm_ensemble* E, bool parts)
 {
     for (gkm_handle* h : E->mem) {
         h->parity ^= 1;
+        h->view_live = false;
         h->splines_valid = parts && h->np > 0;
     }
 }
