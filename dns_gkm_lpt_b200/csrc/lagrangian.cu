@@ -75,209 +75,89 @@ __device__ __forceinline__ void fixed_pivots(int N, const SplineTables& tb, doub
     r_inf = reached ? tb.mt[kPivotRows] : 0.0;
 }
 
-template <int U, class Src>
+// IN_PLACE: the forward value of point i lies in slot i, where the input of point i was, instead of slot
+// i + 1, so c may be the storage f reads (same stride) as long as slots N .. N+pad-1 exist.
+// REREAD: the forward sweep stores one value in U, and the backward sweep forms the others again
+// from the inputs: the line is read twice and written once instead of twice.  For inputs that cost
+// no more than their load (pass 1: DRAM writes weigh more than reads; three components at 256^3, all passes, 1.44 -> 1.31 ms, at 512^3 9.99 -> 8.90);
+// pass 0's cost a division each.
+template <int U, bool IN_PLACE, bool REREAD, class Src>
 __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables& tb, double* c, long long cs)
 {
     double d_inf, r_inf;
     fixed_pivots(N, tb, d_inf, r_inf);
-    if (!periodic) {
-        const double c0 = f(0), cl = f(N - 1);
-        double rp = 0.0;
-        auto fwd = [&](int i, double fi, double m) {
-            double r = mul(6.0, fi);
-            if (i == 1) r = sub(r, c0);
-            if (i == N - 2) r = sub(r, cl);
-            rp = (i == 1) ? r : sub(r, mul(m, rp));
-            c[(long long)(i + 1) * cs] = rp;
-        };
-        int i = 1;
-        for (; i + U - 1 <= N - 2; i += U) {
-            double fv[U];
+    const int lo = periodic ? 0 : 1, hi = periodic ? N - 1 : N - 2;   // the points solved for
+    const double c0 = periodic ? 0.0 : f(0), cl = periodic ? 0.0 : f(N - 1);
+    auto fwd = [&](int i) -> double& { return c[(long long)(i + (IN_PLACE ? 0 : 1)) * cs]; };
+    double rp = 0.0;
+    auto eliminate = [&](int i, double fi, double m) {
+        double r = mul(6.0, fi);
+        if (!periodic && i == 1) r = sub(r, c0);
+        if (!periodic && i == N - 2) r = sub(r, cl);
+        rp = (i == lo) ? r : sub(r, mul(m, rp));
+    };
+    int top = lo;   // batches of U points, the last point not among them, then the others one by one
+    for (; top + U - 1 < hi; top += U) {
+        double fv[U];
 #pragma unroll
-            for (int u = 0; u < U; u++) fv[u] = f(i + u);
+        for (int u = 0; u < U; u++) fv[u] = f(top + u);
 #pragma unroll
-            for (int u = 0; u < U; u++) fwd(i + u, fv[u], i > kPivotRows ? r_inf : tb.mt[i + u]);
+        for (int u = 0; u < U; u++) {
+            eliminate(top + u, fv[u], top > kPivotRows ? r_inf : tb.mt[top + u]);
+            if (!REREAD || u == 0) fwd(top + u) = rp;
         }
-        for (; i <= N - 2; i++) fwd(i, f(i), tb.mt[i]);
-        double x = __ddiv_rn(c[(long long)(N - 1) * cs], tb.dp[N - 2]);
-        c[(long long)(N - 1) * cs] = x;
-        i = N - 3;
-        for (; i - U + 1 >= 1; i -= U) {
-            double cv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u + 1) * cs];
-            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
-#pragma unroll
-                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
-            } else {
-#pragma unroll 1
-                for (int k = i; k > i - U; k--) {
-                    x = __ddiv_rn(sub(c[(long long)(k + 1) * cs], x), tb.dp[k]);
-                    c[(long long)(k + 1) * cs] = x;
-                }
-            }
-        }
-#pragma unroll 1
-        for (; i >= 1; i--) {
-            x = __ddiv_rn(sub(c[(long long)(i + 1) * cs], x), tb.dp[i]);
-            c[(long long)(i + 1) * cs] = x;
-        }
-        // x now holds c_1 (or c_{N-2} when N == 3)
-        const double x1 = (N - 2 >= 1) ? c[2 * cs] : cl;
-        const double xl2 = (N - 2 >= 1) ? c[(long long)(N - 1) * cs] : c0;
-        c[cs] = c0;
-        c[(long long)N * cs] = cl;
-        c[0] = sub(2.0 * c0, x1);
-        c[(long long)(N + 1) * cs] = sub(2.0 * cl, xl2);
-    } else {
-        // y = B^-1 (6 f) stored in slots 1..N
-        double rp = mul(6.0, f(0));
-        c[cs] = rp;
-        int i = 1;
-        for (; i + U - 1 <= N - 1; i += U) {
-            double fv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) fv[u] = f(i + u);
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                rp = sub(mul(6.0, fv[u]), mul(i > kPivotRows ? r_inf : tb.mt[i + u], rp));
-                c[(long long)(i + u + 1) * cs] = rp;
-            }
-        }
-        for (; i < N; i++) {
-            rp = sub(mul(6.0, f(i)), mul(tb.mt[i], rp));
-            c[(long long)(i + 1) * cs] = rp;
-        }
-        double x = __ddiv_rn(c[(long long)N * cs], tb.dp[N - 1]);
-        c[(long long)N * cs] = x;
-        i = N - 2;
-        for (; i - U + 1 >= 0; i -= U) {
-            double cv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u + 1) * cs];
-            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
-#pragma unroll
-                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
-            } else {
-#pragma unroll 1
-                for (int k = i; k > i - U; k--) {
-                    x = __ddiv_rn(sub(c[(long long)(k + 1) * cs], x), tb.dp[k]);
-                    c[(long long)(k + 1) * cs] = x;
-                }
-            }
-        }
-#pragma unroll 1
-        for (; i >= 0; i--) {
-            x = __ddiv_rn(sub(c[(long long)(i + 1) * cs], x), tb.dp[i]);
-            c[(long long)(i + 1) * cs] = x;
-        }
-        const double fac = __ddiv_rn(add(c[cs], mul(-0.25, c[(long long)N * cs])), tb.denom);
-        for (int i = 0; i < N; i++) c[(long long)(i + 1) * cs] = sub(c[(long long)(i + 1) * cs], mul(fac, tb.z[i]));
-        c[0] = c[(long long)N * cs];
-        c[(long long)(N + 1) * cs] = c[cs];
-        c[(long long)(N + 2) * cs] = c[2 * cs];
     }
-}
-
-// line_solve with the intermediate results stored one slot lower (the forward value of point i in
-// slot i, where the input of point i was), so the line may be solved in place: c may be the
-// storage f reads (same stride), as long as slots N .. N+pad-1 exist past the N inputs.  The
-// arithmetic and its order are those of line_solve, so the coefficients are identical.
-template <int U, class Src>
-__device__ void line_solve_ip(const Src& f, int N, int periodic, const SplineTables& tb, double* c, long long cs)
-{
-    double d_inf, r_inf;
-    fixed_pivots(N, tb, d_inf, r_inf);
-    if (!periodic) {
-        const double c0 = f(0), cl = f(N - 1);
-        double rp = 0.0;
-        auto fwd = [&](int i, double fi, double m) {
-            double r = mul(6.0, fi);
-            if (i == 1) r = sub(r, c0);
-            if (i == N - 2) r = sub(r, cl);
-            rp = (i == 1) ? r : sub(r, mul(m, rp));
-            c[(long long)i * cs] = rp;
-        };
-        int i = 1;
-        for (; i + U - 1 <= N - 2; i += U) {
-            double fv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) fv[u] = f(i + u);
-#pragma unroll
-            for (int u = 0; u < U; u++) fwd(i + u, fv[u], i > kPivotRows ? r_inf : tb.mt[i + u]);
-        }
-        for (; i <= N - 2; i++) fwd(i, f(i), tb.mt[i]);
-        double x = __ddiv_rn(c[(long long)(N - 2) * cs], tb.dp[N - 2]);
-        c[(long long)(N - 1) * cs] = x;
-        i = N - 3;
-        for (; i - U + 1 >= 1; i -= U) {
-            double cv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u) * cs];
-            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
-#pragma unroll
-                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
-            } else {
 #pragma unroll 1
-                for (int k = i; k > i - U; k--) {
-                    x = __ddiv_rn(sub(c[(long long)(k) * cs], x), tb.dp[k]);
-                    c[(long long)(k + 1) * cs] = x;
+    for (int i = top; i <= hi; i++) {
+        eliminate(i, f(i), tb.mt[i]);
+        fwd(i) = rp;
+    }
+    double x = 0.0, xl = 0.0;
+    if (hi >= lo) {
+        x = xl = __ddiv_rn(rp, tb.dp[hi]);
+        c[(long long)(hi + 1) * cs] = x;
+    }
+    auto divide = [&](int i) {
+        x = __ddiv_rn(sub(fwd(i), x), tb.dp[i]);
+        c[(long long)(i + 1) * cs] = x;
+    };
+#pragma unroll 1
+    for (int i = hi - 1; i >= top; i--) divide(i);
+    for (int s = top - U; s >= lo; s -= U) {   // points s + U - 1 down to s
+        double cv[U];
+        const bool fixed = s > kPivotRows;
+        cv[U - 1] = fwd(s);
+#pragma unroll
+        for (int u = 1; u < U; u++) cv[U - 1 - u] = REREAD ? f(s + u) : fwd(s + u);
+        if (REREAD) {
+#pragma unroll
+            for (int u = 1; u < U; u++)
+                cv[U - 1 - u] = sub(mul(6.0, cv[U - 1 - u]), mul(fixed ? r_inf : tb.mt[s + u], cv[U - u]));
+        }
+        if (back_rows<U>(cv, s + U - 1, tb, d_inf, r_inf, x)) {
+#pragma unroll
+            for (int u = 0; u < U; u++) c[(long long)(s + U - u) * cs] = cv[u];
+        } else {
+            if (REREAD) {
+                double r = fwd(s);
+#pragma unroll 1
+                for (int i = s + 1; i < s + U; i++) {
+                    r = sub(mul(6.0, f(i)), mul(tb.mt[i], r));
+                    fwd(i) = r;
                 }
             }
-        }
 #pragma unroll 1
-        for (; i >= 1; i--) {
-            x = __ddiv_rn(sub(c[(long long)i * cs], x), tb.dp[i]);
-            c[(long long)(i + 1) * cs] = x;
+            for (int i = s + U - 1; i >= s; i--) divide(i);
         }
-        const double x1 = (N - 2 >= 1) ? c[2 * cs] : cl;
-        const double xl2 = (N - 2 >= 1) ? c[(long long)(N - 1) * cs] : c0;
+    }
+    if (!periodic) {
+        // x: the solution of point 1, xl: of point N - 2 (the ends themselves when there is none)
         c[cs] = c0;
         c[(long long)N * cs] = cl;
-        c[0] = sub(2.0 * c0, x1);
-        c[(long long)(N + 1) * cs] = sub(2.0 * cl, xl2);
+        c[0] = sub(2.0 * c0, hi >= lo ? x : cl);
+        c[(long long)(N + 1) * cs] = sub(2.0 * cl, hi >= lo ? xl : c0);
     } else {
-        double rp = mul(6.0, f(0));
-        c[0] = rp;
-        int i = 1;
-        for (; i + U - 1 <= N - 1; i += U) {
-            double fv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) fv[u] = f(i + u);
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                rp = sub(mul(6.0, fv[u]), mul(i > kPivotRows ? r_inf : tb.mt[i + u], rp));
-                c[(long long)(i + u) * cs] = rp;
-            }
-        }
-        for (; i < N; i++) {
-            rp = sub(mul(6.0, f(i)), mul(tb.mt[i], rp));
-            c[(long long)i * cs] = rp;
-        }
-        double x = __ddiv_rn(c[(long long)(N - 1) * cs], tb.dp[N - 1]);
-        c[(long long)N * cs] = x;
-        i = N - 2;
-        for (; i - U + 1 >= 0; i -= U) {
-            double cv[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) cv[u] = c[(long long)(i - u) * cs];
-            if (back_rows<U>(cv, i, tb, d_inf, r_inf, x)) {
-#pragma unroll
-                for (int u = 0; u < U; u++) c[(long long)(i - u + 1) * cs] = cv[u];
-            } else {
-#pragma unroll 1
-                for (int k = i; k > i - U; k--) {
-                    x = __ddiv_rn(sub(c[(long long)(k) * cs], x), tb.dp[k]);
-                    c[(long long)(k + 1) * cs] = x;
-                }
-            }
-        }
-#pragma unroll 1
-        for (; i >= 0; i--) {
-            x = __ddiv_rn(sub(c[(long long)i * cs], x), tb.dp[i]);
-            c[(long long)(i + 1) * cs] = x;
-        }
-        const double fac = __ddiv_rn(add(c[cs], mul(-0.25, c[(long long)N * cs])), tb.denom);
+        const double fac = __ddiv_rn(add(x, mul(-0.25, xl)), tb.denom);
         for (int i = 0; i < N; i++) c[(long long)(i + 1) * cs] = sub(c[(long long)(i + 1) * cs], mul(fac, tb.z[i]));
         c[0] = c[(long long)N * cs];
         c[(long long)(N + 1) * cs] = c[cs];
@@ -320,7 +200,7 @@ __device__ __forceinline__ void pass0_line(const double* __restrict__ W, const F
         if constexpr (VEL) return __ddiv_rn(W[q * comp + idx], W[idx]);
         else return spline_source(W, comp, fc.gm1, q, idx);
     };
-    line_solve<U>(f, N, g.periodic, tb, out + L, lines);
+    line_solve<U, false, false>(f, N, g.periodic, tb, out + L, lines);
 }
 
 template <bool VEL>
@@ -341,7 +221,7 @@ __device__ __forceinline__ void pass1_line(const double* __restrict__ in, const 
     const int a = (int)(L / N), k = (int)(L - (long long)a * N);
     const double* src = in + (long long)a * N * N + k;
     auto f = [&](int i) { return src[(long long)i * N]; };
-    line_solve<U>(f, N, g.periodic, tb, out + (long long)a * M * N + k, N);
+    line_solve<U, false, true>(f, N, g.periodic, tb, out + (long long)a * M * N + k, N);
 }
 
 __global__ void spline_pass1(const double* __restrict__ in, SplineGrid g, SplineTables tb, double* __restrict__ out)
@@ -361,10 +241,11 @@ constexpr int kLineChunk = 32;
 constexpr int kPass2Warps = 4;
 
 // Rows of one line staged in shared memory: row[t] holds point i0 + t.  Forward elimination of the
-// points [i_lo, i_hi] in that chunk, and back substitution of the same points downwards (the
+// points [i_lo, i_hi] in that chunk (given: rp is the value of the point before i_lo), and back substitution of the same points downwards (the
 // line's last row, whose pivot has no tabled reciprocal, divided first).
 __device__ __forceinline__ void chunk_forward(double* row, int i0, int i_lo, int i_hi, int N, int periodic,
-                                              const SplineTables& tb, double c0, double cl, double r_inf, double& rp)
+                                              const SplineTables& tb, double c0, double cl, double r_inf, double& rp,
+                                              bool given = false)
 {
     const int a = max(i_lo, i0), b = min(i_hi, i0 + kLineChunk - 1);
 #pragma unroll 8
@@ -374,7 +255,7 @@ __device__ __forceinline__ void chunk_forward(double* row, int i0, int i_lo, int
             if (i == 1) r = sub(r, c0);
             if (i == N - 2) r = sub(r, cl);
         }
-        rp = (i == i_lo) ? r : sub(r, mul(i > kPivotRows ? r_inf : tb.mt[i], rp));
+        rp = (i == i_lo && !given) ? r : sub(r, mul(i > kPivotRows ? r_inf : tb.mt[i], rp));
         row[i - i0] = rp;
     }
 }
@@ -451,20 +332,30 @@ __device__ __forceinline__ void pass2_group(const double* __restrict__ in, const
     fixed_pivots(N, tb, d_inf, r_inf);
     const double* src = in + myL * N;
     double* dst = out + myL * M;
+    // The forward value before each chunk is kept in the output rows, 32 lanes side by side at the
+    // first row's slots s0 .. s0 + 31 (beyond its end, in the next row's first slots), until the backward
+    // sweep, which forms the chunk's forward values again, overwrites them with that chunk (the first
+    // slots come last): the lines are read twice and written once instead of twice.
+    double* keep = out + L0 * M + lane;
     if (!g.periodic) {
         const double c0 = mine ? src[0] : 0.0, cl = mine ? src[N - 1] : 0.0;
-        // forward elimination: slot i+1 <- rp_i for i = 1..N-2 (values 0 and N-1 land in slots 1, N)
+        // forward elimination of points 1..N-2 (values 0 and N-1 land in slots 1, N)
         double rp = 0.0;
         for (int s0 = 0; s0 <= s_last; s0 += kLineChunk) {
             load_in(s0);
-            if (mine) chunk_forward(sm[lane], s0 - 1, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
-            store_out(s0);
+            if (mine) {
+                keep[s0] = rp;
+                chunk_forward(sm[lane], s0 - 1, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
+            }
+            __syncwarp();
         }
         // back substitution, chunks in descending order
         double x = 0.0, x1 = 0.0, xl2 = 0.0;
         for (int s0 = s_last; s0 >= 0; s0 -= kLineChunk) {
-            load_out(s0);
+            load_in(s0);
             if (mine) {
+                rp = keep[s0];
+                chunk_forward(sm[lane], s0 - 1, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
                 chunk_back(sm[lane], s0 - 1, 1, N - 2, tb, d_inf, r_inf, x);
                 if (s0 - 1 <= N - 2 && N - 2 < s0 - 1 + kLineChunk) xl2 = sm[lane][N - 2 - (s0 - 1)];
                 x1 = x;   // the last chunk's last value is the solution of point 1
@@ -481,13 +372,18 @@ __device__ __forceinline__ void pass2_group(const double* __restrict__ in, const
         double rp = 0.0;
         for (int s0 = 0; s0 <= s_last; s0 += kLineChunk) {
             load_in(s0);
-            if (mine) chunk_forward(sm[lane], s0 - 1, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
-            store_out(s0);
+            if (mine) {
+                keep[s0] = rp;
+                chunk_forward(sm[lane], s0 - 1, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
+            }
+            __syncwarp();
         }
         double x = 0.0, x0 = 0.0, xl = 0.0;
         for (int s0 = s_last; s0 >= 0; s0 -= kLineChunk) {
-            load_out(s0);
+            load_in(s0);
             if (mine) {
+                rp = keep[s0];
+                chunk_forward(sm[lane], s0 - 1, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
                 chunk_back(sm[lane], s0 - 1, 0, N - 1, tb, d_inf, r_inf, x);
                 if (s0 - 1 <= N - 1 && N - 1 < s0 - 1 + kLineChunk) xl = sm[lane][N - 1 - (s0 - 1)];
                 x0 = x;   // the last chunk's last value is the solution of point 0
@@ -553,12 +449,12 @@ __global__ void spline_pass1_inplace(double* buf, SplineGrid g, SplineTables tb)
         const int a = (int)(L / N), k = (int)(L - (long long)a * N);
         double* line = buf + (long long)a * M * N + k;
         auto f = [&](int i) { return line[(long long)i * N]; };
-        line_solve_ip<kLineBatchSingle>(f, N, g.periodic, tb, line, N);
+        line_solve<kLineBatchSingle, true, true>(f, N, g.periodic, tb, line, N);
     }
 }
 
 // pass 2 with FP32 output: the lines of [M0][M1][N2] along axis 2, 32 per warp through shared
-// memory as pass2_group, the forward values stored in the line's own slots (slot i); natural ends:
+// memory as pass2_group, each chunk's first forward value kept in the place of its input; natural ends:
 // the backward sweep writes each solution rounded as its coefficient; periodic: the solution of
 // point i goes to slot i+1 (i <= N-2; the last one stays in a register) for the correction sweep,
 // which writes the rounded coefficients.  Output [M0][M1][M2] floats.
@@ -578,12 +474,12 @@ __device__ __forceinline__ void pass2_group_f32(double* in, const SplineGrid& g,
         }
         __syncwarp();
     };
-    // staged values of points k (k < kmax) into slots k + off of their lines
-    auto store = [&](int k0, int off, int kmax) {
+    // staged solutions of points k < N - 1 into slots k + 1 of their lines
+    auto store = [&](int k0) {
         __syncwarp();
         for (int j = 0; j < nl; j++) {
             const int k = k0 + lane;
-            if (k < kmax) in[(L0 + j) * N + k + off] = sm[j][lane];
+            if (k < N - 1) in[(L0 + j) * N + k + 1] = sm[j][lane];
         }
         __syncwarp();
     };
@@ -597,6 +493,7 @@ __device__ __forceinline__ void pass2_group_f32(double* in, const SplineGrid& g,
         __syncwarp();
     };
     const double* src = in + myL * N;
+    double* line = in + myL * N;
     float* dst = out + myL * M;
     const int top = ((N - 1) / kLineChunk) * kLineChunk;
     double d_inf, r_inf;
@@ -606,13 +503,18 @@ __device__ __forceinline__ void pass2_group_f32(double* in, const SplineGrid& g,
         double rp = 0.0;
         for (int k0 = 0; k0 < N; k0 += kLineChunk) {
             load(k0);
-            if (mine) chunk_forward(sm[lane], k0, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
-            store(k0, 0, N);
+            if (mine) {
+                chunk_forward(sm[lane], k0, 1, N - 2, N, 0, tb, c0, cl, r_inf, rp);
+                if (k0 > 0) line[k0] = sm[lane][0];
+            }
+            __syncwarp();
         }
         double x = 0.0, x1 = 0.0, xl2 = 0.0;
         for (int k0 = top; k0 >= 0; k0 -= kLineChunk) {
             load(k0);
             if (mine) {
+                rp = sm[lane][0];
+                chunk_forward(sm[lane], k0, k0 > 0 ? k0 + 1 : 1, N - 2, N, 0, tb, c0, cl, r_inf, rp, k0 > 0);
                 chunk_back(sm[lane], k0, 1, N - 2, tb, d_inf, r_inf, x);
                 if (k0 <= N - 2 && N - 2 < k0 + kLineChunk) xl2 = sm[lane][N - 2 - k0];
                 x1 = x;
@@ -629,18 +531,23 @@ __device__ __forceinline__ void pass2_group_f32(double* in, const SplineGrid& g,
         double rp = 0.0;
         for (int k0 = 0; k0 < N; k0 += kLineChunk) {
             load(k0);
-            if (mine) chunk_forward(sm[lane], k0, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
-            store(k0, 0, N);
+            if (mine) {
+                chunk_forward(sm[lane], k0, 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp);
+                if (k0 > 0) line[k0] = sm[lane][0];
+            }
+            __syncwarp();
         }
         double x = 0.0, x0 = 0.0, xl = 0.0;
         for (int k0 = top; k0 >= 0; k0 -= kLineChunk) {
             load(k0);
             if (mine) {
+                rp = sm[lane][0];
+                chunk_forward(sm[lane], k0, k0 > 0 ? k0 + 1 : 0, N - 1, N, 1, tb, 0.0, 0.0, r_inf, rp, k0 > 0);
                 chunk_back(sm[lane], k0, 0, N - 1, tb, d_inf, r_inf, x);
                 if (k0 <= N - 1 && N - 1 < k0 + kLineChunk) xl = sm[lane][N - 1 - k0];
                 x0 = x;
             }
-            store(k0, 1, N - 1);
+            store(k0);
         }
         const double fac = mine ? __ddiv_rn(add(x0, mul(-0.25, xl)), tb.denom) : 0.0;
         double y0 = 0.0, y1 = 0.0;
