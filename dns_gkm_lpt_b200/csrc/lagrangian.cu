@@ -30,11 +30,12 @@ __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, 
 
 // One line: f (N points, stride fs) -> c (N+pad values, stride cs).
 // The recurrences are sequential, but their inputs are not: the loops fetch U inputs ahead (data
-// in the forward sweeps, the forward results in the backward sweeps) so that many loads are in
-// flight per thread; the arithmetic and its order are unchanged.  Measured: U = 8 for the
-// component-batched launches (fewer lines per component, more inputs in flight pay), U = 4 for
-// the one-component launches of large grids (their lines already fill the GPU).
-constexpr int kLineBatchBatched = 8, kLineBatchSingle = 4;
+// in the forward sweeps, those or the forward results in the backward sweeps) so that many loads are in
+// flight per thread; the arithmetic and its order are unchanged.  Pass 1 stores one forward value in U, so
+// longer batches pay there: of 8 / 16 / 24 points three components took 1.304 / 1.260 / 1.276 ms at 256^3, 8.89 /
+// 8.51 / 8.55 at 512^3; one component per launch (FP32 coefficients, 512^3) 4 and 4 points in passes 0
+// and 1 took 9.10 ms, 4 and 8 8.63, 4 and 16 8.67, 8 and 12 8.50.
+constexpr int kLineBatch0 = 8, kLineBatch1Batched = 16, kLineBatch1Single = 12;
 // the component-batched pass kernels hold six 128-thread CTAs per SM (80 registers): more lines
 // in flight than the compiler's own choice (96-112 registers; 256^3 splines 1.57 -> 1.49 ms),
 // where eight (64 registers) spill the fetch-ahead values
@@ -209,7 +210,7 @@ __global__ void spline_pass0(const double* __restrict__ W, FieldConst fc, Spline
 {
     const long long lines = (long long)g.npts * g.npts;
     for (long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x; L < lines; L += (long long)gridDim.x * blockDim.x)
-        pass0_line<kLineBatchSingle, VEL>(W, fc, g, tb, q, out, L);
+        pass0_line<kLineBatch0, VEL>(W, fc, g, tb, q, out, L);
 }
 
 // pass 1: [M0][N1][N2] along axis 1 -> [M0][M1][N2]; one line (a, k)
@@ -228,7 +229,7 @@ __global__ void spline_pass1(const double* __restrict__ in, SplineGrid g, Spline
 {
     const long long lines = (long long)(g.npts + g.pad) * g.npts;
     for (long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x; L < lines; L += (long long)gridDim.x * blockDim.x)
-        pass1_line<kLineBatchSingle>(in, g, tb, out, L);
+        pass1_line<kLineBatch1Single>(in, g, tb, out, L);
 }
 
 // pass 2: [M0][M1][N2] along axis 2 -> [M0][M1][M2].  Lines are contiguous,
@@ -437,7 +438,7 @@ __global__ void spline_pass0_room(const double* __restrict__ W, FieldConst fc, S
     const long long lines = (long long)g.npts * g.npts;
     const long long stride = (long long)(g.npts + g.pad) * g.npts;
     for (long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x; L < lines; L += (long long)gridDim.x * blockDim.x)
-        pass0_line<kLineBatchSingle, true>(W, fc, g, tb, q, out, L, stride);
+        pass0_line<kLineBatch0, true>(W, fc, g, tb, q, out, L, stride);
 }
 
 // pass 1 in place on [M0][M1][N2]: line (a, k) reads rows 0..N-1 and writes rows 0..M-1
@@ -449,7 +450,7 @@ __global__ void spline_pass1_inplace(double* buf, SplineGrid g, SplineTables tb)
         const int a = (int)(L / N), k = (int)(L - (long long)a * N);
         double* line = buf + (long long)a * M * N + k;
         auto f = [&](int i) { return line[(long long)i * N]; };
-        line_solve<kLineBatchSingle, true, true>(f, N, g.periodic, tb, line, N);
+        line_solve<kLineBatch1Single, true, true>(f, N, g.periodic, tb, line, N);
     }
 }
 
@@ -1521,7 +1522,7 @@ __global__ void __launch_bounds__(128, kPassCtasPerSm) ensemble_pass0_kernel(con
         const MemberDev& md = ensemble_group(mem, off, nm, w, 0, q, group);
         const long long L = group * 32 + lane;
         if (L < (long long)md.grid.npts * md.grid.npts)
-            pass0_line<kLineBatchBatched, true>(md.buf[buf], md.fc, md.grid, md.tb, q + 1, md.coef[q], L);
+            pass0_line<kLineBatch0, true>(md.buf[buf], md.fc, md.grid, md.tb, q + 1, md.coef[q], L);
     }
 }
 
@@ -1535,7 +1536,7 @@ __global__ void __launch_bounds__(128, kPassCtasPerSm) ensemble_pass1_kernel(con
         const MemberDev& md = ensemble_group(mem, off, nm, w, 1, q, group);
         const long long L = group * 32 + lane;
         if (L < (long long)(md.grid.npts + md.grid.pad) * md.grid.npts)
-            pass1_line<kLineBatchBatched>(md.coef[q], md.grid, md.tb, md.scratch[q], L);
+            pass1_line<kLineBatch1Batched>(md.coef[q], md.grid, md.tb, md.scratch[q], L);
     }
 }
 
