@@ -71,7 +71,7 @@ struct gkm_handle {
     double* pipe_dense = nullptr;       // odd grids: the pipeline's dense planes, 5 x nt^3 (on first use)
     cudaStream_t pipe_halo = nullptr;   // ghost wrap of each part as it lands, off the copy-in stream
     std::vector<cudaEvent_t> pipe_ev;
-    int pipe_chunk = 0;      // y-planes per chunk (multiple of 16); 0: about n/8
+    int pipe_chunk = 0;      // y-planes per chunk (multiple of 16); 0: 16
     // tensor maps of the two state buffers for the FP64 x / y sweeps' slab copies, in device
     // memory, index (buffer * kSweepVariants64 + variant) * 2 + direction; null when unavailable
     unsigned char* d_tmaps = nullptr;
