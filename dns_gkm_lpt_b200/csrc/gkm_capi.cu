@@ -90,9 +90,10 @@ void destroy_graphs(gkm_handle* h)
 {
     for (int k = 0; k < 3; k++)
         for (int p = 0; p < 2; p++) {
-            if (h->graph[k][p]) cudaGraphExecDestroy(h->graph[k][p]);
-            h->graph[k][p] = nullptr;
-            h->graph_np[k][p] = -1;
+            for (auto& g : h->graph[k][p]) {
+                if (g.exec) cudaGraphExecDestroy(g.exec);
+                g = gkm_handle::StepGraph{};
+            }
         }
 }
 
@@ -316,26 +317,39 @@ gkm::ParticleArrays arrays_of(double* const a[6])
     return gkm::ParticleArrays{{a[0], a[1], a[2], a[3], a[4], a[5]}};
 }
 
-// order the particles by spline-cell blocks (into the sorted copy), then Heun from the sorted
-// copy back into the particle arrays with the dt of the last Eulerian step
+// The particles' order is renewed every kOrderEvery steps: a step moves them by a fraction of a cell, the
+// blocks they are ordered by have 8 cells a side.  Below kOrderMin particles it gains less than its
+// launches cost.  Particle phase of a step, us, ordered every step / 4 / 16 / never: 32^3 with 1k 38 / 30 / 27 /
+// 29, 128^3 with 30k 67 / 48 / 43 / 43, with 100k 116 / 97 / 91 / 93, with 1M 609 / 495 / 466 / 712, 256^3 with 1M 666 /
+// 614 / 607 / 1964.
+constexpr int kOrderEvery = 16;
+constexpr int64_t kOrderMin = 50000;
+bool order_now(const gkm_handle* h) { return h->np >= kOrderMin && h->since_order == 0; }
+void count_order(gkm_handle* h) { h->since_order = (h->since_order + 1) % kOrderEvery; }
+
+// Heun with the dt of the last Eulerian step; where the order is due, the particles are first ordered by
+// spline-cell blocks into the sorted copy, and Heun writes them back from there
 cudaError_t enqueue_advect(gkm_handle* h)
 {
     if (h->np <= 0) return cudaSuccess;
-    int nl = 0;
-    cudaError_t e = gkm::launch_particle_sort(h->grid, h->np, arrays_of(h->P), arrays_of(h->P_sorted), h->tag,
-                                              h->tag_sorted, h->sort_keys, h->sort_counts, h->sort_temp, &nl,
-                                              h->stream);
-    h->launches += nl + 1;
-    if (e != cudaSuccess) return e;
+    const bool order = order_now(h);
+    if (order) {
+        int nl = 0;
+        cudaError_t e = gkm::launch_particle_sort(h->grid, h->np, arrays_of(h->P), arrays_of(h->P_sorted), h->tag,
+                                                  h->tag_sorted, h->sort_keys, h->sort_counts, h->sort_temp, &nl,
+                                                  h->stream);
+        h->launches += nl + 1;
+        if (e != cudaSuccess) return e;
+    }
     h->launches += 1;
+    const gkm::ParticleArrays from = arrays_of(order ? h->P_sorted : h->P), to = arrays_of(h->P);
+    const long long* tag_from = order ? h->tag_sorted : nullptr;
     if (h->spline_f32) {
         const float* c32[3] = {h->coef32[0], h->coef32[1], h->coef32[2]};
-        return gkm::launch_particles_heun(c32, h->grid, h->clock, h->np, arrays_of(h->P_sorted), arrays_of(h->P),
-                                          h->tag_sorted, h->tag, h->stream);
+        return gkm::launch_particles_heun(c32, h->grid, h->clock, h->np, from, to, tag_from, h->tag, h->stream);
     }
     const double* c[3] = {h->coef[0], h->coef[1], h->coef[2]};
-    return gkm::launch_particles_heun(c, h->grid, h->clock, h->np, arrays_of(h->P_sorted), arrays_of(h->P),
-                                      h->tag_sorted, h->tag, h->stream);
+    return gkm::launch_particles_heun(c, h->grid, h->clock, h->np, from, to, tag_from, h->tag, h->stream);
 }
 
 // splines of the state W and Heun advection with the dt of the last Eulerian step
@@ -375,30 +389,32 @@ gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
     for (int s = 0; s < nsteps; s++) {
         const int p = h->parity;
         if (h->cfg.use_graphs) {
-            if (!h->graph[kind][p] || h->graph_np[kind][p] != h->np) {
-                if (h->graph[kind][p]) cudaGraphExecDestroy(h->graph[kind][p]);
-                h->graph[kind][p] = nullptr;
+            gkm_handle::StepGraph& step = h->graph[kind][p][kind != kGraphEulerian && order_now(h)];
+            if (!step.exec || step.np != h->np) {
+                if (step.exec) cudaGraphExecDestroy(step.exec);
+                step.exec = nullptr;
                 cudaGraph_t g = nullptr;
                 const int64_t before = h->launches;
                 CK(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
                 cudaError_t e = enqueue_kind(h, kind);
                 cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
-                h->graph_kernels[kind][p] = h->launches - before;
+                step.kernels = h->launches - before;
                 h->launches = before;   // counted when the graph is replayed
                 if (e != cudaSuccess) return cuda_fail(h, e, "capture step");
                 if (e2 != cudaSuccess) return cuda_fail(h, e2, "cudaStreamEndCapture");
-                e = cudaGraphInstantiate(&h->graph[kind][p], g, 0);
+                e = cudaGraphInstantiate(&step.exec, g, 0);
                 cudaGraphDestroy(g);
                 if (e != cudaSuccess) return cuda_fail(h, e, "cudaGraphInstantiate");
-                h->graph_np[kind][p] = h->np;
+                step.np = h->np;
             }
-            CK(h, cudaGraphLaunch(h->graph[kind][p], h->stream));
-            h->launches += h->graph_kernels[kind][p];
+            CK(h, cudaGraphLaunch(step.exec, h->stream));
+            h->launches += step.kernels;
         } else {
             cudaError_t e = enqueue_kind(h, kind);
             if (e != cudaSuccess) return cuda_fail(h, e, "step launch");
         }
         if (kind != kGraphParticles) h->parity ^= 1;
+        if (kind != kGraphEulerian) count_order(h);
         // the particle path leaves the splines of the current state built
         h->splines_valid = (kind != kGraphEulerian && h->np > 0);
     }
@@ -867,6 +883,7 @@ gkm_status gkm_step_timed(gkm_handle* h, int32_t nsteps, int32_t with_particles,
         cudaEventElapsedTime(&t, ev[0], ev[6]);
         ms[6] += t;
         h->splines_valid = parts;
+        if (parts) count_order(h);
     }
     for (int k = 0; k < 7; k++) cudaEventDestroy(ev[k]);
     return st;
@@ -1270,6 +1287,7 @@ gkm_status gkm_particles_upload(gkm_handle* h, int64_t np, const double* pos, co
         CK(h, cudaStreamSynchronize(h->stream));   // the caller's arrays have been read
     }
     h->np = np;
+    h->since_order = 0;
     if (!U && np > 0) {
         if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "U == NULL needs an uploaded state");
         gkm_status s = ensure_splines(h);

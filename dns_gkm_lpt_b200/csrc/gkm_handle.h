@@ -57,9 +57,12 @@ struct gkm_handle {
     double* props = nullptr;         // [cap][kPropCount] particle properties, in upload order
     gkm::StatsPartial* partials = nullptr;
     double* stats_out = nullptr;
-    cudaGraphExec_t graph[3][2] = {{nullptr, nullptr}, {nullptr, nullptr}, {nullptr, nullptr}};
-    int64_t graph_np[3][2] = {{-1, -1}, {-1, -1}, {-1, -1}};
-    int64_t graph_kernels[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        int64_t np = -1, kernels = 0;
+    };
+    StepGraph graph[3][2][2];   // [kind][parity][the particles are ordered first]
+    int since_order = 0;        // particle steps since they were ordered last (0: order them now)
     int64_t launches = 0;    // kernels launched (graph replays add the kernels they hold)
     // plug-point pipeline (gkm_evolve with pinned or device buffers): copy-in, copy-out and
     // two compute streams, and per-chunk events, created on first use
