@@ -56,6 +56,9 @@ REF_PART = N_PART * REF_N ** 3 // N_CELLS ** 3   # same particle density
 C3_PART = 4_000_000          # particles of the 512^3 mixed-precision case
 HBM_FALLBACK_GBS = 6650.0    # an earlier copy-bandwidth measurement on these B200s, used only without a
                              # measured-peaks file beside this script
+# FP64 instructions the three sweeps execute per cell update (ncu smsp__inst_executed_pipe_fp64 at 192^3, 16 x 8
+# windows: 375.3 M, 376.4 M and 384.7 M warp instructions)
+FP64_INSTR_PER_CELL_UPDATE = 5137
 # DRAM bytes per cell of one sweep launch: mean over the x, y, z sweeps of the ncu capture of this
 # benchmark's 256^3 cube (83.8, 123.3, 141.4 B; compulsory 80, 120, 120)
 SWEEP_DRAM_BYTES_PER_CELL = 116.2
@@ -708,6 +711,8 @@ def ours(args, rank: int, world: int, local_rank: int):
             "roofline": {"kernel": "sweep_kernel (x/y/z, one launch each per step)", "bound": "fp32" if prec else "fp64",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "traffic": traffic if not prec else None, "flops_per_cell_update": flops_cell,
+                         # the numerator is the reference's formulation; what the FP64 sweeps execute, in FMA slots
+                         "executed_frac": None if prec else FP64_INSTR_PER_CELL_UPDATE * 2 * cells / 3 / launch_s / 1e12 / peak,
                          "peak_source": "FMA probe run by this bench (gkm_probe_fma_peak)",
                          "hbm": {"achieved_gbs": bytes_launch / launch_s / 1e9, "peak_gbs": hbm_gbs,
                                  "frac": bytes_launch / launch_s / 1e9 / hbm_gbs, "peak_source": hbm_src}},

@@ -80,8 +80,8 @@ __device__ __forceinline__ void fixed_pivots(int N, const SplineTables& tb, doub
 // i + 1, so c may be the storage f reads (same stride) as long as slots N .. N+pad-1 exist.
 // REREAD: the forward sweep stores one value in U, and the backward sweep forms the others again
 // from the inputs: the line is read twice and written once instead of twice.  For inputs that cost
-// no more than their load (pass 1: DRAM writes weigh more than reads; three components at 256^3, all passes, 1.44 -> 1.31 ms, at 512^3 9.99 -> 8.90);
-// pass 0's cost a division each.
+// no more than their load: with passes 1 and 2 so, all passes of three components went 1.44 -> 1.31 ms at
+// 256^3, 9.99 -> 8.90 at 512^3.  Pass 0's inputs cost a division each (1.31 -> 1.40 ms).
 template <int U, bool IN_PLACE, bool REREAD, class Src>
 __device__ void line_solve(const Src& f, int N, int periodic, const SplineTables& tb, double* c, long long cs)
 {
@@ -593,9 +593,9 @@ __global__ void __launch_bounds__(32 * kPass2Warps) spline_pass2_f32(double* in,
 // through global memory instead, and their loads wait on one another 4 or 8 at a time.  What
 // remains is the lanes' serial chain, which pivot_quotient keeps short.
 // How many warps of such lines an SM holds decides where it pays.  Velocity splines, ms, streaming
-// kernels against these: three components per launch 64^3 0.099 -> 0.048, 128^3 0.270 -> 0.157, 160^3 0.390 ->
-// 0.338, 192^3 0.817 -> 0.640, 224^3 1.08 -> 1.16, 256^3 1.42 -> 1.65; one component per launch (coefficients in
-// FP32) 128^3 0.511 -> 0.198, 224^3 1.28 -> 1.09, 256^3 1.65 -> 1.50, 282^3 1.80 -> 1.90.
+// kernels against these: three components per launch 64^3 0.099 -> 0.048, 128^3 0.270 -> 0.157, 160^3 0.371 ->
+// 0.334, 192^3 0.763 -> 0.631, 224^3 0.99 -> 1.16, 256^3 1.26 -> 1.65; one component per launch (coefficients in
+// FP32) 128^3 0.511 -> 0.198, 200^3 0.99 -> 0.76, 224^3 1.25 -> 1.09, 256^3 1.58 -> 1.50, 282^3 1.80 -> 1.90.
 constexpr int kResidentBatched = 200, kResidentSingle = 264;
 constexpr int kTableRows = kPivotRows + 2;   // rows of the tables a warp keeps beside its lines
 inline size_t resident_bytes(int npts) { return sizeof(double) * (2 * kTableRows + 32 * (size_t)(npts | 1)); }
@@ -1315,7 +1315,8 @@ __global__ void scan_add_kernel(unsigned* __restrict__ data, long long n, const 
 // (the sorted copy's, free between steps): element e of it lies in array e / np.  Export: slot p's
 // triple (positions or velocities) to its upload index; import: the triples into the particle arrays,
 // tags in order.  Scattered 24-byte stores, bound by their sectors; the host then copies whole arrays.
-// With the reordering on the host, one step of 1M particles from upload to download took 37 ms, now 8.7 (0.5 less from the solves).
+// With the reordering on the host, a step of 1M particles and their download took 37 ms, then 8.7 (0.5 of it
+// from the spline solves).
 struct Triple {
     double* a[3];
 };

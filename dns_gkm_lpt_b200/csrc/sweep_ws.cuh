@@ -22,10 +22,10 @@
 // warpgroup to 104 and the consumer warpgroups to 200, which the launch's 64,512
 // registers cover exactly, so the host launches this kernel only when it was
 // compiled to 168 registers (ws_ready()).  Every wait is bounded; one that runs
-// out raises bit 1 of the clock's status word.  Measured at 256^3: x and y
-// sweeps 4.5 % and 3 % faster than the plain 16 x 16 sweep; the z sweep, whose
-// producer moves each slab with per-element cp.async, 16 % slower (the
-// autotuner keeps the plain kernel there).
+// out raises bit 1 of the clock's status word.  Measured, ms per sweep: at 256^3 x 2.51 and y
+// 2.58 against 2.62 and 2.68 of the plain 16 x 16 sweep and 2.52 and 2.59 of the 16 x 8 one; in one round of
+// CTAs, at 96^3, x 0.148 against 0.157 and 0.159.  The z sweep's producer moves each slab with
+// per-element cp.async: 3.44 against 3.02 and 2.97.
 #pragma once
 
 #include "sweep_impl.cuh"
@@ -36,8 +36,9 @@ namespace sweep_ws_detail {
 constexpr int kConsumers = 256;             // 16 x 16 faces, one per consumer thread
 constexpr int kProducers = 128;             // one warpgroup
 constexpr int kThreads = kConsumers + kProducers;
-// 2 x 128 x 200 + 128 x 104 = 384 x 168.  Measured at 256^3 (x / y sweep, ms): 216 / 72 4.75 / 4.75,
-// 208 / 88 4.57 / 4.67, 200 / 104 4.34 / 4.50, 192 / 120 5.75 / 6.20; the plain 16 x 16 sweep 4.55 / 4.65
+// 2 x 128 x 200 + 128 x 104 = 384 x 168.  Chosen with the longer flux code this kernel had first (256^3, x / y, ms:
+// 216 / 72 4.75 / 4.75, 208 / 88 4.57 / 4.67, 200 / 104 4.34 / 4.50, 192 / 120 5.75 / 6.20); with the present one 192 / 120
+// and 184 / 136 stay within 2 % of it
 constexpr int kConsumerRegs = 200, kProducerRegs = 104;
 static_assert(2 * 128 * kConsumerRegs + 128 * kProducerRegs <= kThreads * 168, "register split above the launch's");
 

@@ -134,7 +134,7 @@ class Solver:
         return out
 
     def device_state(self):
-        """The current state in device memory as a CUDA tensor view (5, nt, nt, nt), no copy
+        """The current state in device memory as a CUDA tensor view (5, nt, nt, nt), no copy for even n
         (gkm_device_state); valid until the next step, which writes the other buffer."""
         import torch
 
