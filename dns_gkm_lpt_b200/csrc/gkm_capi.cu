@@ -773,6 +773,10 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
     }
     h->launches += 1;
     CK(h, gkm::launch_halo(dst, h->fc, h->clock, 0, h->parity, 0, 0.0, h->stream));
+    if (h->view_live) {   // the view is the state until the next step: its ghosts are wrapped too
+        CK(h, gkm::launch_rows_compact(dst, h->view, h->fc, h->stream));
+        h->launches += 1;
+    }
     CK(h, cudaMemsetAsync(&h->clock->status, 0, sizeof(int), h->stream));
     gkm_status s = reduce_wave(h);
     if (s != GKM_OK) return s;
