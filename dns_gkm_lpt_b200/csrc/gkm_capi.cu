@@ -607,9 +607,14 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     fc.inv_m_s = 1.0 / (P.den0 * fc.u_s);
     fc.inv_E_s = 1.0 / P.p0;
     fc.inv_T0 = 1.0 / fc.T0;
-    fc.eps_rho = 1e-10 * fc.inv_rho_s * fc.inv_rho_s;
-    fc.eps_m = 1e-10 * fc.inv_m_s * fc.inv_m_s;
-    fc.eps_T = 1e-10 * fc.inv_T0 * fc.inv_T0;
+    // The WENO epsilons there, within [2^-64, 2^40]: the single-precision weights multiply two indicators 4 (eps + IS),
+    // and 4 eps squared has to stay a normal number at both ends.  Beyond them eps decides nothing that
+    // single precision holds: differences of 2^-32 lie far below the rounding of values of order one, and an
+    // eps of 2^40 leaves linear weights.  (Unbounded, flat stencils gave 0/0 from den0 p0 = 3.7e9 or T0 = 6.1e4 K on.)
+    auto eps_in = [](double inv_scale) { return std::min(std::max(1e-10 * inv_scale * inv_scale, 0x1p-64), 0x1p40); };
+    fc.eps_rho = eps_in(fc.inv_rho_s);
+    fc.eps_m = eps_in(fc.inv_m_s);
+    fc.eps_T = eps_in(fc.inv_T0);
     fc.fscale[0] = P.den0 * fc.dx;
     fc.fscale[1] = fc.fscale[2] = fc.fscale[3] = P.den0 * fc.u_s * fc.dx;
     fc.fscale[4] = P.p0 * fc.dx;

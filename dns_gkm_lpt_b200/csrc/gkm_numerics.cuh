@@ -239,7 +239,7 @@ GKM_HD void weno_scalar(T a3, T a2, T a1, T b1, T b2, T b3, T eps, T& fl, T& fr)
     if constexpr (single_t<T>::value) {
         // single precision: products of three (eps + IS) underflow on flat stencils, so the
         // candidates 2 and 3 enter with the ratio (IS_0 IS_1) / (IS_2 IS_3), at most IS_0 / IS_2
-        // because IS_3 is the largest
+        // because IS_3 is the largest; eps is such that a product of two is a normal number
         const WenoParts<T> w = weno_parts<T>(a3, a2, a1, b1, b2, b3, eps);
         const T n = T(9), c16 = T(1.0 / 6.0);
         {
