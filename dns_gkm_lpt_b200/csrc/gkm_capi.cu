@@ -464,7 +464,7 @@ gkm_status upload_triples(gkm_handle* h, int64_t np, const double* in, double* c
 {
     for (int k = 0; k < 3; k++)
         CK(h, cudaMemcpyAsync(s[k], in + (size_t)k * np, sizeof(double) * (size_t)np, cudaMemcpyHostToDevice, h->stream));
-    CK(h, gkm::launch_particle_import(np, s, a, tag, h->stream));
+    CK(h, gkm::launch_particle_import(np, s, a, tag, h->clock, h->stream));
     h->launches += 1;
     return GKM_OK;
 }
@@ -1299,6 +1299,9 @@ gkm_status gkm_particles_upload(gkm_handle* h, int64_t np, const double* pos, co
         if (s == GKM_OK && U) s = upload_triples(h, np, U, h->P_sorted + 3, h->P + 3, nullptr);
         if (s != GKM_OK) return s;
         CK(h, cudaStreamSynchronize(h->stream));   // the caller's arrays have been read
+    } else {
+        CK(h, gkm::launch_particle_import(0, h->P_sorted, h->P, h->tag, h->clock, h->stream));
+        h->launches += 1;
     }
     h->np = np;
     h->since_order = 0;

@@ -220,11 +220,11 @@ cudaError_t launch_particle_props(const double* const coefs[8], const SplineGrid
                                   const double* px, const double* pz, const long long* tag, double* props,
                                   DevClock* clock, cudaStream_t s);
 // np x 3 host values through three device arrays of np (value e of them in array e / np): the particle
-// arrays' triples in upload order, and back with fresh tags (tag may be null)
+// arrays' triples in upload order, and back with fresh tags, which clear kStatusTags (tag may be null)
 cudaError_t launch_particle_export(long long np, const long long* tag, double* const src[3], double* const dst[3],
                                    DevClock* clock, cudaStream_t s);
 cudaError_t launch_particle_import(long long np, double* const src[3], double* const dst[3], long long* tag,
-                                   cudaStream_t s);
+                                   DevClock* clock, cudaStream_t s);
 cudaError_t launch_particle_stats(const double* props, long long np, StatsPartial* partials, int nblocks, double* out6,
                                   cudaStream_t s);
 cudaError_t launch_stats(const double* W, const FieldConst& fc, const SplineGrid& g, const double* const coefs[3],

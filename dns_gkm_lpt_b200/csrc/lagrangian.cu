@@ -1338,8 +1338,10 @@ __global__ void particle_export_kernel(long long np, const long long* __restrict
         for (int c = 0; c < 3; c++) triple_at(dst, np, 3 * t + c) = src.a[c][p];
     }
 }
-__global__ void particle_import_kernel(long long np, Triple src, Triple dst, long long* __restrict__ tag)
+// With tags, a report of damaged ones ends: these are new.
+__global__ void particle_import_kernel(long long np, Triple src, Triple dst, long long* __restrict__ tag, DevClock* clock)
 {
+    if (tag && blockIdx.x == 0 && threadIdx.x == 0) atomicAnd(&clock->status, ~kStatusTags);
     for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < np; p += (long long)gridDim.x * blockDim.x) {
 #pragma unroll
         for (int c = 0; c < 3; c++) dst.a[c][p] = triple_at(src, np, 3 * p + c);
@@ -1720,11 +1722,10 @@ cudaError_t launch_particle_export(long long np, const long long* tag, double* c
 }
 
 cudaError_t launch_particle_import(long long np, double* const src[3], double* const dst[3], long long* tag,
-                                   cudaStream_t s)
+                                   DevClock* clock, cudaStream_t s)
 {
-    if (np <= 0) return cudaSuccess;
     return grid_launch(particle_import_kernel, np, 256, s, np, Triple{{src[0], src[1], src[2]}},
-                       Triple{{dst[0], dst[1], dst[2]}}, tag);
+                       Triple{{dst[0], dst[1], dst[2]}}, tag, clock);
 }
 
 cudaError_t launch_particle_props(const double* const coefs[8], const SplineGrid& g, long long np, const double* py,
