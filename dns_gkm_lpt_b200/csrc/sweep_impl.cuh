@@ -93,7 +93,7 @@ __device__ __forceinline__ double collision_time(const FieldConst& fc, double T,
 
 // |u| + c of a conserved state in FP64: its square |u|^2 + c^2 + 2 |u| c with one reciprocal of rho and
 // one inverse root (the z sweeps' reduction for the next step's dt, whose square root is taken
-// once per thread: within an ulp or two of the reference's; NaN where p < 0), and with the
+// once per thread: within 3 ulp of the reference's, 0.6 of 2^-53 on average; NaN where p < 0), and with the
 // reference's divisions and roots (src/update.cpp:1039-1046 via c2p; the stand-alone timestep,
 // whose dt equals the reference's bit for bit).
 __device__ __forceinline__ double wave_speed_sq(const double w[5], double gam, double gm1)
