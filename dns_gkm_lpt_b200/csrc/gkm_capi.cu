@@ -512,13 +512,11 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 {
     *dense = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
-    if (h->view_live) {
-        *dense = h->view;
-        return GKM_OK;
-    }
     double* out = h->buf[h->parity ^ 1];
-    CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->stream));
-    h->launches += 1;
+    if (!h->view_live) {
+        CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->stream));
+        h->launches += 1;
+    }
     *dense = out;
     return GKM_OK;
 }
@@ -526,7 +524,7 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 gkm_status gkm_host::take_view(gkm_handle* h)
 {
     if (!h->view_live) return GKM_OK;
-    CK(h, gkm::launch_rows_expand(h->view, h->buf[h->parity], h->fc, h->stream));
+    CK(h, gkm::launch_rows_expand(h->buf[h->parity ^ 1], h->buf[h->parity], h->fc, h->stream));
     h->launches += 1;
     return GKM_OK;
 }
@@ -749,7 +747,6 @@ gkm_status gkm_destroy(gkm_handle* h)
     cudaFree(h->lap_nodes);
     cudaFree(h->props);
     cudaFree(h->pipe_dense);
-    cudaFree(h->view);
     for (cudaEvent_t e : h->pipe_ev) cudaEventDestroy(e);
     for (cudaStream_t s : {h->pipe_in, h->pipe_out, h->pipe_comp[0], h->pipe_comp[1], h->pipe_comp[2], h->pipe_comp[3],
                            h->pipe_halo})
@@ -768,8 +765,8 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
         if (!W[q]) return fail(h, GKM_ERR_ARG, "W[q] is NULL");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
     double* dst = h->buf[h->parity];
-    // odd grids: dense rows through the view or the accumulator buffer, free between steps, then to their pitch
-    double* land = h->fc.pitch == h->fc.nt ? dst : (h->view_live ? h->view : h->buf[h->parity ^ 1]);
+    // odd grids: dense rows through the accumulator buffer, free between steps, then to their pitch
+    double* land = h->fc.pitch == h->fc.nt ? dst : h->buf[h->parity ^ 1];
     for (int q = 0; q < 5; q++)
         CK(h, cudaMemcpyAsync(land + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
     if (land != dst) {
@@ -779,7 +776,7 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
     h->launches += 1;
     CK(h, gkm::launch_halo(dst, h->fc, h->clock, 0, h->parity, 0, 0.0, h->stream));
     if (h->view_live) {   // the view is the state until the next step: its ghosts are wrapped too
-        CK(h, gkm::launch_rows_compact(dst, h->view, h->fc, h->stream));
+        CK(h, gkm::launch_rows_compact(dst, land, h->fc, h->stream));
         h->launches += 1;
     }
     CK(h, cudaMemsetAsync(&h->clock->status, 0, sizeof(int), h->stream));
@@ -908,8 +905,8 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     }
     const bool mixed = h->cfg.precision == GKM_PREC_MIXED;
     const int nvar = mixed ? gkm::kSweepVariants32 : gkm::kSweepVariants64;
-    // the sweeps leave W untouched (they write the accumulator A only); the clock
-    // they also touch is saved here and put back afterwards
+    // the sweeps leave W untouched (they write the accumulator A only, a live view of an odd grid with it); the
+    // clock they also touch is saved here and put back afterwards
     DevClock saved;
     CK(h, cudaMemcpyAsync(&saved, h->clock, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -967,6 +964,10 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     h->sweep_chosen = true;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (h->view_live) {   // the sweeps have written over it
+        gkm::launch_rows_compact(h->buf[h->parity], h->buf[h->parity ^ 1], h->fc, h->stream);
+        h->launches += 1;
+    }
     cudaMemcpyAsync(h->clock, &saved, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream);
     cudaStreamSynchronize(h->stream);
     destroy_graphs(h);
@@ -1110,6 +1111,7 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
     cudaEvent_t* ev_cp = &h->pipe_ev[2 + 2 * K];   // copy of part c landed
     double* Wd = h->buf[h->parity];
     double* A = h->buf[h->parity ^ 1];
+    h->view_live = false;
     DevClock* ck = h->clock;
     const bool mixed = h->cfg.precision == GKM_PREC_MIXED;
 
@@ -1224,7 +1226,6 @@ gkm_status evolve_pipelined(gkm_handle* h, double* const W[5], double dt)
     CK(h, copy_out(n + 3, n + 6, h->stream));
     CK(h, cudaStreamWaitEvent(h->stream, ev_done_out, 0));
     h->parity ^= 1;
-    h->view_live = false;
     h->state_loaded = true;
     h->splines_valid = false;
     DevClock c;
@@ -1262,8 +1263,8 @@ gkm_status gkm_evolve(gkm_handle* h, double* const W[5], double dt)
     const double val = h->dt_fixed;
     h->dt_fixed_mode = 1;
     h->dt_fixed = dt;
-    cudaError_t e = enqueue_eulerian(h);
     h->view_live = false;
+    cudaError_t e = enqueue_eulerian(h);
     h->dt_fixed_mode = mode;
     h->dt_fixed = val;
     if (e != cudaSuccess) return cuda_fail(h, e, "evolve");
@@ -1481,17 +1482,17 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
     if (!h || !W) return GKM_ERR_ARG;
     *W = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
-    if (!h->view) CK(h, cudaMalloc(&h->view, sizeof(double) * 5 * (size_t)h->fc.nt3));
+    const double* view = nullptr;
+    gkm_status s = gkm_host::dense_state(h, &view);
+    if (s != GKM_OK) return s;
     if (!h->view_live) {
-        CK(h, gkm::launch_rows_compact(*W, h->view, h->fc, h->stream));
-        h->launches += 1;
         // the caller may read it on any stream, as it may the state of an idle handle
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         CK(h, cudaStreamIsCapturing(h->stream, &capture));
         if (capture == cudaStreamCaptureStatusNone) CK(h, cudaStreamSynchronize(h->stream));
         h->view_live = true;
     }
-    *W = h->view;
+    *W = h->buf[h->parity ^ 1];
     return GKM_OK;
 }
 

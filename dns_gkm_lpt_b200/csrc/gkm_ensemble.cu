@@ -445,6 +445,13 @@ gkm_status gkm_ensemble_autotune(gkm_ensemble* E, int32_t reps)
         if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
         return e == cudaSuccess ? GKM_OK : ecuda(E, e, "gkm_ensemble_autotune");
     };
+    // live views of odd members lie in the accumulators: taken in by the first refresh, handed back below
+    std::vector<gkm_handle*> views;
+    for (gkm_handle* h : E->mem)
+        if (h->view_live) {
+            views.push_back(h);
+            h->view_live = false;
+        }
     for (int d = 0; d < 3 && st == GKM_OK; d++) {
         // 1. the window variant, with one segment length for every member
         int best_v = E->sweep[d].variant, best_L = E->sweep[d].seg_len;
@@ -488,6 +495,10 @@ gkm_status gkm_ensemble_autotune(gkm_ensemble* E, int32_t reps)
         }
     }
     E->launches = launches0;   // tuning launches are not steps
+    for (gkm_handle* h : views) {
+        gkm::launch_rows_compact(h->buf[p], h->buf[p ^ 1], h->fc, E->stream);
+        h->view_live = true;
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     for (int m = 0; m < nm; m++)
