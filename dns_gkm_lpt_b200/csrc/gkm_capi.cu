@@ -386,6 +386,9 @@ gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
         if (s != GKM_OK) return s;
         if (kind != kGraphParticles) h->view_live = false;
     }
+    // steps recorded into the caller's own graph order their particles each: a replay does not count steps
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!h->cfg.use_graphs && cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
     for (int s = 0; s < nsteps; s++) {
         const int p = h->parity;
         if (h->cfg.use_graphs) {
@@ -410,6 +413,7 @@ gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
             CK(h, cudaGraphLaunch(step.exec, h->stream));
             h->launches += step.kernels;
         } else {
+            if (capture != cudaStreamCaptureStatusNone) h->since_order = 0;
             cudaError_t e = enqueue_kind(h, kind);
             if (e != cudaSuccess) return cuda_fail(h, e, "step launch");
         }
