@@ -376,6 +376,14 @@ cudaError_t enqueue_kind(gkm_handle* h, int kind)
     return enqueue_eulerian(h);
 }
 
+// whether the caller records the handle's stream into a graph
+bool recording(gkm_handle* h)
+{
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (h->stream != h->own_stream && cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
+    return capture != cudaStreamCaptureStatusNone;
+}
+
 gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
 {
     if (!h) return GKM_ERR_ARG;
@@ -384,11 +392,11 @@ gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
     if (nsteps > 0) {
         gkm_status s = gkm_host::take_view(h);
         if (s != GKM_OK) return s;
-        if (kind != kGraphParticles) h->view_live = false;
     }
-    // steps recorded into the caller's own graph order their particles each: a replay does not count steps
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (!h->cfg.use_graphs && cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
+    // Steps recorded into the caller's own graph order their particles each, as a replay does not count steps, and
+    // leave a view as it is: their replays find out whether it still is the state.
+    const bool rec = !h->cfg.use_graphs && recording(h);
+    if (nsteps > 0 && kind != kGraphParticles && !rec) h->view_live = false;
     for (int s = 0; s < nsteps; s++) {
         const int p = h->parity;
         if (h->cfg.use_graphs) {
@@ -413,7 +421,7 @@ gkm_status run_steps(gkm_handle* h, int32_t nsteps, int kind)
             CK(h, cudaGraphLaunch(step.exec, h->stream));
             h->launches += step.kernels;
         } else {
-            if (capture != cudaStreamCaptureStatusNone) h->since_order = 0;
+            if (rec) h->since_order = 0;
             cudaError_t e = enqueue_kind(h, kind);
             if (e != cudaSuccess) return cuda_fail(h, e, "step launch");
         }
@@ -517,10 +525,8 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
     *dense = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
     double* out = h->buf[h->parity ^ 1];
-    if (!h->view_live) {
-        CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->stream));
-        h->launches += 1;
-    }
+    CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->view_live ? h->clock : nullptr, h->stream));
+    h->launches += 1;
     *dense = out;
     return GKM_OK;
 }
@@ -528,7 +534,7 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 gkm_status gkm_host::take_view(gkm_handle* h)
 {
     if (!h->view_live) return GKM_OK;
-    CK(h, gkm::launch_rows_expand(h->buf[h->parity ^ 1], h->buf[h->parity], h->fc, h->stream));
+    CK(h, gkm::launch_rows_expand(h->buf[h->parity ^ 1], h->buf[h->parity], h->fc, h->clock, h->stream));
     h->launches += 1;
     return GKM_OK;
 }
@@ -774,13 +780,13 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
     for (int q = 0; q < 5; q++)
         CK(h, cudaMemcpyAsync(land + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
     if (land != dst) {
-        CK(h, gkm::launch_rows_expand(land, dst, h->fc, h->stream));
+        CK(h, gkm::launch_rows_expand(land, dst, h->fc, nullptr, h->stream));
         h->launches += 1;
     }
     h->launches += 1;
     CK(h, gkm::launch_halo(dst, h->fc, h->clock, 0, h->parity, 0, 0.0, h->stream));
     if (h->view_live) {   // the view is the state until the next step: its ghosts are wrapped too
-        CK(h, gkm::launch_rows_compact(dst, land, h->fc, h->stream));
+        CK(h, gkm::launch_rows_compact(dst, land, h->fc, nullptr, h->stream));
         h->launches += 1;
     }
     CK(h, cudaMemsetAsync(&h->clock->status, 0, sizeof(int), h->stream));
@@ -969,7 +975,7 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (h->view_live) {   // the sweeps have written over it
-        gkm::launch_rows_compact(h->buf[h->parity], h->buf[h->parity ^ 1], h->fc, h->stream);
+        gkm::launch_rows_compact(h->buf[h->parity], h->buf[h->parity ^ 1], h->fc, nullptr, h->stream);
         h->launches += 1;
     }
     cudaMemcpyAsync(h->clock, &saved, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream);
@@ -1486,16 +1492,19 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
     if (!h || !W) return GKM_ERR_ARG;
     *W = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
-    const double* view = nullptr;
-    gkm_status s = gkm_host::dense_state(h, &view);
-    if (s != GKM_OK) return s;
-    if (!h->view_live) {
-        // the caller may read it on any stream, as it may the state of an idle handle
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        CK(h, cudaStreamIsCapturing(h->stream, &capture));
-        if (capture == cudaStreamCaptureStatusNone) CK(h, cudaStreamSynchronize(h->stream));
-        h->view_live = true;
-    }
+    // The caller may read it on any stream, as it may the state of an idle handle: done when the call returns,
+    // also while the caller records h->stream.
+    const bool rec = recording(h);
+    cudaStream_t s = rec ? h->own_stream : h->stream;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
+    cudaError_t e = gkm::launch_rows_compact(*W, h->buf[h->parity ^ 1], h->fc, h->view_live ? h->clock : nullptr, s);
+    if (e == cudaSuccess) e = gkm::launch_view_mark(h->clock, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
+    CK(h, e);
+    h->launches += 2;
+    h->view_live = true;
     *W = h->buf[h->parity ^ 1];
     return GKM_OK;
 }

@@ -69,7 +69,7 @@ struct gkm_handle {
     cudaStream_t pipe_in = nullptr, pipe_out = nullptr, pipe_comp[4] = {nullptr, nullptr, nullptr, nullptr};
     // odd grids: gkm_device_state has handed out a dense state, which lies in the accumulator buffer.  From
     // that call to the next step it is the state: callers may write to it, and every use of the state takes
-    // it in first.
+    // it in first.  The device knows whether a step has come since (DevClock::view).
     bool view_live = false;
     double* pipe_dense = nullptr;       // odd grids: the pipeline's dense planes, 5 x nt^3 (on first use)
     cudaStream_t pipe_halo = nullptr;   // ghost wrap of each part as it lands, off the copy-in stream

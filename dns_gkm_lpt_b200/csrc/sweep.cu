@@ -69,10 +69,14 @@ __global__ void halo_planes_kernel(double* W, FieldConst fc, int J0, int J1, con
     }
 }
 
+__global__ void view_mark_kernel(DevClock* clock) { clock->view = clock->iter + 1; }
+
 // rows of odd grids between the pitched layout and dense staging: a warp per row, bound by memory
 template <bool EXPAND>
-__global__ void rows_kernel(const double* __restrict__ src, double* __restrict__ dst, long long rows, int nt, int pitch)
+__global__ void rows_kernel(const double* __restrict__ src, double* __restrict__ dst, long long rows, int nt, int pitch,
+                            const DevClock* view)
 {
+    if (view && (view->view == view->iter + 1) != EXPAND) return;
     const int lane = threadIdx.x & 31;
     for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows;
          r += ((long long)gridDim.x * blockDim.x) >> 5) {
@@ -347,21 +351,26 @@ cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, 
 }
 
 template <bool EXPAND>
-static cudaError_t rows_t(const double* src, double* dst, const FieldConst& fc, cudaStream_t s)
+static cudaError_t rows_t(const double* src, double* dst, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
     const long long rows = 5LL * fc.nt * fc.nt;   // the components follow one another in both layouts
     long long blocks = (rows + 7) / 8;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    rows_kernel<EXPAND><<<(unsigned)blocks, 256, 0, s>>>(src, dst, rows, fc.nt, fc.pitch);
+    rows_kernel<EXPAND><<<(unsigned)blocks, 256, 0, s>>>(src, dst, rows, fc.nt, fc.pitch, view);
     return cudaGetLastError();
 }
-cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, cudaStream_t s)
+cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
-    return rows_t<true>(dense, W, fc, s);
+    return rows_t<true>(dense, W, fc, view, s);
 }
-cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, cudaStream_t s)
+cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
-    return rows_t<false>(W, dense, fc, s);
+    return rows_t<false>(W, dense, fc, view, s);
+}
+cudaError_t launch_view_mark(DevClock* clock, cudaStream_t s)
+{
+    view_mark_kernel<<<1, 1, 0, s>>>(clock);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_clock_finish(DevClock* clock, double dt, cudaStream_t s)

@@ -1,11 +1,11 @@
-"""Steps recorded into a caller's own CUDA graph order their particles each, as a replay does not know how
-many steps have passed since the last ordering."""
+"""Steps recorded into a caller's own CUDA graph: they order their particles each, as a replay does not know how
+many steps have passed since the last ordering, and take in a live device view when they are recorded."""
 import numpy as np
 import pytest
 import torch
 
 from dns_gkm_lpt_b200.solver import Solver
-from tests.gpu_helpers import case
+from tests.gpu_helpers import analytic_case, case
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,49 @@ def test_captured_steps_order_their_particles():
         assert np.array_equal(s.download_state(), want)
         for a, b in zip(s.particles_download(), want_pos):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("late", [False, True])
+@pytest.mark.parametrize("n", [14, 15])
+def test_captured_steps_and_the_device_state(n, late):
+    """Writes to the device state before the recording, or between it and the first replay, count; replays after the
+    first step on from their own result, and every later call sees it."""
+    P, W0 = analytic_case(n, 30 + n)
+    W1 = W0 * 1.0
+    W1[0] *= 1.01
+    with Solver(P, cfl=0.5) as s:
+        s.upload_state(W1)
+        dt = s.timestep()
+        s.set_dt(dt)
+        s.evolve_eulerian(2)
+        half = s.download_state()
+        s.evolve_eulerian(2)
+        want = s.download_state()
+    with Solver(P, cfl=0.5, use_graphs=False) as s:
+        s.set_dt(dt)
+        stream = torch.cuda.Stream()
+        s.set_stream(stream.cuda_stream)
+        s.upload_state(W0)
+        if not late:
+            s.device_state()[0] *= 1.01
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            view = s.device_state()
+            s.evolve_eulerian(2)
+        if late:
+            view[0] *= 1.01
+            torch.cuda.synchronize()
+            assert np.array_equal(s.download_state(), W1)
+        with torch.cuda.stream(stream):
+            g.replay()
+            if late:
+                assert np.array_equal(s.download_state(), half)
+            g.replay()
+        s.synchronize()
+        assert np.array_equal(s.device_state().cpu().numpy(), want)
+        assert np.array_equal(s.download_state(), want)
+        s.upload_state(W1)
+        s.evolve_eulerian(2)
+        s.synchronize()
+        assert np.array_equal(s.device_state().cpu().numpy(), half)
