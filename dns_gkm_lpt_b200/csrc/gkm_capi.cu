@@ -932,36 +932,43 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     a.dt_fixed_mode = h->dt_fixed_mode;
     a.dt_fixed = h->dt_fixed;
     const int nsegs[] = {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 24, 32};
+    constexpr int kTunedSegment = 8;   // the shortest of a tuned shape (gkm.h)
     gkm_status st = GKM_OK;
     for (int d = 0; d < 3 && st == GKM_OK; d++) {
-        SweepChoice best = h->sweep[d];
-        float best_ms = 1e30f;
-        for (int v = 0; v < nvar && st == GKM_OK; v++) {
+        std::vector<SweepChoice> shapes;
+        for (const SweepChoice& c : {h->sweep[d], default_choice(h->fc, mixed, d)})
+            if (c.seg_len >= kTunedSegment) shapes.push_back(c);
+        for (int v = 0; v < nvar; v++) {
             if (!mixed && v == 2 && !gkm::ws_ready()) continue;   // not available on this build
             int last_len = -1;
             for (int ns : nsegs) {
                 SweepChoice c;
                 c.variant = v;
                 c.seg_len = (h->fc.n + ns - 1) / ns;
-                if (c.seg_len < 8 || c.seg_len == last_len) continue;
+                if (c.seg_len < kTunedSegment || c.seg_len == last_len) continue;
                 last_len = c.seg_len;
                 c.nseg = (h->fc.n + c.seg_len - 1) / c.seg_len;
-                h->sweep[d] = c;
-                cudaError_t e = launch_sweep_any(h, d, a);   // warm-up
-                if (e == cudaSuccess) e = cudaEventRecord(e0, h->stream);
-                for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch_sweep_any(h, d, a);
-                if (e == cudaSuccess) e = cudaEventRecord(e1, h->stream);
-                if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-                float ms = 0.f;
-                if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-                if (e != cudaSuccess) {
-                    st = cuda_fail(h, e, "gkm_autotune");
-                    break;
-                }
-                if (ms < best_ms) {
-                    best_ms = ms;
-                    best = c;
-                }
+                shapes.push_back(c);
+            }
+        }
+        SweepChoice best = h->sweep[d];
+        float best_ms = 1e30f;
+        for (const SweepChoice& c : shapes) {
+            h->sweep[d] = c;
+            cudaError_t e = launch_sweep_any(h, d, a);   // warm-up
+            if (e == cudaSuccess) e = cudaEventRecord(e0, h->stream);
+            for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch_sweep_any(h, d, a);
+            if (e == cudaSuccess) e = cudaEventRecord(e1, h->stream);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            float ms = 0.f;
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+            if (e != cudaSuccess) {
+                st = cuda_fail(h, e, "gkm_autotune");
+                break;
+            }
+            if (ms < best_ms) {
+                best_ms = ms;
+                best = c;
             }
         }
         h->sweep[d] = best;
