@@ -441,6 +441,39 @@ gkm_status reduce_wave(gkm_handle* h)
     return GKM_OK;
 }
 
+// [p, p + bytes) lies in one allocation (or one registered range)
+bool one_allocation(const double* p, size_t bytes)
+{
+    using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess || !fn) {
+        cudaGetLastError();
+        return false;
+    }
+    const Query query = reinterpret_cast<Query>(fn);
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
+    return query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) == CUDA_SUCCESS &&
+           query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) == CUDA_SUCCESS && at >= start && at - start + bytes <= size;
+}
+
+// five arrays of `bytes` each in this device's memory, which its kernels may read and write (a copy checks that itself)
+bool on_device(const double* const W[5], size_t bytes, int device)
+{
+    for (int q = 0; q < 5; q++) {
+        cudaPointerAttributes at;
+        if (!W[q] || cudaPointerGetAttributes(&at, W[q]) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (at.type != cudaMemoryTypeDevice || at.device != device || !one_allocation(W[q], bytes)) return false;
+    }
+    return true;
+}
+
 gkm_status read_clock(gkm_handle* h, DevClock* c)
 {
     CK(h, cudaMemcpyAsync(c, h->clock, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
@@ -525,7 +558,8 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
     *dense = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
     double* out = h->buf[h->parity ^ 1];
-    CK(h, gkm::launch_rows_compact(*dense, out, h->fc, h->view_live ? h->clock : nullptr, h->stream));
+    CK(h, gkm::launch_rows_compact(h->buf[h->parity], gkm::dense_rows(out, h->fc), h->fc, h->view_live ? h->clock : nullptr,
+                                   h->stream));
     h->launches += 1;
     *dense = out;
     return GKM_OK;
@@ -534,7 +568,8 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 gkm_status gkm_host::take_view(gkm_handle* h)
 {
     if (!h->view_live) return GKM_OK;
-    CK(h, gkm::launch_rows_expand(h->buf[h->parity ^ 1], h->buf[h->parity], h->fc, h->clock, h->stream));
+    CK(h, gkm::launch_rows_expand(gkm::dense_rows(h->buf[h->parity ^ 1], h->fc), h->buf[h->parity], h->fc, h->clock,
+                                  h->stream));
     h->launches += 1;
     return GKM_OK;
 }
@@ -775,12 +810,14 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
         if (!W[q]) return fail(h, GKM_ERR_ARG, "W[q] is NULL");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
     double* dst = h->buf[h->parity];
-    // odd grids: dense rows through the accumulator buffer, free between steps, then to their pitch
-    double* land = h->fc.pitch == h->fc.nt ? dst : h->buf[h->parity ^ 1];
-    for (int q = 0; q < 5; q++)
-        CK(h, cudaMemcpyAsync(land + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
-    if (land != dst) {
-        CK(h, gkm::launch_rows_expand(land, dst, h->fc, nullptr, h->stream));
+    // odd grids: to their pitch from the device's own arrays, from others through the accumulator buffer, free between steps
+    const bool odd = h->fc.pitch != h->fc.nt;
+    const gkm::DenseRows land = gkm::dense_rows(odd ? h->buf[h->parity ^ 1] : dst, h->fc);
+    const bool direct = odd && on_device(W, bytes, h->cfg.device);
+    for (int q = 0; q < 5 && !direct; q++) CK(h, cudaMemcpyAsync(land.a[q], W[q], bytes, cudaMemcpyDefault, h->stream));
+    if (odd) {
+        const gkm::DenseRows own{{(double*)W[0], (double*)W[1], (double*)W[2], (double*)W[3], (double*)W[4]}};
+        CK(h, gkm::launch_rows_expand(direct ? own : land, dst, h->fc, nullptr, h->stream));
         h->launches += 1;
     }
     h->launches += 1;
@@ -802,6 +839,13 @@ gkm_status gkm_download_state(gkm_handle* h, double* const W[5])
     if (!h || !W) return GKM_ERR_ARG;
     if (!h->state_loaded) return fail(h, GKM_ERR_STATE, "no state uploaded");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
+    if (h->fc.pitch != h->fc.nt && !h->view_live && on_device(W, bytes, h->cfg.device)) {
+        const gkm::DenseRows own{{W[0], W[1], W[2], W[3], W[4]}};
+        CK(h, gkm::launch_rows_compact(h->buf[h->parity], own, h->fc, nullptr, h->stream));
+        h->launches += 1;
+        DevClock c;
+        return read_clock(h, &c);
+    }
     const double* src = nullptr;
     gkm_status s = gkm_host::dense_state(h, &src);
     if (s != GKM_OK) return s;
@@ -977,7 +1021,7 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (h->view_live) {   // the sweeps have written over it
-        gkm::launch_rows_compact(h->buf[h->parity], h->buf[h->parity ^ 1], h->fc, nullptr, h->stream);
+        gkm::launch_rows_compact(h->buf[h->parity], gkm::dense_rows(h->buf[h->parity ^ 1], h->fc), h->fc, nullptr, h->stream);
         h->launches += 1;
     }
     cudaMemcpyAsync(h->clock, &saved, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream);
@@ -1047,25 +1091,6 @@ bool async_capable(const double* p)
         return false;
     }
     return at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
-}
-
-// [p, p + bytes) lies in one allocation (or one registered range)
-bool one_allocation(const double* p, size_t bytes)
-{
-    using Query = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &found) != cudaSuccess ||
-        found != cudaDriverEntryPointSuccess || !fn) {
-        cudaGetLastError();
-        return false;
-    }
-    const Query query = reinterpret_cast<Query>(fn);
-    CUdeviceptr start = 0;
-    size_t size = 0;
-    const CUdeviceptr at = (CUdeviceptr)(uintptr_t)p;
-    return query(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) == CUDA_SUCCESS &&
-           query(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) == CUDA_SUCCESS && at >= start && at - start + bytes <= size;
 }
 
 // The plug point evolve(W, dt) as a pipeline over chunks of y-planes: the host -> device copy of
@@ -1500,7 +1525,8 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
     cudaStream_t s = rec ? h->own_stream : h->stream;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
-    cudaError_t e = gkm::launch_rows_compact(*W, h->buf[h->parity ^ 1], h->fc, h->view_live ? h->clock : nullptr, s);
+    cudaError_t e = gkm::launch_rows_compact(*W, gkm::dense_rows(h->buf[h->parity ^ 1], h->fc), h->fc,
+                                             h->view_live ? h->clock : nullptr, s);
     if (e == cudaSuccess) e = gkm::launch_view_mark(h->clock, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));

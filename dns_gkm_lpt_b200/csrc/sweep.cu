@@ -71,18 +71,29 @@ __global__ void halo_planes_kernel(double* W, FieldConst fc, int J0, int J1, con
 
 __global__ void view_mark_kernel(DevClock* clock) { clock->view = clock->iter + 1; }
 
-// rows of odd grids between the pitched layout and dense staging: a warp per row, bound by memory
+// rows of odd grids between the pitched layout and dense arrays: a warp per row, a component per blockIdx.y, bound
+// by memory
 template <bool EXPAND>
-__global__ void rows_kernel(const double* __restrict__ src, double* __restrict__ dst, long long rows, int nt, int pitch,
-                            const DevClock* view)
+__global__ void rows_kernel(DenseRows dense, double* __restrict__ W, FieldConst fc, const DevClock* view)
 {
     if (view && (view->view == view->iter + 1) != EXPAND) return;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, nt = fc.nt;
+    const long long rows = (long long)nt * nt;
+    double* __restrict__ D = dense.a[blockIdx.y];
+    double* __restrict__ P = W + blockIdx.y * fc.comp;
     for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows;
          r += ((long long)gridDim.x * blockDim.x) >> 5) {
-        const double* s = src + r * (EXPAND ? nt : pitch);
-        double* d = dst + r * (EXPAND ? pitch : nt);
-        for (int k = lane; k < nt; k += 32) d[k] = s[k];
+        const double* s = EXPAND ? D + r * nt : P + r * fc.pitch;
+        double* d = EXPAND ? P + r * fc.pitch : D + r * nt;
+        int k = lane;
+        for (; k + 96 < nt; k += 128) {   // four loads in flight per lane
+            const double v0 = s[k], v1 = s[k + 32], v2 = s[k + 64], v3 = s[k + 96];
+            d[k] = v0;
+            d[k + 32] = v1;
+            d[k + 64] = v2;
+            d[k + 96] = v3;
+        }
+        for (; k < nt; k += 32) d[k] = s[k];
     }
 }
 
@@ -351,21 +362,21 @@ cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, 
 }
 
 template <bool EXPAND>
-static cudaError_t rows_t(const double* src, double* dst, const FieldConst& fc, const DevClock* view, cudaStream_t s)
+static cudaError_t rows_t(const DenseRows& dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
-    const long long rows = 5LL * fc.nt * fc.nt;   // the components follow one another in both layouts
+    const long long rows = (long long)fc.nt * fc.nt;
     long long blocks = (rows + 7) / 8;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    rows_kernel<EXPAND><<<(unsigned)blocks, 256, 0, s>>>(src, dst, rows, fc.nt, fc.pitch, view);
+    if (blocks > 148 * 4) blocks = 148 * 4;
+    rows_kernel<EXPAND><<<dim3((unsigned)blocks, 5), 256, 0, s>>>(dense, W, fc, view);
     return cudaGetLastError();
 }
-cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
+cudaError_t launch_rows_expand(const DenseRows& dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
     return rows_t<true>(dense, W, fc, view, s);
 }
-cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, const DevClock* view, cudaStream_t s)
+cudaError_t launch_rows_compact(double* W, const DenseRows& dense, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
-    return rows_t<false>(W, dense, fc, view, s);
+    return rows_t<false>(dense, W, fc, view, s);
 }
 cudaError_t launch_view_mark(DevClock* clock, cudaStream_t s)
 {
