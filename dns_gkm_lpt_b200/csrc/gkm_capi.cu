@@ -262,7 +262,8 @@ cudaError_t enqueue_splines(gkm_handle* h, const double* W)
         w.group1 = h->d_self_off + 2;
         w.group2 = h->d_self_off + 4;
         h->launches += 3;
-        return gkm::launch_ensemble_splines(h->d_self, w, h->self_totals, 1, h->grid.npts, W == h->buf[0] ? 0 : 1,
+        return gkm::launch_ensemble_splines(h->d_self, w, h->self_totals, 1,
+                                            gkm::spline_launch(&h->grid.npts, 1), W == h->buf[0] ? 0 : 1,
                                             h->stream);
     }
     h->launches += kSplinePasses;
@@ -299,9 +300,10 @@ cudaError_t setup_batched_splines(gkm_handle* h)
     md.scratch[0] = h->scratch;
     md.scratch[1] = h->scratch_extra[0];
     md.scratch[2] = h->scratch_extra[1];
-    const int pad = h->grid.pad;
-    const long long off[6] = {0, 3 * gkm::spline_groups(0, N, pad), 0, 3 * gkm::spline_groups(1, N, pad),
-                              0, 3 * gkm::spline_groups(2, N, pad)};
+    const int npts = h->grid.npts, pad = h->grid.pad;
+    const gkm::SplineLaunch l = gkm::spline_launch(&npts, 1);
+    const long long off[6] = {0, gkm::spline_items(0, npts, pad, l), 0, gkm::spline_items(1, npts, pad, l),
+                              0, gkm::spline_items(2, npts, pad, l)};
     h->self_totals[0] = off[1];
     h->self_totals[1] = off[3];
     h->self_totals[2] = off[5];

@@ -38,6 +38,7 @@ struct gkm_ensemble {
     std::vector<gkm_handle*> mem;
     std::vector<double*> extra_scratch;   // two more spline scratch arrays per member (unless it has its own)
     bool mixed = false;
+    gkm::SplineLaunch splines{0, 0};
     int device = 0;
     cudaStream_t stream = nullptr;
     SweepChoice sweep[3];                 // window variant shared by all members (seg_len unused)
@@ -102,6 +103,10 @@ gkm_status refresh(gkm_ensemble* E, bool need_state)
         gkm_status s = gkm_host::take_view(E->mem[m]);
         if (s != GKM_OK) return efail(E, s, E->mem[m]->err);
     }
+    std::vector<int> lines;   // members without particles skip the spline work
+    for (const gkm_handle* h : E->mem)
+        if (h->np > 0) lines.push_back(h->grid.npts);
+    E->splines = lines.empty() ? gkm::SplineLaunch{0, 0} : gkm::spline_launch(lines.data(), (int)lines.size());
     std::vector<MemberDev> hm((size_t)nm);
     std::vector<long long> off((size_t)kNumSets * (nm + 1), 0);
     std::vector<std::vector<long long>> items(3, std::vector<long long>((size_t)nm, 0));
@@ -136,17 +141,16 @@ gkm_status refresh(gkm_ensemble* E, bool need_state)
         for (int c = 0; c < 6; c++) md.P[c] = h->P[c];
         md.np = h->np;
         md.tmaps = h->d_tmaps;
-        const long long N = h->grid.npts;
-        const int pad = h->grid.pad;
+        const int npts = h->grid.npts, pad = h->grid.pad;
         const long long nt = h->fc.nt;
-        const bool parts = h->np > 0;   // members without particles skip the spline work
+        const bool parts = h->np > 0;
         const long long count[kPart + 1] = {0,
                                             0,
                                             0,
                                             nt * nt * nt - n * n * n,
-                                            parts ? 3 * gkm::spline_groups(0, N, pad) : 0,
-                                            parts ? 3 * gkm::spline_groups(1, N, pad) : 0,
-                                            parts ? 3 * gkm::spline_groups(2, N, pad) : 0,
+                                            parts ? gkm::spline_items(0, npts, pad, E->splines) : 0,
+                                            parts ? gkm::spline_items(1, npts, pad, E->splines) : 0,
+                                            parts ? gkm::spline_items(2, npts, pad, E->splines) : 0,
                                             h->np};
         for (int s = kGhost; s <= kPart; s++) at(s, m + 1) = at(s, m) + count[s];
     }
@@ -202,11 +206,8 @@ cudaError_t launch_splines_all(gkm_ensemble* E, int parity)
     w.group2 = off_ptr(E, kGroup2);
     w.part = off_ptr(E, kPart);
     const long long totals[3] = {E->total[kGroup0], E->total[kGroup1], E->total[kGroup2]};
-    int max_npts = 0;
-    for (const gkm_handle* h : E->mem)
-        if (h->np > 0) max_npts = std::max(max_npts, h->grid.npts);
     E->launches += 3;
-    return gkm::launch_ensemble_splines(E->d_mem, w, totals, nm_of(E), max_npts, parity ^ 1, E->stream);
+    return gkm::launch_ensemble_splines(E->d_mem, w, totals, nm_of(E), E->splines, parity ^ 1, E->stream);
 }
 
 cudaError_t launch_particles_all(gkm_ensemble* E)

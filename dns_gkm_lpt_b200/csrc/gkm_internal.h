@@ -186,6 +186,14 @@ __host__ __device__ inline long long spline_groups(int pass, long long N, int pa
     const long long M = N + pad, lines = pass == 0 ? N * N : (pass == 1 ? M * N : M * M);
     return (lines + 31) / 32;
 }
+// How an ensemble's (or a handle's) spline passes run, by the points per line of each member with particles: warps per
+// block and bytes of shared memory of resident lines, or streamed lines (warps 0); and a member's work items in a
+// pass, of all three components
+struct SplineLaunch {
+    int warps, smem;
+};
+SplineLaunch spline_launch(const int* npts, int count);
+long long spline_items(int pass, int npts, int pad, const SplineLaunch& l);
 cudaError_t spline_prepare();   // the line kernels' shared-memory limit, on the current device
 cudaError_t launch_spline_build(const double* W, const FieldConst& fc, const SplineGrid& g, const SplineTables& tb,
                                 double* coef_u, double* coef_v, double* coef_w, double* scratch, cudaStream_t s);
@@ -271,7 +279,7 @@ struct MemberDev {
 struct EnsembleWork {           // prefix offsets, nm + 1 entries each, in device memory
     const long long* item[3];   // sweep work items per direction
     const long long* ghost;     // ghost cells
-    const long long* group0;    // groups of 32 spline lines of the 3 components, pass 0
+    const long long* group0;    // spline_items of pass 0
     const long long* group1;    // pass 1
     const long long* group2;    // pass 2
     const long long* part;      // particles
@@ -301,7 +309,7 @@ cudaError_t launch_ensemble_sweep32(int dir, int variant, const MemberDev* mem, 
 cudaError_t launch_ensemble_halo(const MemberDev* mem, const long long* off, int nm, long long total, int buf,
                                  int finish_step, cudaStream_t s);
 cudaError_t launch_ensemble_splines(const MemberDev* mem, const EnsembleWork& w, const long long totals[3], int nm,
-                                    int max_npts, int buf, cudaStream_t s);
+                                    const SplineLaunch& l, int buf, cudaStream_t s);
 cudaError_t launch_ensemble_heun(const MemberDev* mem, const long long* off, int nm, long long total, cudaStream_t s);
 
 // Thomas tables of the spline line solves (gkm_capi.cu)

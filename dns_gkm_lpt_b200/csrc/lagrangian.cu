@@ -21,6 +21,8 @@
 #include "gkm_internal.h"
 #include "pivot_div.cuh"
 
+#include <algorithm>
+
 namespace gkm {
 namespace {
 
@@ -587,7 +589,7 @@ __global__ void __launch_bounds__(32 * kPass2Warps) spline_pass2_f32(double* in,
         pass2_group_f32(in, g, tb, out, L0, lines, stage[warp]);
 }
 
-// ---- lines resident in shared memory.  A warp (one CTA) takes 32 lines: their values come in at
+// ---- lines resident in shared memory.  A warp (a CTA of its own, but for ensembles) takes 32 lines: their values come in at
 // once, all loads in flight, each lane solves its line in place, and the coefficients go out, so a
 // pass reads and writes global memory once.  The forward values of the kernels above make the round
 // through global memory instead, and their loads wait on one another 4 or 8 at a time.  What
@@ -598,7 +600,7 @@ __global__ void __launch_bounds__(32 * kPass2Warps) spline_pass2_f32(double* in,
 // FP32) 128^3 0.511 -> 0.198, 200^3 0.99 -> 0.76, 224^3 1.25 -> 1.09, 256^3 1.58 -> 1.50, 282^3 1.80 -> 1.90.
 constexpr int kResidentBatched = 200, kResidentSingle = 264;
 constexpr int kTableRows = kPivotRows + 2;   // rows of the tables a warp keeps beside its lines
-inline size_t resident_bytes(int npts) { return sizeof(double) * (2 * kTableRows + 32 * (size_t)(npts | 1)); }
+__host__ __device__ inline int resident_bytes(int npts) { return (int)sizeof(double) * (2 * kTableRows + 32 * (npts | 1)); }
 
 // 8-byte asynchronous copies, a thread's own (its wait covers them)
 __device__ __forceinline__ void copy8_async(double* dst, const double* src)
@@ -621,7 +623,7 @@ struct LineTables {
 // issued with the lines' own copies; the caller waits and synchronises the warp
 __device__ __forceinline__ LineTables line_tables(const SplineTables& tb, int N, int periodic, double* smem)
 {
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     if (lane < kTableRows && lane <= N) {
         copy8_async(smem + lane, tb.mt + lane);
         copy8_async(smem + kTableRows + lane, tb.dp + lane);
@@ -738,7 +740,7 @@ __device__ __forceinline__ void resident_pass0(const double* __restrict__ W, con
                                                const SplineTables& tb, int q, double* __restrict__ out, long long stride,
                                                long long group, double* smem)
 {
-    const int N = g.npts, lane = threadIdx.x;
+    const int N = g.npts, lane = threadIdx.x & 31;
     const LineTables T = line_tables(tb, N, g.periodic, smem);
     const bool mine = group * 32 + lane < (long long)N * N;
     const long long L = mine ? group * 32 + lane : (long long)N * N - 1;   // a lane beyond the lines repeats the last
@@ -788,7 +790,7 @@ __device__ __forceinline__ void resident_pass0(const double* __restrict__ W, con
 __device__ __forceinline__ void resident_pass1(const double* in, int in_rows, const SplineGrid& g, const SplineTables& tb,
                                                double* out, long long group, double* smem)
 {
-    const int N = g.npts, M = N + g.pad, lane = threadIdx.x;
+    const int N = g.npts, M = N + g.pad, lane = threadIdx.x & 31;
     const LineTables T = line_tables(tb, N, g.periodic, smem);
     const bool mine = group * 32 + lane < (long long)M * N;
     const long long L = mine ? group * 32 + lane : (long long)M * N - 1;
@@ -813,7 +815,7 @@ template <class OutT>
 __device__ __forceinline__ void resident_pass2(const double* __restrict__ in, const SplineGrid& g, const SplineTables& tb,
                                                OutT* __restrict__ out, long long group, double* smem)
 {
-    const int N = g.npts, M = N + g.pad, S = N | 1, lane = threadIdx.x;
+    const int N = g.npts, M = N + g.pad, S = N | 1, lane = threadIdx.x & 31;
     const long long lines = (long long)M * M, L0 = group * 32;
     const int nl = (int)min(32LL, lines - L0);
     const LineTables T = line_tables(tb, N, g.periodic, smem);
@@ -1496,7 +1498,8 @@ cudaError_t grid_launch(K kernel, long long work, int threads, cudaStream_t s, A
 }
 
 // ---- ensemble forms: one launch per pass over every member's lines / particles; the lines in groups of
-// 32, one warp each, off[] the members' groups of all three components
+// 32, one warp each, off[] the members' work items of all three components: groups, or with resident lines
+// blocks of them (spline_items)
 __device__ __forceinline__ const MemberDev& ensemble_group(const MemberDev* __restrict__ mem,
                                                            const long long* __restrict__ off, int nm, long long w,
                                                            int pass, int& q, long long& group)
@@ -1509,33 +1512,78 @@ __device__ __forceinline__ const MemberDev& ensemble_group(const MemberDev* __re
     return md;
 }
 
-__global__ void __launch_bounds__(32) ensemble_resident0(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
-                                                         int nm, int buf)
+// Resident lines of members of several sizes: a block has the shared memory of the largest member's group, rounded up as
+// far as no block per SM is lost, and takes as many groups of one component of a member as fit it (a warp each),
+// so small members' lines fill the SMs as well.  With one group per block whatever its size, 64 members of
+// 48^3 beside one of 194^3 took 1.75 ms (four warps per SM for all lines) against 1.39 streamed; so 1.18.
+constexpr int kEnsembleWarps = 4;
+__host__ __device__ inline int resident_per_block(int npts, int warps, int smem)
 {
-    extern __shared__ double line_smem[];
-    int q;
-    long long group;
-    const MemberDev& md = ensemble_group(mem, off, nm, blockIdx.x, 0, q, group);
-    resident_pass0<true>(md.buf[buf], md.fc, md.grid, md.tb, q + 1, md.coef[q], (long long)md.grid.npts * md.grid.npts,
-                         group, line_smem);
+    const int fit = smem / resident_bytes(npts);
+    return fit < warps ? fit : warps;
 }
-__global__ void __launch_bounds__(32) ensemble_resident1(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
-                                                         int nm)
+// this warp's group of component q of a member and its part of the shared memory; false without one
+template <int WARPS>
+__device__ __forceinline__ bool ensemble_resident(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
+                                                  int nm, int pass, int bytes, const MemberDev*& md, int& q,
+                                                  long long& group, double*& smem)
 {
     extern __shared__ double line_smem[];
-    int q;
-    long long group;
-    const MemberDev& md = ensemble_group(mem, off, nm, blockIdx.x, 1, q, group);
-    resident_pass1(md.coef[q], md.grid.npts, md.grid, md.tb, md.scratch[q], group, line_smem);
+    const int m = find_member(off, nm, blockIdx.x);
+    md = mem + m;
+    const int N = md->grid.npts;
+    if constexpr (WARPS == 1) {
+        const long long local = blockIdx.x - off[m], groups = spline_groups(pass, N, md->grid.pad);
+        q = (int)(local / groups);
+        group = local - q * groups;
+        smem = line_smem;
+        return true;
+    }
+    const int warp = threadIdx.x >> 5, per = resident_per_block(N, blockDim.x >> 5, bytes);
+    const long long groups = spline_groups(pass, N, md->grid.pad), blocks = (groups + per - 1) / per;
+    const long long local = blockIdx.x - off[m];
+    q = (int)(local / blocks);
+    group = (local - q * blocks) * per + warp;
+    smem = line_smem + warp * (resident_bytes(N) / (int)sizeof(double));
+    return warp < per && group < groups;
 }
-__global__ void __launch_bounds__(32) ensemble_resident2(const MemberDev* __restrict__ mem, const long long* __restrict__ off,
-                                                         int nm)
+
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) ensemble_resident0(const MemberDev* __restrict__ mem,
+                                                                  const long long* __restrict__ off, int nm,
+                                                                  int buf, int bytes)
 {
-    extern __shared__ double line_smem[];
+    const MemberDev* md;
     int q;
     long long group;
-    const MemberDev& md = ensemble_group(mem, off, nm, blockIdx.x, 2, q, group);
-    resident_pass2<double>(md.scratch[q], md.grid, md.tb, md.coef[q], group, line_smem);
+    double* smem;
+    if (!ensemble_resident<WARPS>(mem, off, nm, 0, bytes, md, q, group, smem)) return;
+    resident_pass0<true>(md->buf[buf], md->fc, md->grid, md->tb, q + 1, md->coef[q],
+                         (long long)md->grid.npts * md->grid.npts, group, smem);
+}
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) ensemble_resident1(const MemberDev* __restrict__ mem,
+                                                                  const long long* __restrict__ off, int nm,
+                                                                  int bytes)
+{
+    const MemberDev* md;
+    int q;
+    long long group;
+    double* smem;
+    if (!ensemble_resident<WARPS>(mem, off, nm, 1, bytes, md, q, group, smem)) return;
+    resident_pass1(md->coef[q], md->grid.npts, md->grid, md->tb, md->scratch[q], group, smem);
+}
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) ensemble_resident2(const MemberDev* __restrict__ mem,
+                                                                  const long long* __restrict__ off, int nm,
+                                                                  int bytes)
+{
+    const MemberDev* md;
+    int q;
+    long long group;
+    double* smem;
+    if (!ensemble_resident<WARPS>(mem, off, nm, 2, bytes, md, q, group, smem)) return;
+    resident_pass2<double>(md->scratch[q], md->grid, md->tb, md->coef[q], group, smem);
 }
 
 __global__ void __launch_bounds__(128, kPassCtasPerSm) ensemble_pass0_kernel(const MemberDev* __restrict__ mem, const long long* __restrict__ off, int nm,
@@ -1597,11 +1645,14 @@ __global__ void ensemble_heun_kernel(const MemberDev* __restrict__ mem, const lo
 // the line kernels' shared-memory limit, on the current device
 cudaError_t resident_prepare()
 {
-    const int bytes = (int)resident_bytes(kResidentSingle > kResidentBatched ? kResidentSingle : kResidentBatched);
+    const int bytes = resident_bytes(kResidentSingle > kResidentBatched ? kResidentSingle : kResidentBatched);
     const void* kernels[] = {(const void*)spline_resident0<true>,    (const void*)spline_resident0<false>,
                              (const void*)spline_resident1,          (const void*)spline_resident2<double>,
-                             (const void*)spline_resident2<float>,   (const void*)ensemble_resident0,
-                             (const void*)ensemble_resident1,        (const void*)ensemble_resident2};
+                             (const void*)spline_resident2<float>,   (const void*)ensemble_resident0<1>,
+                             (const void*)ensemble_resident1<1>,     (const void*)ensemble_resident2<1>,
+                             (const void*)ensemble_resident0<kEnsembleWarps>,
+                             (const void*)ensemble_resident1<kEnsembleWarps>,
+                             (const void*)ensemble_resident2<kEnsembleWarps>};
     for (const void* k : kernels) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) return e;
@@ -1615,7 +1666,7 @@ template <class OutT>
 cudaError_t resident_component(const double* W, const FieldConst& fc, const SplineGrid& g, const SplineTables& tb, int q,
                                double* mid, long long stride0, int in_rows, double* buf, OutT* out, cudaStream_t s)
 {
-    const size_t smem = resident_bytes(g.npts);
+    const int smem = resident_bytes(g.npts);
     const unsigned g0 = (unsigned)spline_groups(0, g.npts, g.pad), g1 = (unsigned)spline_groups(1, g.npts, g.pad),
                    g2 = (unsigned)spline_groups(2, g.npts, g.pad);
     if (q >= 1 && q <= 3) spline_resident0<true><<<g0, 32, smem, s>>>(W, fc, g, tb, q, mid, stride0);
@@ -1669,20 +1720,52 @@ cudaError_t launch_spline_component(const double* W, const FieldConst& fc, const
     return launch_pass2((const double*)scratch, g, tb, coef, s);
 }
 
-cudaError_t launch_ensemble_splines(const MemberDev* mem, const EnsembleWork& w, const long long totals[3], int nm,
-                                    int max_npts, int buf, cudaStream_t s)
+SplineLaunch spline_launch(const int* npts, int count)
 {
-    if (max_npts <= kResidentBatched) {
-        const size_t smem = resident_bytes(max_npts);
-        ensemble_resident0<<<(unsigned)totals[0], 32, smem, s>>>(mem, w.group0, nm, buf);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        ensemble_resident1<<<(unsigned)totals[1], 32, smem, s>>>(mem, w.group1, nm);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-        ensemble_resident2<<<(unsigned)totals[2], 32, smem, s>>>(mem, w.group2, nm);
-        return cudaGetLastError();
+    const int most = *std::max_element(npts, npts + count), least = *std::min_element(npts, npts + count);
+    if (most > kResidentBatched) return {0, 0};
+    constexpr int kPerSm = 228 * 1024, kReserved = 1024;   // an SM's shared memory, and what it keeps of it per block
+    const int bytes = resident_bytes(most), ctas = kPerSm / (bytes + kReserved);
+    const int smem = (kPerSm / (ctas < 32 ? ctas : 32) - kReserved) & ~15;
+    const int warps = resident_per_block(least, kEnsembleWarps, smem);
+    // Blocks of several groups where they save a tenth of the groups' time, taken as points over groups per SM: below
+    // that their longer code decides (16 members of 32^3 to 2 of 96^3, 7 % by this count: 0.432 -> 0.446 ms; 30 of
+    // 32^3 and 2 of 96^3, 22 %: 0.282 -> 0.260; 31 of 32^3 and one of 194^3, 13 %: 0.847 -> 0.728).
+    double single = 0.0, packed = 0.0;
+    for (int k = 0; k < count; k++) {
+        const double points = (double)npts[k] * npts[k] * npts[k];
+        single += points;
+        packed += points / resident_per_block(npts[k], warps, smem);
     }
+    if (packed > 0.9 * single) return {1, bytes};
+    return {warps, smem};
+}
+long long spline_items(int pass, int npts, int pad, const SplineLaunch& l)
+{
+    const long long groups = spline_groups(pass, npts, pad), per = l.warps ? resident_per_block(npts, l.warps, l.smem) : 1;
+    return 3 * ((groups + per - 1) / per);
+}
+
+template <int WARPS>
+static cudaError_t ensemble_resident_t(const MemberDev* mem, const EnsembleWork& w, const long long totals[3], int nm,
+                                       const SplineLaunch& l, int buf, cudaStream_t s)
+{
+    const int threads = 32 * l.warps;
+    ensemble_resident0<WARPS><<<(unsigned)totals[0], threads, l.smem, s>>>(mem, w.group0, nm, buf, l.smem);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    ensemble_resident1<WARPS><<<(unsigned)totals[1], threads, l.smem, s>>>(mem, w.group1, nm, l.smem);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    ensemble_resident2<WARPS><<<(unsigned)totals[2], threads, l.smem, s>>>(mem, w.group2, nm, l.smem);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_ensemble_splines(const MemberDev* mem, const EnsembleWork& w, const long long totals[3], int nm,
+                                    const SplineLaunch& l, int buf, cudaStream_t s)
+{
+    if (l.warps == 1) return ensemble_resident_t<1>(mem, w, totals, nm, l, buf, s);
+    if (l.warps > 1) return ensemble_resident_t<kEnsembleWarps>(mem, w, totals, nm, l, buf, s);
     cudaError_t e = grid_launch(ensemble_pass0_kernel, totals[0] * 32, 128, s, mem, w.group0, nm, buf);
     if (e != cudaSuccess) return e;
     e = grid_launch(ensemble_pass1_kernel, totals[1] * 32, 128, s, mem, w.group1, nm);
