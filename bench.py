@@ -22,7 +22,8 @@ same cell count;
 c2_256_curves, both forms over 200 steps of the 256^3 case with the
 PrintStats curves every 10 steps; c3_512, the 512^3 case (Mt 0.5,
 Re_lambda 100, 4 x 10^6 particles) over 500 steps in both forms, with the
-mixed form's field and curve errors against the FP64 run.
+mixed form's field and curve errors against the FP64 run.  The line carries their rates and largest
+errors; --details FILE writes the forms in full: curve and error tables, phases, sweep shapes.
 
 --impl reference: the reference's own CPU code (oracle/_ref, compiled from
 the reference sources) on all host cores, one 64^3 cube per process (the
@@ -56,12 +57,41 @@ REF_PART = N_PART * REF_N ** 3 // N_CELLS ** 3   # same particle density
 C3_PART = 4_000_000          # particles of the 512^3 mixed-precision case
 HBM_FALLBACK_GBS = 6650.0    # an earlier copy-bandwidth measurement on these B200s, used only without a
                              # measured-peaks file beside this script
-# FP64 instructions the three sweeps execute per cell update (ncu smsp__inst_executed_pipe_fp64 at 192^3, 16 x 8
-# windows: 375.3 M, 376.4 M and 384.7 M warp instructions)
-FP64_INSTR_PER_CELL_UPDATE = 5137
-# DRAM bytes per cell of one sweep launch: mean over the x, y, z sweeps of the ncu capture of this
-# benchmark's 256^3 cube (83.8, 123.3, 141.4 B; compulsory 80, 120, 120)
-SWEEP_DRAM_BYTES_PER_CELL = 116.2
+# FP64 instructions the FP64 sweeps execute per face, by window variant, for x, y and z (ncu
+# smsp__inst_executed_pipe_fp64 at 192^3 with 48-face segments; a segment of L faces computes L + 1.  With 64 faces at
+# 256^3 the same within 0.1 %, with 16 at 192^3 within 0.3 %).  Whole windows: grids of a multiple of 16 cells
+FP64_INSTR_PER_FACE = {0: (1662.2, 1667.1, 1703.6), 1: (1609.5, 1615.4, 1650.9), 2: (1688.4, 1706.2, 1714.8)}
+# DRAM bytes per cell of one FP64 sweep launch of this benchmark's 256^3 cube: mean over the x, y, z sweeps of the ncu
+# capture (warp-specialized x and y, 16 x 8 z, 64 faces: 84.4, 124.3, 147.0 B; compulsory 80, 120, 120)
+SWEEP_DRAM_BYTES_PER_CELL = 118.6
+
+
+def fp64_instr_per_cell_update(n: int, shapes):
+    """FP64 instructions per cell update that sweeps of these shapes (Solver.sweep_config) execute, or None
+    where they were not counted."""
+    if n % 16 or any(c["variant"] not in FP64_INSTR_PER_FACE for c in shapes):
+        return None
+    return sum(FP64_INSTR_PER_FACE[c["variant"]][d] * (n + -(-n // c["segment"])) / n for d, c in enumerate(shapes))
+
+
+def short_line(line: dict, details: str) -> str:
+    """The result as one line of JSON with numbers of seven digits, the side forms without what is long: their curve
+    and error tables, phases, shapes, workloads and remarks go to the file `details` (without a name they are left out)."""
+    if details:
+        with open(details, "w") as f:
+            json.dump(line["forms"], f)
+    long = {"curves", "sweep_shapes", "stats_rel_err_vs_fp64", "particle_stats_rel_err_vs_fp64",
+            "curve_max_rel_err_mixed_vs_fp64", "curve_max_rel_err_vs_fp64", "phases_ms_per_step", "config", "what"}
+
+    def cut(v, left_out=frozenset()):
+        if isinstance(v, dict):
+            return {k: cut(x, left_out) for k, x in v.items() if k not in left_out}
+        if isinstance(v, (list, tuple)):
+            return [cut(x, left_out) for x in v]
+        return float(f"{v:.7g}") if isinstance(v, float) else v
+
+    shapes = [[c["variant"], c["segment"]] for c in line["sweep_shapes"]]
+    return json.dumps(dict(cut(line), sweep_shapes=shapes, forms=cut(line["forms"], long)))
 
 
 def hbm_peak():
@@ -696,7 +726,8 @@ def ours(args, rank: int, world: int, local_rank: int):
     flops_launch = flops_cell * cells / 3                   # one of the three sweeps
     achieved = flops_launch / launch_s / 1e12
     bytes_launch = (80 + 120 + 120) / 3 * cells             # compulsory W read + accumulator traffic
-    traffic = None if SWEEP_DRAM_BYTES_PER_CELL is None else SWEEP_DRAM_BYTES_PER_CELL * cells
+    traffic = SWEEP_DRAM_BYTES_PER_CELL * cells if n == N_CELLS and not prec else None
+    executed = None if prec else fp64_instr_per_cell_update(n, sweep_cfg)
     peak = fp32_peak if prec else fp64_peak
     hbm_gbs, hbm_src = hbm_peak()
 
@@ -710,9 +741,9 @@ def ours(args, rank: int, world: int, local_rank: int):
             "phases_ms_per_step": {k: v / args.steps for k, v in ph.items()},
             "roofline": {"kernel": "sweep_kernel (x/y/z, one launch each per step)", "bound": "fp32" if prec else "fp64",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                         "traffic": traffic if not prec else None, "flops_per_cell_update": flops_cell,
+                         "traffic": traffic, "flops_per_cell_update": flops_cell,
                          # the numerator is the reference's formulation; what the FP64 sweeps execute, in FMA slots
-                         "executed_frac": None if prec else FP64_INSTR_PER_CELL_UPDATE * 2 * cells / 3 / launch_s / 1e12 / peak,
+                         "executed_frac": executed and executed * 2 * cells / 3 / launch_s / 1e12 / peak,
                          "peak_source": "FMA probe run by this bench (gkm_probe_fma_peak)",
                          "hbm": {"achieved_gbs": bytes_launch / launch_s / 1e9, "peak_gbs": hbm_gbs,
                                  "frac": bytes_launch / launch_s / 1e9 / hbm_gbs, "peak_source": hbm_src}},
@@ -727,7 +758,7 @@ def ours(args, rank: int, world: int, local_rank: int):
                                 "kind": r["kind"],
                                 "sample": reference_sample_text(workers, args.warmup, args.steps, r["wall_s"], r["kind"]),
                                 "particle_steps_per_s": r["psteps"]}
-    print(json.dumps(line), flush=True)
+    print(short_line(line, args.details), flush=True)
 
 
 def main():
@@ -754,6 +785,7 @@ def main():
                          "(window variant:segment length)")
     ap.add_argument("--autotune-reps", type=int, default=2,
                     help="timed launches per sweep shape; 0 keeps the default shapes (profiling runs)")
+    ap.add_argument("--details", default="", help="file for the side forms in full: curve tables, error tables, shapes")
     args = ap.parse_args()
     if args.warmup < 3:
         args.warmup = 3
