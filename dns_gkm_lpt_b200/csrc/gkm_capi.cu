@@ -555,14 +555,19 @@ gkm_status compute_props(gkm_handle* h)
 
 }  // namespace
 
+// A live view is the state where steps are the host's alone (use_graphs: they cannot be recorded by a caller); else
+// its launches ask the device.
+static const DevClock* ask_device(const gkm_handle* h) { return h->cfg.use_graphs ? nullptr : h->clock; }
+
 gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 {
     *dense = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
     double* out = h->buf[h->parity ^ 1];
-    CK(h, gkm::launch_rows_compact(h->buf[h->parity], gkm::dense_rows(out, h->fc), h->fc, h->view_live ? h->clock : nullptr,
-                                   h->stream));
-    h->launches += 1;
+    if (!h->view_live || ask_device(h)) {
+        CK(h, gkm::launch_rows_compact(h->buf[h->parity], out, h->fc, h->view_live ? h->clock : nullptr, h->stream));
+        h->launches += 1;
+    }
     *dense = out;
     return GKM_OK;
 }
@@ -570,8 +575,7 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 gkm_status gkm_host::take_view(gkm_handle* h)
 {
     if (!h->view_live) return GKM_OK;
-    CK(h, gkm::launch_rows_expand(gkm::dense_rows(h->buf[h->parity ^ 1], h->fc), h->buf[h->parity], h->fc, h->clock,
-                                  h->stream));
+    CK(h, gkm::launch_rows_expand(h->buf[h->parity ^ 1], h->buf[h->parity], h->fc, ask_device(h), h->stream));
     h->launches += 1;
     return GKM_OK;
 }
@@ -814,13 +818,18 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
     double* dst = h->buf[h->parity];
     // odd grids: to their pitch from the device's own arrays, from others through the accumulator buffer, free between steps
     const bool odd = h->fc.pitch != h->fc.nt;
-    const gkm::DenseRows land = gkm::dense_rows(odd ? h->buf[h->parity ^ 1] : dst, h->fc);
-    const bool direct = odd && on_device(W, bytes, h->cfg.device);
-    for (int q = 0; q < 5 && !direct; q++) CK(h, cudaMemcpyAsync(land.a[q], W[q], bytes, cudaMemcpyDefault, h->stream));
-    if (odd) {
+    double* land = odd ? h->buf[h->parity ^ 1] : dst;
+    if (odd && on_device(W, bytes, h->cfg.device)) {
         const gkm::DenseRows own{{(double*)W[0], (double*)W[1], (double*)W[2], (double*)W[3], (double*)W[4]}};
-        CK(h, gkm::launch_rows_expand(direct ? own : land, dst, h->fc, nullptr, h->stream));
+        CK(h, gkm::launch_arrays(true, own, dst, h->fc, h->stream));
         h->launches += 1;
+    } else {
+        for (int q = 0; q < 5; q++)
+            CK(h, cudaMemcpyAsync(land + (size_t)q * h->fc.nt3, W[q], bytes, cudaMemcpyDefault, h->stream));
+        if (odd) {
+            CK(h, gkm::launch_rows_expand(land, dst, h->fc, nullptr, h->stream));
+            h->launches += 1;
+        }
     }
     h->launches += 1;
     CK(h, gkm::launch_halo(dst, h->fc, h->clock, 0, h->parity, 0, 0.0, h->stream));
@@ -843,7 +852,7 @@ gkm_status gkm_download_state(gkm_handle* h, double* const W[5])
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
     if (h->fc.pitch != h->fc.nt && !h->view_live && on_device(W, bytes, h->cfg.device)) {
         const gkm::DenseRows own{{W[0], W[1], W[2], W[3], W[4]}};
-        CK(h, gkm::launch_rows_compact(h->buf[h->parity], own, h->fc, nullptr, h->stream));
+        CK(h, gkm::launch_arrays(false, own, h->buf[h->parity], h->fc, h->stream));
         h->launches += 1;
         DevClock c;
         return read_clock(h, &c);
@@ -1023,7 +1032,7 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (h->view_live) {   // the sweeps have written over it
-        gkm::launch_rows_compact(h->buf[h->parity], gkm::dense_rows(h->buf[h->parity ^ 1], h->fc), h->fc, nullptr, h->stream);
+        gkm::launch_rows_compact(h->buf[h->parity], h->buf[h->parity ^ 1], h->fc, nullptr, h->stream);
         h->launches += 1;
     }
     cudaMemcpyAsync(h->clock, &saved, sizeof(DevClock), cudaMemcpyHostToDevice, h->stream);
@@ -1521,19 +1530,21 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
     if (!h || !W) return GKM_ERR_ARG;
     *W = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
+    if (h->view_live && !ask_device(h)) {
+        *W = h->buf[h->parity ^ 1];
+        return GKM_OK;
+    }
     // The caller may read it on any stream, as it may the state of an idle handle: done when the call returns,
     // also while the caller records h->stream.
     const bool rec = recording(h);
     cudaStream_t s = rec ? h->own_stream : h->stream;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
-    cudaError_t e = gkm::launch_rows_compact(*W, gkm::dense_rows(h->buf[h->parity ^ 1], h->fc), h->fc,
-                                             h->view_live ? h->clock : nullptr, s);
-    if (e == cudaSuccess) e = gkm::launch_view_mark(h->clock, s);
+    cudaError_t e = gkm::launch_view(*W, h->buf[h->parity ^ 1], h->fc, h->clock, h->view_live, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
     CK(h, e);
-    h->launches += 2;
+    h->launches += h->view_live ? 2 : 1;
     h->view_live = true;
     *W = h->buf[h->parity ^ 1];
     return GKM_OK;

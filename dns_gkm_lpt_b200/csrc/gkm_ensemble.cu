@@ -497,7 +497,7 @@ gkm_status gkm_ensemble_autotune(gkm_ensemble* E, int32_t reps)
     }
     E->launches = launches0;   // tuning launches are not steps
     for (gkm_handle* h : views) {
-        gkm::launch_rows_compact(h->buf[p], gkm::dense_rows(h->buf[p ^ 1], h->fc), h->fc, nullptr, E->stream);
+        gkm::launch_rows_compact(h->buf[p], h->buf[p ^ 1], h->fc, nullptr, E->stream);
         h->view_live = true;
     }
     cudaEventDestroy(e0);

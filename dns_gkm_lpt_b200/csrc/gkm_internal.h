@@ -122,20 +122,18 @@ cudaError_t launch_sweep(int dir, int variant, const SweepArgs& a, int nseg, cud
 // The cells updated are exactly those of planes [j0, j1).
 cudaError_t launch_sweep_rows(int dir, int variant, SweepArgs a, int j0, int j1, cudaStream_t s);
 cudaError_t launch_sweep_mixed_rows(int dir, int variant, SweepArgs a, int j0, int j1, cudaStream_t s);
-// The state between the device's pitched rows and dense arrays of nt^3 in device memory, one per component.
+// The state between the device's pitched rows and dense rows (dense: 5 components of nt^3 in device memory).
 // With `view`, dense is the caller's view: expanded only while it is the state, compacted only where it is not (a
 // graph that a caller recorded takes steps that the host does not see).
+cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s);
+cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, const DevClock* view, cudaStream_t s);
+// dense becomes the view: from now to the next step it is the state; maybe: it may be that already
+cudaError_t launch_view(const double* W, double* dense, const FieldConst& fc, DevClock* clock, bool maybe, cudaStream_t s);
+// and between those rows and the caller's five device arrays
 struct DenseRows {
     double* a[5];
 };
-inline DenseRows dense_rows(double* base, const FieldConst& fc)
-{
-    return {{base, base + fc.nt3, base + 2 * fc.nt3, base + 3 * fc.nt3, base + 4 * fc.nt3}};
-}
-cudaError_t launch_rows_expand(const DenseRows& dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s);
-cudaError_t launch_rows_compact(double* W, const DenseRows& dense, const FieldConst& fc, const DevClock* view, cudaStream_t s);
-// from now to the next step the view is the state
-cudaError_t launch_view_mark(DevClock* clock, cudaStream_t s);
+cudaError_t launch_arrays(bool expand, const DenseRows& dense, double* W, const FieldConst& fc, cudaStream_t s);
 // Ghost cells of the ghost-layout y-planes [J0, J1) (0 <= J0 < J1 <= nt) from their periodic images;
 // odd grids' plug point: with `from` every cell of those planes from the dense state, with `to` the planes
 // written to it as well

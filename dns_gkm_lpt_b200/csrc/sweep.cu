@@ -71,29 +71,43 @@ __global__ void halo_planes_kernel(double* W, FieldConst fc, int J0, int J1, con
 
 __global__ void view_mark_kernel(DevClock* clock) { clock->view = clock->iter + 1; }
 
-// rows of odd grids between the pitched layout and dense arrays: a warp per row, a component per blockIdx.y, bound
-// by memory
+// Rows of odd grids between the pitched layout and dense ones: a warp per row, bound by memory.  The components follow one
+// another in both.
 template <bool EXPAND>
-__global__ void rows_kernel(DenseRows dense, double* __restrict__ W, FieldConst fc, const DevClock* view)
+__global__ void rows_kernel(const double* __restrict__ src, double* __restrict__ dst, long long rows, int nt, int pitch,
+                            const DevClock* view, DevClock* mark)
 {
     if (view && (view->view == view->iter + 1) != EXPAND) return;
+    if (mark && blockIdx.x == 0 && threadIdx.x == 0) mark->view = mark->iter + 1;
+    const int lane = threadIdx.x & 31;
+    for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows;
+         r += ((long long)gridDim.x * blockDim.x) >> 5) {
+        const double* s = src + r * (EXPAND ? nt : pitch);
+        double* d = dst + r * (EXPAND ? pitch : nt);
+        for (int k = lane; k < nt; k += 32) d[k] = s[k];
+    }
+}
+// the same with the caller's five arrays, a component per blockIdx.y, eight loads in flight per lane
+template <bool EXPAND>
+__global__ void arrays_kernel(DenseRows dense, double* W, FieldConst fc)
+{
     const int lane = threadIdx.x & 31, nt = fc.nt;
     const long long rows = (long long)nt * nt;
-    double* __restrict__ D = dense.a[blockIdx.y];
-    double* __restrict__ P = W + blockIdx.y * fc.comp;
+    double* D = dense.a[blockIdx.y];
+    double* P = W + blockIdx.y * fc.comp;
     for (long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; r < rows;
          r += ((long long)gridDim.x * blockDim.x) >> 5) {
         const double* s = EXPAND ? D + r * nt : P + r * fc.pitch;
         double* d = EXPAND ? P + r * fc.pitch : D + r * nt;
-        int k = lane;
-        for (; k + 96 < nt; k += 128) {   // four loads in flight per lane
-            const double v0 = s[k], v1 = s[k + 32], v2 = s[k + 64], v3 = s[k + 96];
-            d[k] = v0;
-            d[k + 32] = v1;
-            d[k + 64] = v2;
-            d[k + 96] = v3;
+        for (int k = lane; k < nt; k += 256) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (k + 32 * u < nt) v[u] = s[k + 32 * u];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (k + 32 * u < nt) d[k + 32 * u] = v[u];
         }
-        for (; k < nt; k += 32) d[k] = s[k];
     }
 }
 
@@ -362,25 +376,39 @@ cudaError_t launch_halo_planes(double* W, const FieldConst& fc, int J0, int J1, 
 }
 
 template <bool EXPAND>
-static cudaError_t rows_t(const DenseRows& dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
+static cudaError_t rows_t(const double* src, double* dst, const FieldConst& fc, const DevClock* view, DevClock* mark,
+                          cudaStream_t s)
 {
-    const long long rows = (long long)fc.nt * fc.nt;
+    const long long rows = 5LL * fc.nt * fc.nt;
     long long blocks = (rows + 7) / 8;
-    if (blocks > 148 * 4) blocks = 148 * 4;
-    rows_kernel<EXPAND><<<dim3((unsigned)blocks, 5), 256, 0, s>>>(dense, W, fc, view);
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    rows_kernel<EXPAND><<<(unsigned)blocks, 256, 0, s>>>(src, dst, rows, fc.nt, fc.pitch, view, mark);
     return cudaGetLastError();
 }
-cudaError_t launch_rows_expand(const DenseRows& dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
+cudaError_t launch_rows_expand(const double* dense, double* W, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
-    return rows_t<true>(dense, W, fc, view, s);
+    return rows_t<true>(dense, W, fc, view, nullptr, s);
 }
-cudaError_t launch_rows_compact(double* W, const DenseRows& dense, const FieldConst& fc, const DevClock* view, cudaStream_t s)
+cudaError_t launch_rows_compact(const double* W, double* dense, const FieldConst& fc, const DevClock* view, cudaStream_t s)
 {
-    return rows_t<false>(dense, W, fc, view, s);
+    return rows_t<false>(W, dense, fc, view, nullptr, s);
 }
-cudaError_t launch_view_mark(DevClock* clock, cudaStream_t s)
+cudaError_t launch_view(const double* W, double* dense, const FieldConst& fc, DevClock* clock, bool maybe, cudaStream_t s)
 {
+    if (!maybe) return rows_t<false>(W, dense, fc, nullptr, clock, s);
+    // every block of the copy reads the mark, so it is set behind it
+    const cudaError_t e = rows_t<false>(W, dense, fc, clock, nullptr, s);
+    if (e != cudaSuccess) return e;
     view_mark_kernel<<<1, 1, 0, s>>>(clock);
+    return cudaGetLastError();
+}
+cudaError_t launch_arrays(bool expand, const DenseRows& dense, double* W, const FieldConst& fc, cudaStream_t s)
+{
+    long long blocks = ((long long)fc.nt * fc.nt + 7) / 8;
+    if (blocks > 148 * 4) blocks = 148 * 4;
+    const dim3 grid((unsigned)blocks, 5);
+    if (expand) arrays_kernel<true><<<grid, 256, 0, s>>>(dense, W, fc);
+    else arrays_kernel<false><<<grid, 256, 0, s>>>(dense, W, fc);
     return cudaGetLastError();
 }
 
