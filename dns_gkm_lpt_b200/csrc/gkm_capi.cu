@@ -563,7 +563,7 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 {
     *dense = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
-    double* out = h->buf[h->parity ^ 1];
+    double* out = h->view_live ? h->view_buffer() : h->buf[h->parity ^ 1];
     if (!h->view_live || ask_device(h)) {
         CK(h, gkm::launch_rows_compact(h->buf[h->parity], out, h->fc, h->view_live ? h->clock : nullptr, h->stream));
         h->launches += 1;
@@ -575,7 +575,7 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 gkm_status gkm_host::take_view(gkm_handle* h)
 {
     if (!h->view_live) return GKM_OK;
-    CK(h, gkm::launch_rows_expand(h->buf[h->parity ^ 1], h->buf[h->parity], h->fc, ask_device(h), h->stream));
+    CK(h, gkm::launch_rows_expand(h->view_buffer(), h->buf[h->parity], h->fc, ask_device(h), h->stream));
     h->launches += 1;
     return GKM_OK;
 }
@@ -797,6 +797,7 @@ gkm_status gkm_destroy(gkm_handle* h)
     cudaFree(h->lap_nodes);
     cudaFree(h->props);
     cudaFree(h->pipe_dense);
+    cudaFree(h->view);
     for (cudaEvent_t e : h->pipe_ev) cudaEventDestroy(e);
     for (cudaStream_t s : {h->pipe_in, h->pipe_out, h->pipe_comp[0], h->pipe_comp[1], h->pipe_comp[2], h->pipe_comp[3],
                            h->pipe_halo})
@@ -815,9 +816,10 @@ gkm_status gkm_upload_state(gkm_handle* h, const double* const W[5])
         if (!W[q]) return fail(h, GKM_ERR_ARG, "W[q] is NULL");
     const size_t bytes = sizeof(double) * (size_t)h->fc.nt3;
     double* dst = h->buf[h->parity];
-    // odd grids: to their pitch from the device's own arrays, from others through the accumulator buffer, free between steps
+    // odd grids: to their pitch from the device's own arrays, from others through the accumulator buffer, free between
+    // steps, or the view
     const bool odd = h->fc.pitch != h->fc.nt;
-    double* land = odd ? h->buf[h->parity ^ 1] : dst;
+    double* land = !odd ? dst : (h->view_live ? h->view_buffer() : h->buf[h->parity ^ 1]);
     if (odd && on_device(W, bytes, h->cfg.device)) {
         const gkm::DenseRows own{{(double*)W[0], (double*)W[1], (double*)W[2], (double*)W[3], (double*)W[4]}};
         CK(h, gkm::launch_arrays(true, own, dst, h->fc, h->stream));
@@ -969,7 +971,7 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     }
     const bool mixed = h->cfg.precision == GKM_PREC_MIXED;
     const int nvar = mixed ? gkm::kSweepVariants32 : gkm::kSweepVariants64;
-    // the sweeps leave W untouched (they write the accumulator A only, a live view of an odd grid with it); the
+    // the sweeps leave W untouched (they write the accumulator A only, an odd grid's view with it where that lies there); the
     // clock they also touch is saved here and put back afterwards
     DevClock saved;
     CK(h, cudaMemcpyAsync(&saved, h->clock, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
@@ -1030,7 +1032,7 @@ gkm_status gkm_autotune(gkm_handle* h, int32_t reps)
     h->sweep_chosen = true;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (h->view_live) {   // the sweeps have written over it
+    if (h->view_live && !h->view) {   // the sweeps have written over it
         gkm::launch_rows_compact(h->buf[h->parity], h->buf[h->parity ^ 1], h->fc, nullptr, h->stream);
         h->launches += 1;
     }
@@ -1530,7 +1532,7 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
     *W = h->buf[h->parity];
     if (h->fc.pitch == h->fc.nt) return GKM_OK;
     if (h->view_live && !ask_device(h)) {
-        *W = h->buf[h->parity ^ 1];
+        *W = h->view_buffer();
         return GKM_OK;
     }
     // The caller may read it on any stream, as it may the state of an idle handle: done when the call returns,
@@ -1539,13 +1541,17 @@ gkm_status gkm_device_state(gkm_handle* h, double** W)
     cudaStream_t s = rec ? h->own_stream : h->stream;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
-    cudaError_t e = gkm::launch_view(*W, h->buf[h->parity ^ 1], h->fc, h->clock, h->view_live, s);
+    if (!h->view && !h->view_live && cudaMalloc(&h->view, sizeof(double) * 5 * (size_t)h->fc.nt3) != cudaSuccess) {
+        cudaGetLastError();
+        h->view = nullptr;
+    }
+    cudaError_t e = gkm::launch_view(*W, h->view_buffer(), h->fc, h->clock, h->view_live, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (rec) CK(h, cudaThreadExchangeStreamCaptureMode(&mode));
     CK(h, e);
     h->launches += h->view_live ? 2 : 1;
     h->view_live = true;
-    *W = h->buf[h->parity ^ 1];
+    *W = h->view_buffer();
     return GKM_OK;
 }
 

@@ -446,10 +446,10 @@ gkm_status gkm_ensemble_autotune(gkm_ensemble* E, int32_t reps)
         if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
         return e == cudaSuccess ? GKM_OK : ecuda(E, e, "gkm_ensemble_autotune");
     };
-    // live views of odd members lie in the accumulators: taken in by the first refresh, handed back below
+    // live views of odd members that lie in the accumulators: taken in by the first refresh, handed back below
     std::vector<gkm_handle*> views;
     for (gkm_handle* h : E->mem)
-        if (h->view_live) {
+        if (h->view_live && !h->view) {
             views.push_back(h);
             h->view_live = false;
         }

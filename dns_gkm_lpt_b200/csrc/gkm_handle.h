@@ -67,10 +67,13 @@ struct gkm_handle {
     // plug-point pipeline (gkm_evolve with pinned or device buffers): copy-in, copy-out and
     // two compute streams, and per-chunk events, created on first use
     cudaStream_t pipe_in = nullptr, pipe_out = nullptr, pipe_comp[4] = {nullptr, nullptr, nullptr, nullptr};
-    // odd grids: gkm_device_state has handed out a dense state, which lies in the accumulator buffer.  From
-    // that call to the next step it is the state: callers may write to it, and every use of the state takes
-    // it in first.  The device knows whether a step has come since (DevClock::view).
+    // odd grids: gkm_device_state has handed out a dense state.  From that call to the next step it is the
+    // state: callers may write to it, and every use of the state takes it in first.  The device knows whether
+    // a step has come since (DevClock::view).  It has a buffer of its own, which steps leave alone while a
+    // caller's streams still read it (allocated on first use), or without memory for one the accumulator's.
+    double* view = nullptr;
     bool view_live = false;
+    double* view_buffer() const { return view ? view : buf[parity ^ 1]; }
     double* pipe_dense = nullptr;       // odd grids: the pipeline's dense planes, 5 x nt^3 (on first use)
     cudaStream_t pipe_halo = nullptr;   // ghost wrap of each part as it lands, off the copy-in stream
     std::vector<cudaEvent_t> pipe_ev;
@@ -107,7 +110,7 @@ inline gkm_status cuda_fail(gkm_handle* h, cudaError_t e, const char* where)
     } while (0)
 
 // the current state as dense rows (5 components of nt^3, device memory): the state itself, or on odd
-// grids a copy in the accumulator buffer, which is free between steps, or the caller's view there
+// grids the caller's view or a copy in the accumulator buffer, which is free between steps
 gkm_status dense_state(gkm_handle* h, const double** dense);
 // before work on the state: what the caller may have written to the view, into the state's rows
 gkm_status take_view(gkm_handle* h);

@@ -328,9 +328,10 @@ gkm_status gkm_weno_faces(const double* stencils, int64_t n, double gam, double*
 gkm_status gkm_set_stream(gkm_handle* h, void* stream);
 /* Device pointer of the current state (5 x nt^3 doubles, component-major);
  * valid until the next step; until then it is the state, and what a caller
- * writes there counts.  Odd n: a dense view of the handle's padded rows in the
- * buffer of the next step, copied by the call (which then synchronises) and
- * taken in before each use. */
+ * writes there counts.  Odd n: a dense view of the handle's padded rows, copied
+ * by the call (which then synchronises) and taken in before each use; it has a
+ * buffer of its own (5 x nt^3 doubles, allocated on first use) or, without memory
+ * for one, the next step's. */
 gkm_status gkm_device_state(gkm_handle* h, double** W);
 
 /* ---------------------------------------------------------------- ensemble
