@@ -575,7 +575,9 @@ gkm_status gkm_host::dense_state(gkm_handle* h, const double** dense)
 gkm_status gkm_host::take_view(gkm_handle* h)
 {
     if (!h->view_live) return GKM_OK;
-    CK(h, gkm::launch_rows_expand(h->view_buffer(), h->buf[h->parity], h->fc, ask_device(h), h->stream));
+    // a recorded launch may be replayed after the view's time
+    CK(h, gkm::launch_rows_expand(h->view_buffer(), h->buf[h->parity], h->fc, recording(h) ? h->clock : ask_device(h),
+                                  h->stream));
     h->launches += 1;
     return GKM_OK;
 }

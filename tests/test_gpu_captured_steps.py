@@ -85,3 +85,23 @@ def test_captured_steps_and_the_device_state(n, late):
         s.evolve_eulerian(2)
         s.synchronize()
         assert np.array_equal(s.device_state().cpu().numpy(), half)
+
+
+@pytest.mark.parametrize("n", [14, 15])
+def test_recorded_splines_leave_later_states_alone(n):
+    """Splines recorded while a device view was live, replayed after steps of the host: no old view comes back."""
+    P, W0 = analytic_case(n, 60 + n)
+    with Solver(P, cfl=0.5) as s:
+        stream = torch.cuda.Stream()
+        s.set_stream(stream.cuda_stream)
+        s.upload_state(W0)
+        s.device_state()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            s.generate_splines()
+        s.evolve_eulerian(2)
+        want = s.download_state()
+        with torch.cuda.stream(stream):
+            g.replay()
+        s.synchronize()
+        assert np.array_equal(s.download_state(), want)
