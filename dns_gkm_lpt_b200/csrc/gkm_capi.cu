@@ -674,7 +674,8 @@ gkm_status gkm_create(const gkm_config* cfg, gkm_handle** out)
     fc.k4 = K + 4;
     fc.k5 = K + 5;
     fc.k7 = K + 7;
-    fc.iPrK3 = (1.0 / gkm::kPrandtl) * (1.0 / (K + 3));
+    fc.iK3 = 1.0 / (K + 3);
+    fc.iPrK3 = (1.0 / gkm::kPrandtl) * fc.iK3;
     fc.dK2 = (K + 3) - 2.0 / fc.gm1;
     fc.suth_c = fc.mu0 * (fc.T0 + 110.4) * gkm::kR / ((gkm::kR * fc.T0) * std::sqrt(gkm::kR * fc.T0));
 

@@ -44,9 +44,9 @@ struct FieldConst {
     double p0, u_s, inv_rho_s, inv_m_s, inv_E_s, inv_T0;
     double eps_rho, eps_m, eps_T;   // the WENO epsilon 1e-10 expressed in those units
     double fscale[5];
-    // the flux's constants of K (K + 2 .. K + 7, 1/(Pr (K+3)), Phys::dK2) and the Sutherland
+    // the flux's constants of K (K + 2 .. K + 7, 1/(K+3), 1/(Pr (K+3)), Phys::dK2) and the Sutherland
     // factor mu0 (T0 + 110.4) R / (R T0)^(3/2)
-    double k2, k3, k4, k5, k7, iPrK3, dK2, suth_c;
+    double k2, k3, k4, k5, k7, iK3, iPrK3, dK2, suth_c;
 };
 
 // Sweep geometry: a CTA covers a TB x TA window of faces in the plane normal

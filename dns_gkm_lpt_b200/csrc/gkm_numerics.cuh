@@ -96,7 +96,7 @@ struct Phys {
     // K + 2 .. K + 7 and 1 / (Pr (K + 3)) as the flux uses them (the sweeps take them from the launch's
     // constants, so they occupy no registers)
     T k2 = T(K + 2), k3 = T(K + 3), k4 = T(K + 4), k5 = T(K + 5), k7 = T(K + 7);
-    T iPrK3 = T(1.0 / kPrandtl) * (T(1) / T(K + 3));
+    T iK3 = T(1) / T(K + 3), iPrK3 = T(1.0 / kPrandtl) * (T(1) / T(K + 3));
     // twice what the energy of a Maxwellian with K internal degrees of freedom exceeds p / (gam - 1) by,
     // over p: zero but for rounding where (5-3g)/(g-1) is whole
     T dK2 = T(K + 3) - T(2) / gm1;
@@ -395,13 +395,15 @@ GKM_HD void build_moments(Moments<T>& M, const T U[3], T lam, int K, int half)
     full_table<T, 6>(M.Z, U[2], inv2lam);
 }
 
+#define GKM_TABLES(S) S.Y, S.Z
 #define TM(A, B, C) (I[k + (A)] * Y[l + (B)] * Z[m + (C)])
+#define GKM_YZ_PARAM const T* Y, const T* Z
 
 // ----------------------------------------------------------- MCal -----
 // <psi (u^k v^l w^m) (a0 + a1 u + a2 v + a3 w + a4 psi4)> with psi = (1,u,v,w,psi4),
 // psi4 = (u^2+v^2+w^2+xi^2)/2; I = normal table (full or half), Y, Z tangential.
 template <int k, int l, int m, class T>
-GKM_HD void mcal(T M[5], const T* I, const T* Y, const T* Z, T Ie2, T Ie4, const T a[5])
+GKM_HD void mcal(T M[5], const T* I, GKM_YZ_PARAM, T Ie2, T Ie4, const T a[5])
 {
     T t000 = TM(0, 0, 0), t100 = TM(1, 0, 0), t010 = TM(0, 1, 0), t001 = TM(0, 0, 1);
     T t200 = TM(2, 0, 0), t020 = TM(0, 2, 0), t002 = TM(0, 0, 2);
@@ -421,7 +423,7 @@ GKM_HD void mcal(T M[5], const T* I, const T* Y, const T* Z, T Ie2, T Ie4, const
 }
 
 template <int k, int l, int m, class T>
-GKM_HD void mcal0(T M[5], const T* I, const T* Y, const T* Z, T Ie2)
+GKM_HD void mcal0(T M[5], const T* I, GKM_YZ_PARAM, T Ie2)
 {
     M[0] = TM(0, 0, 0);
     M[1] = TM(1, 0, 0);
@@ -592,7 +594,7 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
         build_moments<T>(S, Us, lam, K, side == 0 ? +1 : -1);
         SlopeState<T> ss = slope_state<T>(Us, lam, K);
         T iden = T(1) / den;
-        mcal0<0, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2);
+        mcal0<0, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2);
         axpy5<T>(We, den, M);
         T Bs[5] = {0, 0, 0, 0, 0};   // -(Mf100 ax + Mf010 ay + Mf001 az)
         T b[5], a[5];
@@ -600,44 +602,44 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
 #pragma unroll
         for (int q = 0; q < 5; q++) b[q] = in.DW(0 + side, q) * iden;
         slope_solve<T>(b, ss, a);
-        mcal<1, 0, 0, T>(M, S.X, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<1, 0, 0, T>(M, S.X, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bs, T(-1), M);
-        mcal<1, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<1, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bacc, cB * den, M);
-        mcal<2, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<2, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Facc, p4 * den, M);
         // first tangential slope
 #pragma unroll
         for (int q = 0; q < 5; q++) b[q] = in.DW(2 + side, q) * iden;
         slope_solve<T>(b, ss, a);
-        mcal<0, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(by_, T(1), M);
-        mcal<0, 1, 0, T>(M, S.X, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 1, 0, T>(M, S.X, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bs, T(-1), M);
-        mcal<0, 1, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 1, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bacc, cB * den, M);
-        mcal<1, 1, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<1, 1, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Facc, p4 * den, M);
         // second tangential slope
 #pragma unroll
         for (int q = 0; q < 5; q++) b[q] = in.DW(4 + side, q) * iden;
         slope_solve<T>(b, ss, a);
-        mcal<0, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(bz_, T(1), M);
-        mcal<0, 0, 1, T>(M, S.X, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 0, 1, T>(M, S.X, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bs, T(-1), M);
-        mcal<0, 0, 1, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 0, 1, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bacc, cB * den, M);
-        mcal<1, 0, 1, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<1, 0, 1, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Facc, p4 * den, M);
         // time slope of this side, src/GKMflux.cpp:145-151
         slope_solve<T>(Bs, ss, a);
-        mcal<0, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<0, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Bacc, gm5 * den, M);
-        mcal<1, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2, S.Ie4, a);
+        mcal<1, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2, S.Ie4, a);
         axpy5<T>(Facc, p5 * den, M);
         // free transport of the initial half-Maxwellian
-        mcal0<1, 0, 0, T>(M, S.H, S.Y, S.Z, S.Ie2);
+        mcal0<1, 0, 0, T>(M, S.H, GKM_TABLES(S), S.Ie2);
         axpy5<T>(Facc, p3 * den, M);
     }
 
@@ -659,37 +661,37 @@ GKM_HD void gks_flux_mcal(const Prov& in, T tau0, T dt, T dx, const Phys<T>& ph,
 #pragma unroll
     for (int q = 0; q < 5; q++) b[q] = (We[q] - in.WL(q)) * idx2;
     slope_solve<T>(b, se, a);
-    mcal<1, 0, 0, T>(M, E.H, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<1, 0, 0, T>(M, E.H, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Bacc, gm2 * dene, M);
-    mcal<2, 0, 0, T>(M, E.H, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<2, 0, 0, T>(M, E.H, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Facc, p2 * dene, M);
 #pragma unroll
     for (int q = 0; q < 5; q++) b[q] = (in.WR(q) - We[q]) * idx2;
     slope_solve<T>(b, se, a);
-    mcal<1, 0, 0, T>(M, H2, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<1, 0, 0, T>(M, H2, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Bacc, gm2 * dene, M);
-    mcal<2, 0, 0, T>(M, H2, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<2, 0, 0, T>(M, H2, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Facc, p2 * dene, M);
     // tangential equilibrium slopes
     slope_solve<T>(by_, se, a);
-    mcal<0, 1, 0, T>(M, E.X, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<0, 1, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Bacc, gm2 * dene, M);
-    mcal<1, 1, 0, T>(M, E.X, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<1, 1, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Facc, p2 * dene, M);
     slope_solve<T>(bz_, se, a);
-    mcal<0, 0, 1, T>(M, E.X, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<0, 0, 1, T>(M, E.X, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Bacc, gm2 * dene, M);
-    mcal<1, 0, 1, T>(M, E.X, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<1, 0, 1, T>(M, E.X, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Facc, p2 * dene, M);
     // time derivative of the equilibrium, src/GKMflux.cpp:183-191
-    mcal0<0, 0, 0, T>(M, E.X, E.Y, E.Z, E.Ie2);
+    mcal0<0, 0, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2);
     T idene = T(1) / dene;
 #pragma unroll
     for (int q = 0; q < 5; q++) b[q] = (gm1 * dene * M[q] + Bacc[q] + gm3 * We[q]) * idene;
     slope_solve<T>(b, se, a);
-    mcal<1, 0, 0, T>(M, E.X, E.Y, E.Z, E.Ie2, E.Ie4, a);
+    mcal<1, 0, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2, E.Ie4, a);
     axpy5<T>(Facc, p1 * dene, M);
-    mcal0<1, 0, 0, T>(M, E.X, E.Y, E.Z, E.Ie2);
+    mcal0<1, 0, 0, T>(M, E.X, GKM_TABLES(E), E.Ie2);
     axpy5<T>(Facc, p0 * dene, M);
 #pragma unroll
     for (int q = 0; q < 5; q++) F[q] = Facc[q];

@@ -132,6 +132,7 @@ __device__ __forceinline__ Phys<T> sweep_phys(const FieldConst& fc)
     ph.k4 = T(fc.k4);
     ph.k5 = T(fc.k5);
     ph.k7 = T(fc.k7);
+    ph.iK3 = T(fc.iK3);
     ph.iPrK3 = T(fc.iPrK3);
     if (sizeof(T) == 8) ph.dK2 = T(fc.dK2);   // the float's own rounding of gamma - 1 enters the mixed one
     return ph;
